@@ -78,6 +78,8 @@ bool fft_plan_radices(int n, int order, FftPlan* p) {
   for (int s = 0; s < ns; ++s) {
     p->L[s] = L;
     L /= p->radix[s];
+    p->mul_m[s] = fast_div_mul((uint32_t)L);
+    p->mul_nb[s] = fast_div_mul((uint32_t)(n / p->radix[s]));
   }
   return true;
 }
@@ -537,8 +539,8 @@ int phgpu_ctx_init(phgpu_ctx* ctx) {
   CK(cudaStreamCreateWithFlags(&ctx->s1, cudaStreamNonBlocking));
   CK(cudaEventCreateWithFlags(&ctx->ev_a, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&ctx->ev_b, cudaEventDisableTiming));
-  CK(spatial_init_attributes());
-  CK(so3_init_attributes());
+  CK(spatial_init_attributes(N, ctx->M));
+  CK(so3_init_attributes(2 * bw_out));
   CK(sht_init_attributes());
   std::string perr;
   if (!make_fft_plan(2 * bw, &ctx->plan_s2, &ctx->d_tw[0], &perr) ||
@@ -547,24 +549,10 @@ int phgpu_ctx_init(phgpu_ctx* ctx) {
     ctx->err = perr;
     return PHGPU_ERR_INVALID;
   }
-  if (spatial_slab_path(N)) {
-    if (!make_fft_plan(N / 2, &ctx->plan_sp_half, &ctx->d_tw[3], &perr)) {
-      ctx->err = perr;
-      return PHGPU_ERR_INVALID;
-    }
-    ctx->has_sp_half = true;
-  }
   if (ctx->pad) {
-    if (!make_fft_plan(ctx->M, &ctx->plan_pad, &ctx->d_tw_pad[0], &perr)) {
+    if (!make_fft_plan(ctx->M, &ctx->plan_pad, &ctx->d_tw_pad, &perr)) {
       ctx->err = perr;
       return PHGPU_ERR_INVALID;
-    }
-    if (spatial_slab_path(ctx->M)) {
-      if (!make_fft_plan(ctx->M / 2, &ctx->plan_pad_half, &ctx->d_tw_pad[1], &perr)) {
-        ctx->err = perr;
-        return PHGPU_ERR_INVALID;
-      }
-      ctx->has_pad_half = true;
     }
   }
   ctx->bands_s2 = make_bands((uint32_t)(bw * bw), (int)prm->fusion_levels, 4.0f);
@@ -663,8 +651,8 @@ int phgpu_ctx_init(phgpu_ctx* ctx) {
     CKV(dalloc(ctx, &ctx->d_grids[s], sizeof(float) * 5 * nv));
     CKV(dalloc(ctx, &ctx->d_rowlive[s], (size_t)N * N));
   }
-  CKV(dalloc(ctx, &ctx->d_slab_nz, (size_t)8 * N));
-  CK(cudaMemset(ctx->d_slab_nz, 1, (size_t)8 * N));  // nothing known to be zero yet
+  CKV(dalloc(ctx, &ctx->d_rowmask, (size_t)2 * N * N));
+  CKV(dalloc(ctx, &ctx->d_slab_live, (size_t)2 * N));
   CKV(dalloc(ctx, &ctx->d_spec, sizeof(float2) * 8 * H));
   CKV(dalloc(ctx, &ctx->d_cspec, sizeof(float2) * H));
   // volumes: kept on request, and needed by the peak-neighbourhood fits
@@ -700,10 +688,9 @@ int phgpu_ctx_destroy(phgpu_ctx* ctx) {
   if (ctx->s1) cudaStreamSynchronize(ctx->s1);
   for (void* p : ctx->allocs) cudaFree(p);
   ctx->allocs.clear();
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < 3; ++i)
     if (ctx->d_tw[i]) cudaFree(ctx->d_tw[i]);
-  for (int i = 0; i < 2; ++i)
-    if (ctx->d_tw_pad[i]) cudaFree(ctx->d_tw_pad[i]);
+  if (ctx->d_tw_pad) cudaFree(ctx->d_tw_pad);
   if (ctx->h_argmax) cudaFreeHost(ctx->h_argmax);
   if (ctx->h_T) cudaFreeHost(ctx->h_T);
   if (ctx->h_np) cudaFreeHost(ctx->h_np);
@@ -856,6 +843,7 @@ static FuseS2Args fuse_args(phgpu_ctx* ctx, int n_data, int n_total, int laplace
   f.bands = ctx->bands_s2;
   f.coef = ctx->d_coef;
   f.fused = ctx->d_fused;
+  f.argmax = ctx->d_argmax;
   return f;
 }
 
@@ -889,12 +877,12 @@ int phgpu_run_sph_leg_fuse_batch(phgpu_ctx* const* ctx, int k, int n_data, int n
   for (int i = 0; i < k; ++i) {
     f.coef_b[i] = ctx[i]->d_coef;
     f.fused_b[i] = ctx[i]->d_fused;
+    f.argmax_b[i] = ctx[i]->d_argmax;
   }
   {
     ProfScope ps(c0, st, PS_FUSE_S2);
     CKC(c0, launch_fuse_s2(f, st));
   }
-  for (int i = 0; i < k; ++i) CKC(c0, cudaMemsetAsync(ctx[i]->d_argmax, 0, sizeof(unsigned long long), st));
   return PHGPU_OK;
 }
 
@@ -909,7 +897,6 @@ int phgpu_run_sph_front(phgpu_ctx* ctx, int n_data, int n_total, int laplace, cu
     ProfScope ps(ctx, st, PS_FUSE_S2);
     CK(launch_fuse_s2(fuse_args(ctx, n_data, n_total, laplace), st));
   }
-  CK(cudaMemsetAsync(ctx->d_argmax, 0, sizeof(unsigned long long), st));
   return PHGPU_OK;
 }
 
@@ -1057,18 +1044,12 @@ int phgpu_run_voxelize(phgpu_ctx* ctx, int side, const float* T12, int n_data, c
   return PHGPU_OK;
 }
 
-// After the forward transform of a voxelised side inside register_pair (the
-// grids are internal there): zero what the voxelisation wrote, so the next
-// voxelisation of this side needs no full-grid memset.
-static int clear_voxelized(phgpu_ctx* ctx, int side, cudaStream_t st) {
-  const int planes = ctx->vox_ch[side] + 1;
-  const size_t nv = (size_t)ctx->N * ctx->N * ctx->N;
-  CK(launch_clear_voxels(ctx->d_lin[side], ctx->dev_counts ? (int)ctx->cap_points : (int)ctx->np[side],
-                         ctx->d_grids[side], nv, planes, ctx->d_rowlive[side], ctx->N, st,
-                         ctx->dev_counts ? ctx->d_np + side : nullptr));
-  ctx->clean_planes[side] = planes;
+// Inside register_pair the grids are internal: the forward transform of a
+// voxelised side zeroes what the voxelisation wrote (SpatialArgs::clear), so the
+// next voxelisation of this side needs no full-grid memset.
+static void voxels_cleared(phgpu_ctx* ctx, int side) {
+  ctx->clean_planes[side] = ctx->vox_ch[side] + 1;
   ctx->grids_live[side] = false;
-  return PHGPU_OK;
 }
 
 int phgpu_voxelize(phgpu_ctx* ctx, const phgpu_cloud* cloud, int side, const float* T12) {
@@ -1091,7 +1072,7 @@ int phgpu_get_voxel_index(phgpu_ctx* ctx, int side, uint32_t* lin, uint32_t n_po
   return PHGPU_OK;
 }
 
-static SpatialArgs spatial_args(phgpu_ctx* ctx, int n_data, int n_total, int laplace, int means) {
+static SpatialArgs spatial_args(phgpu_ctx* ctx, int n_data, int n_total, int laplace, int means, int clear) {
   SpatialArgs a;
   a.N = ctx->N;
   a.n_data_ch = n_data;
@@ -1105,18 +1086,17 @@ static SpatialArgs spatial_args(phgpu_ctx* ctx, int n_data, int n_total, int lap
   a.bands = ctx->bands_sp;
   a.grids_f = ctx->d_grids[0];
   a.grids_g = ctx->d_grids[1];
+  a.count_plane = n_data;
   a.grids_are_means = means;
-  // row flags describe voxelised grids only (host-written grids are dense)
-  a.rowlive_f = means ? nullptr : ctx->d_rowlive[0];
-  a.rowlive_g = means ? nullptr : ctx->d_rowlive[1];
-  // the padded path transforms the spectra in place: no slab stays known-zero
-  a.slab_nz = ctx->pad ? nullptr : ctx->d_slab_nz;
+  a.clear = clear;
+  for (int s = 0; s < 2; ++s) a.rowlive[s] = ctx->d_rowlive[s];
+  a.rowmask = ctx->d_rowmask;
+  a.slab_live = ctx->d_slab_live;
+  a.full_spec = ctx->pad ? 1 : 0;  // the padded path transforms whole spectra in place
   a.spec = ctx->d_spec;
   a.cspec = ctx->d_cspec;
   a.plan = &ctx->plan_sp;
-  a.plan_half = ctx->has_sp_half ? &ctx->plan_sp_half : nullptr;
   a.argmax = ctx->d_argmax + 1;
-  a.status = ctx->d_argmax + 2;
   a.volume = ctx->d_transvol;
   a.fuse_tile = (int)ctx->tune.fuse_z_tile;
   return a;
@@ -1146,8 +1126,6 @@ static int run_spatial_padded(phgpu_ctx* ctx, const SpatialArgs& a, cudaStream_t
     pa.spec = a.spec;
     pa.prev_f = (a.laplace && ctx->prev_valid[0]) ? ctx->d_prev[0] : nullptr;
     pa.prev_g = (a.laplace && ctx->prev_valid[1]) ? ctx->d_prev[1] : nullptr;
-    pa.x_natural_N = (spatial_slab_path(N) && a.plan_half) ? 1 : 0;
-    pa.x_natural_M = ctx->has_pad_half ? 1 : 0;
     pa.planN = ctx->plan_sp;
     pa.planM = ctx->plan_pad;
     pa.bands = ctx->bands_sp;
@@ -1172,7 +1150,6 @@ static int run_spatial_padded(phgpu_ctx* ctx, const SpatialArgs& a, cudaStream_t
   am.N = M;
   am.cspec = ctx->d_cspec_pad;
   am.plan = &ctx->plan_pad;
-  am.plan_half = ctx->has_pad_half ? &ctx->plan_pad_half : nullptr;
   am.argmax_limit = ctx->corr_size;
   CK(cudaMemsetAsync(ctx->d_argmax + 1, 0, sizeof(unsigned long long), st));
   {
@@ -1183,7 +1160,7 @@ static int run_spatial_padded(phgpu_ctx* ctx, const SpatialArgs& a, cudaStream_t
 }
 
 int phgpu_run_spatial(phgpu_ctx* ctx, int n_data, int n_total, int laplace, int means, cudaStream_t st) {
-  SpatialArgs a = spatial_args(ctx, n_data, n_total, laplace, means);
+  SpatialArgs a = spatial_args(ctx, n_data, n_total, laplace, means, 0);
   {
     ProfScope ps(ctx, st, PS_SPATIAL_FWD);
     CK(launch_spatial_forward(a, 0, st));
@@ -1196,7 +1173,6 @@ int phgpu_run_spatial(phgpu_ctx* ctx, int n_data, int n_total, int laplace, int 
     ctx->have_trans = true;
     return PHGPU_OK;
   }
-  CK(cudaMemsetAsync(ctx->d_argmax + 1, 0, sizeof(unsigned long long), st));
   {
     ProfScope ps(ctx, st, PS_FUSE_Z);
     CK(launch_spatial_fuse_z(a, st));
@@ -1259,10 +1235,6 @@ int phgpu_spatial_result(phgpu_ctx* ctx, uint32_t* voxel, float* peak, double* c
   }
   cudaSetDevice(ctx->prm.device);
   CK(cudaStreamSynchronize(ctx->s0));
-  if (ctx->h_argmax[2] & 1ull) {
-    ctx->err = "a bulk-copy wait in the translation kernels timed out";
-    return PHGPU_ERR_CUDA;
-  }
   const unsigned long long k = ctx->h_argmax[1];
   if (voxel) *voxel = unpack_index(k);
   if (peak) *peak = float_from_order_bits((uint32_t)(k >> 32));
@@ -1298,12 +1270,12 @@ int phgpu_pair_front(phgpu_ctx* ctx, const PairPlan& pp, bool until_phi) {
   CK(cudaEventRecord(ctx->ev_a, s0));
   CK(cudaStreamWaitEvent(s1, ctx->ev_a, 0));
   CKV(phgpu_run_voxelize(ctx, 0, nullptr, pp.nd_sp, s1));
-  const SpatialArgs sa = spatial_args(ctx, pp.nd_sp, (int)ctx->prm.n_channels, pp.laplace_sp, 0);
+  const SpatialArgs sa = spatial_args(ctx, pp.nd_sp, (int)ctx->prm.n_channels, pp.laplace_sp, 0, 1);
   {
     ProfScope ps(ctx, s1, PS_SPATIAL_FWD);
     CK(launch_spatial_forward(sa, 0, s1));
   }
-  CKV(clear_voxelized(ctx, 0, s1));
+  voxels_cleared(ctx, 0);
   CK(cudaEventRecord(ctx->ev_b, s1));
   // rotation up to the fused spectra
   CKV(run_sample(ctx, 0, s0));
@@ -1319,18 +1291,17 @@ int phgpu_pair_front(phgpu_ctx* ctx, const PairPlan& pp, bool until_phi) {
 
 int phgpu_pair_back(phgpu_ctx* ctx, const PairPlan& pp, const float* T, const float* T_dev) {
   cudaStream_t s0 = ctx->s0;
-  const SpatialArgs sa = spatial_args(ctx, pp.nd_sp, (int)ctx->prm.n_channels, pp.laplace_sp, 0);
+  const SpatialArgs sa = spatial_args(ctx, pp.nd_sp, (int)ctx->prm.n_channels, pp.laplace_sp, 0, 1);
   CKV(phgpu_run_voxelize(ctx, 1, T, pp.nd_sp, s0, T_dev));
   {
     ProfScope ps(ctx, s0, PS_SPATIAL_FWD);
     CK(launch_spatial_forward(sa, 1, s0));
   }
-  CKV(clear_voxelized(ctx, 1, s0));
+  voxels_cleared(ctx, 1);
   CK(cudaStreamWaitEvent(s0, ctx->ev_b, 0));
   if (ctx->pad) {
     CKV(run_spatial_padded(ctx, sa, s0));
   } else {
-    CK(cudaMemsetAsync(ctx->d_argmax + 1, 0, sizeof(unsigned long long), s0));
     {
       ProfScope ps(ctx, s0, PS_FUSE_Z);
       CK(launch_spatial_fuse_z(sa, s0));
@@ -1388,10 +1359,6 @@ int phgpu_pair_finish(phgpu_ctx* ctx, const PairPlan& pp, bool device_pose, phgp
     CK(cudaEventRecord(ctx->ev_b, ctx->s1));
     CKV(phgpu_pair_back(ctx, pp, T, nullptr));
     CK(cudaStreamSynchronize(s0));
-  }
-  if (ctx->h_argmax[2] & 1ull) {
-    ctx->err = "a bulk-copy wait in the translation kernels timed out";
-    return PHGPU_ERR_CUDA;
   }
   const unsigned long long tk = ctx->h_argmax[1];
   out->voxel = unpack_index(tk);

@@ -38,9 +38,8 @@ struct phgpu_ctx {
   cudaStream_t s0 = nullptr, s1 = nullptr;
   cudaEvent_t ev_a = nullptr, ev_b = nullptr;
   // plans and tables
-  phgpu::FftPlan plan_s2, plan_so3, plan_sp, plan_sp_half;
-  bool has_sp_half = false;
-  float2* d_tw[4] = {nullptr, nullptr, nullptr, nullptr};
+  phgpu::FftPlan plan_s2, plan_so3, plan_sp;
+  float2* d_tw[3] = {nullptr, nullptr, nullptr};
   phgpu::FusionBands bands_s2, bands_sp;
   float4* d_grid = nullptr;
   double* d_weights = nullptr;
@@ -73,9 +72,10 @@ struct phgpu_ctx {
   // translation
   float* d_grids[2] = {nullptr, nullptr};  // [(C+1)][N^3]
   uint8_t* d_rowlive[2] = {nullptr, nullptr};  // [N][N] rows holding a point of the last voxelisation
-  uint8_t* d_slab_nz = nullptr;                 // [8][N] spectrum slabs that may be non-zero (k_slab_fwd)
+  uint8_t* d_slab_live = nullptr;              // [2][N] z-slabs holding a point of the last forward transform
+  uint8_t* d_rowmask = nullptr;  // [2][N][N] row flags of the last forward transform
   // leading grid planes (and row flags) known to be zero: a voxelisation whose
-  // grids were cleared afterwards leaves them zero, so the next one needs no memset
+  // transform cleared its voxels leaves them zero, so the next one needs no memset
   int clean_planes[2] = {0, 0};
   bool grids_live[2] = {false, false};  // grids hold the last voxelisation (not yet cleared)
   float2* d_spec = nullptr;
@@ -84,9 +84,8 @@ struct phgpu_ctx {
   // zero-padded translation (spatial_zero_padding > 0): M = N + 2 pad
   int pad = 0, M = 0;
   uint32_t corr_size = 0;  // the reference's correlation length uint32(N^3 (M / N)^3) (M^3 or M^3 - 1)
-  phgpu::FftPlan plan_pad, plan_pad_half;
-  bool has_pad_half = false;
-  float2* d_tw_pad[2] = {nullptr, nullptr};
+  phgpu::FftPlan plan_pad;
+  float2* d_tw_pad = nullptr;
   float2* d_cspec_pad = nullptr;           // [M][M][H2p(M)]
   float2* d_prev[2] = {nullptr, nullptr};  // Laplace: last channel spectrum of the previous call, per side
   bool prev_valid[2] = {false, false};

@@ -23,8 +23,22 @@ struct FftPlan {
   int nstage;
   int radix[kMaxFftStages];
   int L[kMaxFftStages];
+  uint32_t mul_m[kMaxFftStages];   // fast_div factors of m_s = L_s / r_s
+  uint32_t mul_nb[kMaxFftStages];  // and of the butterfly count n / r_s
   const float2* tw;  // n entries
 };
+
+// x / d by one high multiplication with fast_div_mul(d) (0 for d = 1): exact
+// while x d < 2^32 (the transforms' item counts and lengths stay below 2^18
+// and 2^11).
+__host__ __device__ inline uint32_t fast_div_mul(uint32_t d) { return d > 1 ? 0xffffffffu / d + 1u : 0u; }
+__device__ __forceinline__ int fast_div(int x, uint32_t mul) {
+  return mul ? (int)__umulhi((uint32_t)x, mul) : x;
+}
+
+// Largest radix of the passes' register butterflies (fft_pass.cuh); larger
+// primes take the shared-memory stage there.
+constexpr int kMaxRegRadix = 8;
 
 // Position after a forward (DIF) transform of frequency k.
 __host__ __device__ inline int fft_freq2pos(int k, const FftPlan& p) {
@@ -51,6 +65,44 @@ __host__ __device__ inline int fft_pos2freq(int pos, const FftPlan& p) {
     L = m;
   }
   return k;
+}
+
+// ---------------------------------------------------------------- constexpr twiddles
+
+constexpr double kPiD = 3.14159265358979323846264338327950288;
+
+constexpr double cx_sin_taylor(double x) {
+  double term = x, sum = x;
+  for (int n = 1; n < 30; ++n) {
+    term *= -x * x / ((2.0 * n) * (2.0 * n + 1.0));
+    sum += term;
+  }
+  return sum;
+}
+constexpr double cx_reduce(double a) {
+  while (a > kPiD) a -= 2.0 * kPiD;
+  while (a < -kPiD) a += 2.0 * kPiD;
+  return a;
+}
+constexpr double cx_sin(double a) { return cx_sin_taylor(cx_reduce(a)); }
+constexpr double cx_cos(double a) { return cx_sin_taylor(cx_reduce(a + 0.5 * kPiD)); }
+
+// w_M^e = exp(-2 pi i e / M) for e in [0, M)
+template <int M>
+struct ConstTw {
+  float re[M], im[M];
+  constexpr ConstTw() : re(), im() {
+    for (int e = 0; e < M; ++e) {
+      re[e] = (float)cx_cos(-2.0 * kPiD * e / M);
+      im[e] = (float)cx_sin(-2.0 * kPiD * e / M);
+    }
+  }
+};
+
+template <int M>
+__device__ __forceinline__ float2 ctw(int e) {
+  constexpr ConstTw<M> t;
+  return make_float2(t.re[e], t.im[e]);
 }
 
 // Packed FP32 pairs (sm_100 FADD2 / FFMA2 / FMUL2, PK = true): one
@@ -148,19 +200,29 @@ __device__ __forceinline__ void dft_small(float2 (&x)[R]) {
     x[3] = padd<PK>(e[3], o3);
     x[7] = psub<PK>(e[3], o3);
   } else {
-    // generic small odd prime
+    // small odd prime: sums s_j = x_j + x_{R-j} and differences d_j, then
+    // X_k, X_{R-k} = (x_0 + sum cos s_j) -+ i (sum sin d_j), a quarter of the
+    // plain sum's products
+    constexpr int h = (R - 1) / 2;
+    float2 sj[h], dj[h], y0 = x[0];
+#pragma unroll
+    for (int j = 0; j < h; ++j) {
+      sj[j] = padd<PK>(x[j + 1], x[R - 1 - j]);
+      dj[j] = psub<PK>(x[j + 1], x[R - 1 - j]);
+      y0 = padd<PK>(y0, sj[j]);
+    }
     float2 y[R];
+    y[0] = y0;
 #pragma unroll
-    for (int k = 0; k < R; ++k) {
-      float2 acc = x[0];
+    for (int k = 1; k <= h; ++k) {
+      float2 A = x[0], D = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int j = 1; j < R; ++j) {
-        float s, c;
-        sincospif(2.0f * (float)((j * k) % R) / (float)R, &s, &c);
-        const float2 w = make_float2(c, sg * s);
-        acc = cadd(acc, cmul(x[j], w));
+      for (int j = 0; j < h; ++j) {
+        const float2 w = ctw<R>(((j + 1) * k) % R);  // (cos, -sin)
+        A = pfma<PK>(w.x, sj[j], A);
+        D = pfma<PK>(-w.y, dj[j], D);
       }
-      y[k] = acc;
+      rot_pm<INV>(A, D, y[k], y[R - k]);
     }
 #pragma unroll
     for (int k = 0; k < R; ++k) x[k] = y[k];
@@ -174,22 +236,23 @@ __device__ __forceinline__ void dft_small(float2 (&x)[R]) {
 template <int R, bool INV>
 __device__ __forceinline__ void fft_stage(float2* buf, int ntrans, int tstride, int estride, int n,
                                           int L, const float2* __restrict__ tw, int tid,
-                                          int nthr) {
+                                          int nthr, uint32_t mul_m, uint32_t mul_nb) {
   const int m = L / R;
   const int nb = n / R;
   const int total = ntrans * nb;
   const int twstep = n / L;
   const int es = m * estride;
+  const uint32_t mul_t = estride == 1 ? mul_nb : fast_div_mul(ntrans);
   for (int it = tid; it < total; it += nthr) {
     int t, bf;
     if (estride == 1) {
-      t = it / nb;
+      t = fast_div(it, mul_t);
       bf = it - t * nb;
     } else {
-      bf = it / ntrans;
+      bf = fast_div(it, mul_t);
       t = it - bf * ntrans;
     }
-    const int blk = bf / m;
+    const int blk = fast_div(bf, mul_m);
     const int j2 = bf - blk * m;
     float2* base = buf + t * tstride + (blk * L + j2) * estride;
     float2 x[R];
@@ -338,14 +401,14 @@ __device__ void fft_smem(float2* buf, int ntrans, int tstride, int estride, cons
     const int s = INV ? (p.nstage - 1 - si) : si;
     const int L = p.L[s];
     switch (p.radix[s]) {
-      case 2: fft_stage<2, INV>(buf, ntrans, tstride, estride, p.n, L, p.tw, tid, nthr); break;
-      case 3: fft_stage<3, INV>(buf, ntrans, tstride, estride, p.n, L, p.tw, tid, nthr); break;
-      case 4: fft_stage<4, INV>(buf, ntrans, tstride, estride, p.n, L, p.tw, tid, nthr); break;
-      case 5: fft_stage<5, INV>(buf, ntrans, tstride, estride, p.n, L, p.tw, tid, nthr); break;
-      case 7: fft_stage<7, INV>(buf, ntrans, tstride, estride, p.n, L, p.tw, tid, nthr); break;
-      case 8: fft_stage<8, INV>(buf, ntrans, tstride, estride, p.n, L, p.tw, tid, nthr); break;
-      case 11: fft_stage<11, INV>(buf, ntrans, tstride, estride, p.n, L, p.tw, tid, nthr); break;
-      case 13: fft_stage<13, INV>(buf, ntrans, tstride, estride, p.n, L, p.tw, tid, nthr); break;
+      case 2: fft_stage<2, INV>(buf, ntrans, tstride, estride, p.n, L, p.tw, tid, nthr, p.mul_m[s], p.mul_nb[s]); break;
+      case 3: fft_stage<3, INV>(buf, ntrans, tstride, estride, p.n, L, p.tw, tid, nthr, p.mul_m[s], p.mul_nb[s]); break;
+      case 4: fft_stage<4, INV>(buf, ntrans, tstride, estride, p.n, L, p.tw, tid, nthr, p.mul_m[s], p.mul_nb[s]); break;
+      case 5: fft_stage<5, INV>(buf, ntrans, tstride, estride, p.n, L, p.tw, tid, nthr, p.mul_m[s], p.mul_nb[s]); break;
+      case 7: fft_stage<7, INV>(buf, ntrans, tstride, estride, p.n, L, p.tw, tid, nthr, p.mul_m[s], p.mul_nb[s]); break;
+      case 8: fft_stage<8, INV>(buf, ntrans, tstride, estride, p.n, L, p.tw, tid, nthr, p.mul_m[s], p.mul_nb[s]); break;
+      case 11: fft_stage<11, INV>(buf, ntrans, tstride, estride, p.n, L, p.tw, tid, nthr, p.mul_m[s], p.mul_nb[s]); break;
+      case 13: fft_stage<13, INV>(buf, ntrans, tstride, estride, p.n, L, p.tw, tid, nthr, p.mul_m[s], p.mul_nb[s]); break;
       default:
         fft_stage_generic<INV>(buf, p.radix[s], ntrans, tstride, estride, p.n, L, p.tw, tid, nthr);
         break;
@@ -518,99 +581,6 @@ __device__ __forceinline__ void fft_any(float2* buf, int ntrans, int tstride, in
   } else {
     fft_smem<INV>(buf, ntrans, tstride, estride, p);
   }
-}
-
-// Column transforms with a column-resident thread mapping: thread tid keeps
-// column t = tid % ntrans and walks the butterflies g, g + groups, ... of each
-// stage (g = tid / ntrans, groups = nthr / ntrans), so the index arithmetic
-// is one division per call instead of one per butterfly, and a warp touches
-// neighbouring columns of one butterfly.  Needs ntrans <= nthr (callers fall
-// back to fft_fixed otherwise).
-// PODD: element i of a column sits `podd` further when i is odd (a row-parity
-// slot that spreads neighbouring rows over both halves of the banks).
-template <int N, int R, int L, bool INV, bool PODD = false>
-__device__ __forceinline__ void fixed_col_stage(float2* buf, int stride, const float2* __restrict__ tw, int t, int g,
-                                                int groups, int podd = 0) {
-  constexpr int m = L / R;
-  constexpr int nb = N / R;
-  constexpr int twstep = N / L;
-  if (g >= groups) return;
-  const size_t es = (size_t)m * stride;
-  for (int bf = g; bf < nb; bf += groups) {
-    const int blk = bf / m, j2 = bf - blk * m;
-    const int r0 = blk * L + j2;
-    float2* base = buf + t + (size_t)r0 * stride;
-    // element j is row r0 + j m: its parity is r0's when j m is even
-    const int po0 = PODD ? (r0 & 1) * podd : 0, po1 = PODD ? podd - po0 : 0;
-    float2 x[R];
-#pragma unroll
-    for (int j = 0; j < R; ++j) x[j] = base[j * es + (((j * m) & 1) ? po1 : po0)];
-    // m == 1 (the last forward / first inverse stage): j2 == 0, every twiddle is 1
-    if constexpr (INV) {
-      if constexpr (m > 1) {
-#pragma unroll
-        for (int k = 1; k < R; ++k) x[k] = cmul(x[k], cconj(__ldg(&tw[twstep * j2 * k])));
-      }
-      dft_small<R, true>(x);
-    } else {
-      dft_small<R, false>(x);
-      if constexpr (m > 1) {
-#pragma unroll
-        for (int k = 1; k < R; ++k) x[k] = cmul(x[k], __ldg(&tw[twstep * j2 * k]));
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < R; ++j) base[j * es + (((j * m) & 1) ? po1 : po0)] = x[j];
-  }
-}
-
-template <int N, bool INV, bool PODD = false, int SI = 0>
-__device__ __forceinline__ void fixed_col_stages(float2* buf, int stride, const float2* __restrict__ tw, int t, int g,
-                                                 int groups, int podd = 0) {
-  if constexpr (SI < FixedFft<N>::count) {
-    constexpr int S = INV ? (FixedFft<N>::count - 1 - SI) : SI;
-    fixed_col_stage<N, FixedFft<N>::r[S], fixed_L<N, S>(), INV, PODD>(buf, stride, tw, t, g, groups, podd);
-    __syncthreads();
-    fixed_col_stages<N, INV, PODD, SI + 1>(buf, stride, tw, t, g, groups, podd);
-  }
-}
-
-// Columns t < ntrans of a [N][stride] buffer (element i of column t at
-// buf[t + i * stride]).  Caller synchronises before; ends with __syncthreads().
-template <int NF, bool INV>
-__device__ __forceinline__ void fft_any_cols(float2* buf, int ntrans, int stride, const FftPlan& p) {
-  const int nthr = blockDim.x;
-  if constexpr (NF > 0) {
-    if (ntrans <= nthr) {
-      const int tid = threadIdx.x;
-      fixed_col_stages<NF, INV>(buf, stride, p.tw, tid % ntrans, tid / ntrans, nthr / ntrans);
-      return;
-    }
-  }
-  fft_any<NF, INV, -2>(buf, ntrans, 1, stride, p);
-}
-
-// The same with the row-parity slot: element i of column t at
-// buf[t + i * stride + (i odd ? podd : 0)].  Compile-time lengths only, and
-// ntrans <= blockDim.x.
-template <int NF, bool INV>
-__device__ __forceinline__ void fft_fixed_cols_podd(float2* buf, int ntrans, int stride, int podd,
-                                                    const float2* __restrict__ tw) {
-  static_assert(NF > 0, "row-parity slots need a compile-time plan");
-  const int tid = threadIdx.x, nthr = blockDim.x;
-  fixed_col_stages<NF, INV, true>(buf, stride, tw, tid % ntrans, tid / ntrans, nthr / ntrans, podd);
-}
-
-
-// Column transforms with every count known at compile time: NTRANS columns
-// of a buffer with row stride STRIDE, NTHR threads (== blockDim.x), so the
-// shared-memory offsets and the thread-to-column split fold to constants.
-// PODD as in fixed_col_stage.
-template <int NF, bool INV, int NTRANS, int STRIDE, int NTHR, bool PODD>
-__device__ __forceinline__ void fixed_cols_ct(float2* buf, const float2* __restrict__ tw, int podd) {
-  static_assert(NF > 0 && NTRANS <= NTHR, "compile-time column plan");
-  const int tid = threadIdx.x;
-  fixed_col_stages<NF, INV, PODD>(buf, STRIDE, tw, tid % NTRANS, tid / NTRANS, NTHR / NTRANS, podd);
 }
 
 template <int NF>

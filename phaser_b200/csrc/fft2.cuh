@@ -19,44 +19,6 @@
 
 namespace phgpu {
 
-// ---------------------------------------------------------------- constexpr twiddles
-
-constexpr double kPiD = 3.14159265358979323846264338327950288;
-
-constexpr double cx_sin_taylor(double x) {
-  double term = x, sum = x;
-  for (int n = 1; n < 30; ++n) {
-    term *= -x * x / ((2.0 * n) * (2.0 * n + 1.0));
-    sum += term;
-  }
-  return sum;
-}
-constexpr double cx_reduce(double a) {
-  while (a > kPiD) a -= 2.0 * kPiD;
-  while (a < -kPiD) a += 2.0 * kPiD;
-  return a;
-}
-constexpr double cx_sin(double a) { return cx_sin_taylor(cx_reduce(a)); }
-constexpr double cx_cos(double a) { return cx_sin_taylor(cx_reduce(a + 0.5 * kPiD)); }
-
-// w_M^e = exp(-2 pi i e / M) for e in [0, M)
-template <int M>
-struct ConstTw {
-  float re[M], im[M];
-  constexpr ConstTw() : re(), im() {
-    for (int e = 0; e < M; ++e) {
-      re[e] = (float)cx_cos(-2.0 * kPiD * e / M);
-      im[e] = (float)cx_sin(-2.0 * kPiD * e / M);
-    }
-  }
-};
-
-template <int M>
-__device__ __forceinline__ float2 ctw(int e) {
-  constexpr ConstTw<M> t;
-  return make_float2(t.re[e], t.im[e]);
-}
-
 // ---------------------------------------------------------------- register blocks
 
 // In-register DIF transform of M points (M = RA * RB or a single radix);

@@ -478,6 +478,7 @@ __global__ void k_fuse_s2(FuseS2Args a) {
   float2* __restrict__ fused = a.fused_b[blockIdx.y];
   const int w = 2 * bw - 1;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx == 0) *a.argmax_b[blockIdx.y] = 0ull;
   if (idx >= bw * w) return;
   const int l = idx / w, mi = idx % w;
   const int m = mi - (bw - 1);
@@ -540,6 +541,7 @@ cudaError_t launch_fuse_s2(const FuseS2Args& a0, cudaStream_t st) {
     a.count = 1;
     a.coef_b[0] = a.coef;
     a.fused_b[0] = a.fused;
+    a.argmax_b[0] = a.argmax;
   }
   if (a.count > kMaxWave) return cudaErrorInvalidValue;
   const int tot = a.bw * (2 * a.bw - 1);

@@ -323,13 +323,9 @@ static cudaError_t so3_attrs() {
   return e;
 }
 
-cudaError_t so3_init_attributes() {
+cudaError_t so3_init_attributes(int n) {
   cudaError_t e = cudaSuccess;
-  for (int n : {64, 128, 200, 256, 320, 512, 0}) {  // every length PHGPU_DISPATCH_N instantiates
-    cudaError_t r = cudaSuccess;
-    PHGPU_DISPATCH_N(n, r = so3_attrs<NF>());
-    if (r != cudaSuccess) e = r;
-  }
+  PHGPU_DISPATCH_N(n, e = so3_attrs<NF>());
   if (e == cudaSuccess) e = so3_tc_init_attributes();
   return e;
 }

@@ -18,14 +18,14 @@
 //    half-complex inverse over y, which reads only the real part of the DC and
 //    Nyquist terms), first-occurrence argmax of the signed output.
 //
-// Passes (FP32): A1 r2c along y per row; A2 forward FFT along x per (z, ky
-// tile); B forward FFT along z for all channels of both clouds per (x, ky
-// tile) + fusion + cross power + inverse FFT along z; C1 inverse FFT along x;
-// C2 complex-to-real along y with argmax.  Forward transforms leave x and z in
+// Passes (FP32): sums along y of the rows' occupied voxels (an FFT for grids
+// handed in by the host); forward along x of the z slabs that hold a voxel; forward along z of all channels of both clouds
+// per (x, ky tile) + fusion + cross power + inverse along z; inverse along x;
+// complex-to-real along y with argmax.  Forward transforms leave x and z in
 // digit-reversed order; the inverse transforms consume that order directly.
-#include <cuda.h>  // CUtensorMap (encoded through the runtime's driver entry point)
+#include <algorithm>
 
-#include "fft2.cuh"
+#include "fft_pass.cuh"
 #include "kernels.h"
 
 namespace phgpu {
@@ -103,571 +103,662 @@ cudaError_t launch_voxelize(const VoxelArgs& a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-__global__ void k_clear_voxels(const uint32_t* __restrict__ lin, int n_points, float* __restrict__ grids, size_t nv,
-                               int n_planes, uint8_t* __restrict__ rowlive, int N, const uint32_t* __restrict__ n_dev) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (n_dev ? (int)*n_dev : n_points)) return;
-  const uint32_t l = lin[i];
-  if (l == 0xffffffffu) return;
-  for (int p = 0; p < n_planes; ++p) grids[(size_t)p * nv + l] = 0.0f;
-  if (rowlive) rowlive[l / (uint32_t)N] = 0;
-}
+constexpr int kMaxVoxels = 1024;  // longest transform
 
-cudaError_t launch_clear_voxels(const uint32_t* lin, int n_points, float* grids, size_t nv, int n_planes,
-                                uint8_t* rowlive, int N, cudaStream_t st, const uint32_t* n_dev) {
-  if (n_points > 0) {
-    k_clear_voxels<<<(n_points + 255) / 256, 256, 0, st>>>(lin, n_points, grids, nv, n_planes, rowlive, N, n_dev);
-    count_launches(1);
-  }
-  return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------- A1
-// mean of a voxel: sum / count, 0 for empty voxels (reference: non-finite -> 0)
-__device__ __forceinline__ float voxel_mean(float v, float c) { return c > 0.0f ? v * __frcp_rn(c) : 0.0f; }
-
-constexpr int kRowsR2C = 16;
-
-// rows r = z*N + x of one channel; out spec[ch][r][ky], ky in [0, N/2].
-// A block takes kRowsR2C rows; rows without any point (row flags of the
-// voxeliser) are written as zeros without being read, and the live rows are
-// transformed two at a time as the real and imaginary parts of one complex
-// row, Z = X0 + i X1, separated afterwards by
-//   X0[k] = (Z[k] + conj Z[-k]) / 2,   X1[k] = (Z[k] - conj Z[-k]) / 2i.
-template <int NF>
-__global__ void k_r2c_y(int N, const float* __restrict__ grid, const float* __restrict__ count,
-                        const uint8_t* __restrict__ rowlive, float2* __restrict__ spec, FftPlan plan) {
-  extern __shared__ float2 rows[];  // [kRowsR2C / 2][n] packed rows, then int pos[n]
-  constexpr int R = kRowsR2C;
-  __shared__ int s_slot[R];         // 2 * packed row + part, or -1 for a row without points
-  __shared__ int s_src[R];          // live rows in order
-  __shared__ int s_nlive;
-  const int n = NF > 0 ? NF : N;
-  const int H2 = n / 2 + 1;
-  const int H2p = spatial_h2p(n);
-  int* pos = reinterpret_cast<int*>(rows + (size_t)(R / 2) * n);
-  const size_t nrows = (size_t)n * n;
-  const size_t r0 = (size_t)blockIdx.x * R;
-  if (threadIdx.x < 32) {
-    const int rr = threadIdx.x;
-    const bool live = rr < R && r0 + rr < nrows && (!rowlive || rowlive[r0 + rr]);
-    const unsigned m = __ballot_sync(0xffffffffu, live);
-    const int k = __popc(m & ((1u << rr) - 1u));
-    if (rr < R) s_slot[rr] = live ? k : -1;
-    if (live) s_src[k] = rr;
-    if (rr == 0) s_nlive = __popc(m);
-  }
-  for (int k = threadIdx.x; k < n; k += blockDim.x) pos[k] = freq2pos<NF>(k, plan);
-  __syncthreads();
-  const int nlive = s_nlive;
-  const int npk = (nlive + 1) / 2;
-  for (int e = threadIdx.x; e < npk * n; e += blockDim.x) {
-    const int pk = e / n, y = e - pk * n;
-    float v[2] = {0.f, 0.f};
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int li = 2 * pk + h;
-      if (li < nlive) {
-        const size_t idx = (r0 + s_src[li]) * n + y;
-        v[h] = count ? voxel_mean(grid[idx], count[idx]) : grid[idx];
-      }
-    }
-    rows[e] = make_float2(v[0], v[1]);
-  }
-  __syncthreads();
-  if (npk > 0) fft_any<NF, false>(rows, npk, n, 1, plan);
-  for (int e = threadIdx.x; e < R * H2; e += blockDim.x) {
-    const int rr = e / H2, ky = e - rr * H2;
-    const size_t r = r0 + rr;
-    if (r >= nrows) continue;
-    const int sl = s_slot[rr];
-    float2 X = make_float2(0.f, 0.f);
-    if (sl >= 0) {
-      const float2* Z = rows + (size_t)(sl >> 1) * n;
-      const float2 a = Z[pos[ky]], b = Z[pos[ky == 0 ? 0 : n - ky]];
-      X = (sl & 1) ? make_float2(0.5f * (a.y + b.y), -0.5f * (a.x - b.x))  // (a - conj b) / 2i
-                   : make_float2(0.5f * (a.x + b.x), 0.5f * (a.y - b.y));  // (a + conj b) / 2
-    }
-    spec[r * H2p + ky] = X;
-  }
-}
-
-// ---------------------------------------------------------------- A2 / C1
-// In-place transform along x for a tile of ky at one z: spec[z][x][ky].
-template <int NF, bool INV>
-__global__ void k_fft_x(int N, float2* __restrict__ spec, FftPlan plan) {
-  extern __shared__ float2 tile[];
-  constexpr int Wt = 16;
-  const int n = NF > 0 ? NF : N;
-  const int H2 = n / 2 + 1;
-  const int H2p = spatial_h2p(n);
-  const int ky0 = blockIdx.x * Wt;
-  const int wt = min(Wt, H2 - ky0);
-  float2* base = spec + (size_t)blockIdx.y * n * H2p;
-  for (int e = threadIdx.x; e < n * Wt; e += blockDim.x) {
-    const int x = e / Wt, t = e % Wt;
-    tile[e] = t < wt ? base[(size_t)x * H2p + ky0 + t] : make_float2(0.f, 0.f);
-  }
-  __syncthreads();
-  fft_any<NF, INV, 4>(tile, Wt, 1, Wt, plan);
-  for (int e = threadIdx.x; e < n * Wt; e += blockDim.x) {
-    const int x = e / Wt, t = e % Wt;
-    if (t < wt) base[(size_t)x * H2p + ky0 + t] = tile[e];
-  }
-}
-
-// ---------------------------------------------------------------- B
-// For one x position (digit-reversed) and a tile of ky: forward z FFT of all
-// 2C arrays, fusion + cross power, inverse z FFT of the product.
+// ---------------------------------------------------------------- rows of scans (y)
+// A scan occupies a few voxels per row (N = 200 over a 20 m cube: three to
+// five of 200), so a row's transform along y is summed directly from them,
+//   X[ky] = sum_v mean_v exp(-2 pi i ky y_v / N),
+// instead of an FFT over every row that holds a point: per voxel and 32
+// frequencies one table twiddle (its index, ky y mod N, is exact) and one
+// packed multiply-add per channel.  Rows without a point are neither read nor
+// written: the x transform takes them as zero.
 //
-// The [z][array][ky tile] block arrives by one bulk tensor copy per z chunk
-// (TMA, when the host could encode the tensor map; each box <= 256 z rows)
-// into the same layout the element loader produces.  Dynamic shared memory:
-// tile [zrows][rowlen] float2 | mbarrier (16 B) | fusion bands.
+// Block: kRowsBlock rows of one z-slab; a warp takes a live row, gathers its
+// occupied voxels in order (counts, then every channel's sums, all loads of 256
+// voxels in flight) into shared memory and gives each lane up to four
+// frequencies at a time.  Small blocks spread a slab full of long rows (a floor
+// seen level) over many SMs.  With `clear` the voxels and row flags are zeroed
+// on the way, so a grid that is only transformed needs no memset and no
+// separate pass before its next voxelisation.
+constexpr int kRowsBlock = 16;
+constexpr int kRowsWarps = 4;
 
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// Waits for phase 0 of a shared-memory mbarrier; gives up after a bounded
-// number of polls (returns false).
-__device__ __forceinline__ bool mbar_wait0(uint64_t* bar) {
-  uint32_t done = 0;
-  for (int it = 0; it < (1 << 22) && !done; ++it) {
-    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0; selp.u32 %0, 1, 0, p; }"
-                 : "=r"(done)
-                 : "r"(smem_addr(bar))
-                 : "memory");
-  }
-  return done != 0;
-}
-
-// Channel sums (MEAN) and the first channel of largest energy (MAX) of both
-// sides at one position of a fuse_z tile row: channel c of side f in slot c,
-// of side g in slot C + c.  Odd rows (odd = true) load g before f, which
-// keeps the two loads on different banks (see k_fuse_z).  CC > 0: C == CC
-// known at compile time.
-template <int CC>
-__device__ __forceinline__ void fuse_sides(const float2* row, int C, int Wt, int t, bool odd, float2& sf, float2& sg,
-                                           float2& mf, float2& mg) {
-  if constexpr (CC > 0) C = CC;
-  sf = make_float2(0.f, 0.f);
-  sg = sf;
-  mf = sf;
-  mg = sf;
-  float bf = -1.f, bg = -1.f;
-#pragma unroll
-  for (int c = 0; c < (CC > 0 ? CC : C); ++c) {
-    const float2 p0 = row[(odd ? C + c : c) * Wt + t];
-    const float2 p1 = row[(odd ? c : C + c) * Wt + t];
-    const float2 u = odd ? p1 : p0;
-    const float2 v = odd ? p0 : p1;
-    sf = cadd(sf, u);
-    sg = cadd(sg, v);
-    const float eu = u.x * u.x + u.y * u.y;
-    const float ev = v.x * v.x + v.y * v.y;
-    mf = eu > bf ? u : mf;
-    bf = eu > bf ? eu : bf;
-    mg = ev > bg ? v : mg;
-    bg = ev > bg ? ev : bg;
-  }
-}
-
-struct FuseZTma {
-  int enabled;  // tensor map valid
-  int zbox;     // z rows per copy
-  int chunks;   // copies (zbox * chunks >= N)
+struct ScanRowArgs {
+  int N;
+  float* grids;         // [channel][N^3] sums
+  const float* tw;      // N complex twiddles
+  size_t count_plane;   // offset of the point counts
+  uint8_t* rowlive;     // [N (z)][N (x)] rows that hold a point
+  uint8_t* rowmask;     // [N][N]: the flags again, kept for the x transform
+  float2* spec;         // [channel][z][x][H2p]
+  size_t spec_stride;
+  int clear;
 };
 
-// Two blocks per SM for the compile-time lengths (the bound lets the
-// compiler schedule for it: 0.1294 against 0.1336 ms at N = 200; 640 or 672
-// threads, whose radix passes divide more evenly, ran the same); the runtime
-// plan's generic transform needs its 128 registers.
-// CA, CW > 0: the Laplace fusion of C = CA / 2 channels with tile width CW,
-// known at compile time (every shared-memory offset of the transforms folds
-// to a constant); CA = CW = 0: any shape (the host picks).
-constexpr int kFuseZThreads = 512;
-template <int NF, int CA = 0, int CW = 0>
-__global__ void __launch_bounds__(kFuseZThreads, NF > 0 ? 2 : 1)
-    k_fuse_z(SpatialArgs a, FftPlan plan, int Wt_arg, int x_natural, const __grid_constant__ CUtensorMap tmap,
-             FuseZTma tma) {
-  extern __shared__ __align__(128) float2 tile[];  // [z][arr][t]
-  static_assert(CA == 0 || (NF > 0 && CW == 8 && CA % 2 == 0), "compile-time shape: NF > 0, Wt = 8");
-  const int N = NF > 0 ? NF : a.N;
-  const int H2 = N / 2 + 1;
-  const int H2p = spatial_h2p(N);
-  const int C = CA > 0 ? CA / 2 : a.n_data_ch;
-  const int A = CA > 0 ? CA : (a.laplace ? 2 * C : 2);
-  const int Wt = CW > 0 ? CW : Wt_arg;
-  const int ky0 = blockIdx.x * Wt;
-  const int wt = min(Wt, H2 - ky0);
-  const int xp = blockIdx.y;
-  const size_t plane = (size_t)N * N * H2p;
-  const int rowlen = A * Wt;
-  const int zrows = tma.enabled ? tma.zbox * tma.chunks : N;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(tile + (size_t)zrows * rowlen);
-  FusionBands* s_bands = reinterpret_cast<FusionBands*>(bar + 2);
-  int* s_kz = reinterpret_cast<int*>(s_bands + 1);  // [N] z frequency of each position
-  if (threadIdx.x == 0) *s_bands = a.bands;  // divergent band lookups are cheap in shared memory
-  for (int zp = threadIdx.x; zp < N; zp += kFuseZThreads) s_kz[zp] = pos2freq<NF>(zp, plan);
-  // the bulk copy needs a 128-byte aligned destination (block-uniform test)
-  const bool use_tma = tma.enabled && (smem_addr(tile) & 127u) == 0;
-  if (use_tma) {
-    if (threadIdx.x == 0) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)));
-      asm volatile("fence.mbarrier_init.release.cluster;");
-      asm volatile("fence.proxy.async.shared::cta;");
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const uint32_t bytes = (uint32_t)((size_t)zrows * rowlen * sizeof(float2));
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
-                   : "memory");
-      for (int ch = 0; ch < tma.chunks; ++ch) {
-        const int z0 = ch * tma.zbox;
-        asm volatile(
-            "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-            " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_addr(tile + (size_t)z0 * rowlen)),
-            "l"(&tmap), "r"(ky0), "r"(0), "r"(xp), "r"(z0), "r"(smem_addr(bar))
-            : "memory");
+// Shared memory: N twiddles, then per warp N float4 (means) and N uint16 (y).
+static size_t scan_rows_smem(int N) { return (size_t)N * (8 + kRowsWarps * 18) + 16 * (kRowsWarps + 1); }
+
+template <int CC>
+__global__ void __launch_bounds__(kRowsWarps * 32) k_scan_rows(const ScanRowArgs a) {
+  extern __shared__ __align__(16) float4 s_mem[];
+  constexpr int U = 8, Q = 4;
+  const int n = a.N, H2 = n / 2 + 1, H2p = spatial_h2p(n);
+  const int z = blockIdx.x, x0 = blockIdx.y * kRowsBlock, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const size_t nv = (size_t)n * n * n;
+  const bool mine = lane < kRowsBlock && x0 + lane < n;
+  const bool live_l = mine && a.rowlive[(size_t)z * n + x0 + lane];
+  const unsigned live = __ballot_sync(0xffffffffu, live_l);  // every warp: the block's rows
+  if (warp == 0 && mine) a.rowmask[(size_t)z * n + x0 + lane] = live_l ? 1 : 0;
+  if (!live) return;
+  float4* s_val = s_mem + (size_t)warp * n;
+  float2* s_tw = reinterpret_cast<float2*>(s_mem + (size_t)kRowsWarps * n);
+  uint16_t* s_y = reinterpret_cast<uint16_t*>(s_tw + n) + (size_t)warp * n;
+  for (int i = threadIdx.x; i < n; i += kRowsWarps * 32) s_tw[i] = __ldg(reinterpret_cast<const float2*>(a.tw) + i);
+  __syncthreads();
+  if (a.clear && warp == 0 && live_l) a.rowlive[(size_t)z * n + x0 + lane] = 0;
+  const uint32_t mul = fast_div_mul(n);
+  int seen = 0;
+  for (unsigned todo = live; todo; todo &= todo - 1) {
+    if ((seen++ & (kRowsWarps - 1)) != warp) continue;
+    const size_t row = (size_t)z * n + x0 + __ffs(todo) - 1;
+    float* c = a.grids + a.count_plane + row * n;
+    float* g = a.grids + row * n;
+    int cnt = 0;
+    for (int y0 = 0; y0 < n; y0 += 32 * U) {
+      float q[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) q[u] = y0 + 32 * u + lane < n ? c[y0 + 32 * u + lane] : 0.f;
+      float v[CC][U];
+#pragma unroll
+      for (int ch = 0; ch < CC; ++ch)
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[ch][u] = q[u] > 0.f ? g[ch * nv + y0 + 32 * u + lane] : 0.f;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const bool occ = q[u] > 0.f;
+        const unsigned m = __ballot_sync(0xffffffffu, occ);
+        if (occ) {
+          const int y = y0 + 32 * u + lane, at = cnt + __popc(m & ((1u << lane) - 1u));
+          const float inv = __frcp_rn(q[u]);  // mean = sum * (1 / count)
+          s_y[at] = (uint16_t)y;
+          s_val[at] = make_float4(v[0][u] * inv, CC > 1 ? v[CC > 1 ? 1 : 0][u] * inv : 0.f,
+                                  CC > 2 ? v[CC > 2 ? 2 : 0][u] * inv : 0.f, CC > 3 ? v[CC > 3 ? 3 : 0][u] * inv : 0.f);
+          if (a.clear) {
+            c[y] = 0.f;
+#pragma unroll
+            for (int ch = 0; ch < CC; ++ch) g[ch * nv + y] = 0.f;
+          }
+        }
+        cnt += __popc(m);
       }
     }
-    if (!mbar_wait0(bar)) {
-      if (threadIdx.x == 0) atomicOr(a.status, 1ull);
-      mbar_wait0(bar);  // once more (bounded) so no copy is left in flight
+    __syncwarp();
+    float2* out = a.spec + row * H2p;
+    for (int k0 = 0; k0 < H2; k0 += 32 * Q) {
+      float2 acc[CC][Q];
+#pragma unroll
+      for (int ch = 0; ch < CC; ++ch)
+#pragma unroll
+        for (int i = 0; i < Q; ++i) acc[ch][i] = make_float2(0.f, 0.f);
+#pragma unroll 2
+      for (int e = 0; e < cnt; ++e) {
+        const uint32_t y = s_y[e];
+        const float4 w = s_val[e];
+        const float ws[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int i = 0; i < Q; ++i) {
+          const uint32_t k = (uint32_t)(k0 + 32 * i + lane) * y;
+          const float2 t = s_tw[k - __umulhi(k, mul) * (uint32_t)n];
+#pragma unroll
+          for (int ch = 0; ch < CC; ++ch) acc[ch][i] = __ffma2_rn(make_float2(ws[ch], ws[ch]), t, acc[ch][i]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < Q; ++i) {
+        const int ky = k0 + 32 * i + lane;
+        if (ky < H2) {
+#pragma unroll
+          for (int ch = 0; ch < CC; ++ch) out[ch * a.spec_stride + ky] = acc[ch][i];
+        }
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// ---------------------------------------------------------------- rows (y)
+constexpr int kRowPairs = 16;      // row pairs per block of the forward row transforms
+constexpr int kInvPairs = 16;      // row pairs per block of the inverse row transforms
+// Row stride in shared memory: odd, so threads that take one element of
+// neighbouring rows touch different banks.
+__host__ __device__ constexpr int row_stride(int n) { return n | 1; }
+
+// Real transforms along y of every row of a grid of values (grids handed in
+// by the host; voxelised clouds take the list of occupied voxels instead).
+// Rows are transformed two at a time as the real and imaginary parts of one
+// complex row, Z = X0 + i X1, separated afterwards by
+//   X0[k] = (Z[k] + conj Z[-k]) / 2,   X1[k] = (Z[k] - conj Z[-k]) / 2i.
+template <int NF>
+__global__ void __launch_bounds__(320, NF > 0 ? 3 : 2) k_r2c_rows(int N, const float* __restrict__ grids,
+                                                                  size_t grid_stride, float2* __restrict__ specs,
+                                                                  size_t spec_stride,
+                                                                  const __grid_constant__ FftPlan plan) {
+  extern __shared__ __align__(16) float2 rows[];  // [kRowPairs][st] | float4 cs[] (runtime plans)
+  __shared__ short s_pos[kMaxVoxels];
+  const int n = NF > 0 ? NF : N;
+  const int H2 = n / 2 + 1, H2p = spatial_h2p(n), st = row_stride(n);
+  const int tid = threadIdx.x, nthr = blockDim.x;
+  float4* cs = reinterpret_cast<float4*>(rows + (size_t)kRowPairs * st);
+  const int r0 = blockIdx.x * 2 * kRowPairs;
+  const int rows_here = min(2 * kRowPairs, n * n - r0), np = (rows_here + 1) / 2;
+  const int lwp = 32 - __clz(np - 1);  // columns of the shared stages: the next power of two
+  const float* grid = grids + (size_t)blockIdx.y * grid_stride + (size_t)r0 * n;
+  float2* spec = specs + (size_t)blockIdx.y * spec_stride + (size_t)r0 * H2p;
+  for (int k = tid; k < n; k += nthr) s_pos[k] = (short)freq2pos<NF>(k, plan);
+  auto at = [=](int g, int t, int i, int m) { return SmemCursor{rows + (g + t) * st + i, m, 0}; };
+  auto ld = [=](int g, int t, int i, int m) {
+    const float* p = grid + 2 * (g + t) * n + i;
+    const bool two = 2 * (g + t) + 1 < rows_here;
+    return [=](int, int j) { return make_float2(__ldg(p + j * m), two ? __ldg(p + n + j * m) : 0.f); };
+  };
+  if constexpr (NF > 0) {
+    pass_ct<NF, false, 1, false, 0, 1>(PassMap{np, 0}, plan.tw, tid, nthr, ld, at, at);
+    __syncthreads();
+    pass_ct<NF, false, 1, true, 1, -1>(PassMap{1, lwp}, plan.tw, tid, nthr, at, at, at);
+  } else {
+    pass_rt<false, 1, false>(plan, PassMap{np, 0}, PassMap{1, lwp}, PassMap{1, lwp}, cs, tid, nthr, ld, at, at);
+  }
+  __syncthreads();
+  // separate the rows: one warp per row
+  for (int rr = tid >> 5; rr < rows_here; rr += nthr >> 5) {
+    const float2* Z = rows + (rr >> 1) * st;
+    for (int ky = tid & 31; ky < H2; ky += 32) {
+      const float2 u = Z[s_pos[ky]], v = Z[s_pos[ky == 0 ? 0 : n - ky]];
+      spec[rr * H2p + ky] = (rr & 1) ? make_float2(0.5f * (u.y + v.y), -0.5f * (u.x - v.x))   // (u - conj v) / 2i
+                                     : make_float2(0.5f * (u.x + v.x), 0.5f * (u.y - v.y));  // (u + conj v) / 2
+    }
+  }
+}
+
+// Real inverse over y of 2 kInvPairs consecutive rows with first-occurrence
+// argmax.  A half-complex inverse reads only the real parts of the ky = 0 and
+// ky = N/2 terms, so each row is made exactly Hermitian that way, and rows are
+// inverted two at a time as Z = X0 + i X1 (output x0 = Re, x1 = Im).  The
+// first inverse stage reads the spectrum directly: the R positions it joins
+// hold the frequencies b, b + n/R, ..., so neighbouring threads (b) read
+// neighbouring frequencies; the last stage's outputs go to the argmax without
+// passing through shared memory.
+template <int NF>
+__global__ void __launch_bounds__(320, NF > 0 ? 3 : 2) k_c2r_rows(int N, const float2* __restrict__ cspec, const __grid_constant__ FftPlan plan,
+                                                  unsigned long long* __restrict__ argmax, float* __restrict__ volume,
+                                                  uint32_t limit) {
+  extern __shared__ __align__(16) float2 rows[];  // [kInvPairs][st] | float4 cs[] | int pos[n] (runtime plans)
+  const int n = NF > 0 ? NF : N;
+  const int H2p = spatial_h2p(n), st = row_stride(n);
+  const int tid = threadIdx.x, nthr = blockDim.x;
+  const int nrows = n * n;
+  const int r0 = blockIdx.x * 2 * kInvPairs;
+  const int np = min(kInvPairs, (nrows - r0 + 1) / 2);
+  const int lwp = 32 - __clz(np - 1);
+  auto at = [&](int g, int t, int i, int m) { return SmemCursor{rows + (g + t) * st + i, m, 0}; };
+  // Z at frequency k (mirrored: read at n - k) of a row pair, edge: k = 0 or 2 k = n
+  auto zval = [&](const float2* ca, int k, bool mir, bool edge, bool two) -> float2 {
+    ca += mir ? n - k : k;
+    float2 u = __ldg(ca), v = two ? __ldg(ca + H2p) : make_float2(0.f, 0.f);
+    if (edge) u.y = v.y = 0.f;
+    return mir ? make_float2(u.x + v.y, v.x - u.y)   // conj u + i conj v
+               : make_float2(u.x - v.y, u.y + v.x);  // u + i v
+  };
+  // per thread: the first index of its largest value (NaN compares false; a
+  // thread that saw nothing else keeps its first value)
+  float bv = -INFINITY, fv = 0.f;
+  uint32_t bi = 0xffffffffu, fi = 0xffffffffu;
+  const bool bounded = limit < (uint32_t)nrows * (uint32_t)n;
+  auto take = [&](float v, uint32_t idx) {
+    if (bounded && idx >= limit) return;
+    if (fi == 0xffffffffu) {
+      fi = idx;
+      fv = v;
+    }
+    if (v > bv || (v == bv && idx < bi)) {
+      bv = v;
+      bi = idx;
+    }
+  };
+  auto sv = [&](int g, int t, int y, int m) {
+    const uint32_t idx = (uint32_t)((r0 + 2 * (g + t)) * n + y);
+    const bool two = r0 + 2 * (g + t) + 1 < nrows;
+    return [=, &take](int, int j, float2 v) {
+      take(v.x, idx + j * m);
+      if (two) take(v.y, idx + j * m + n);
+      if (volume) {
+        volume[idx + j * m] = v.x;
+        if (two) volume[idx + j * m + n] = v.y;
+      }
+    };
+  };
+  if constexpr (NF > 0) {
+    constexpr int R = FixedFft<NF>::r[FixedFft<NF>::count - 1];
+    constexpr int nb = NF / R;
+    for (int it = tid; it < np * nb; it += nthr) {
+      const int pk = it / nb, b = it - pk * nb;
+      const float2* ca = cspec + (size_t)(r0 + 2 * pk) * H2p;
+      float2 x[R];
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        // NF is even: whole runs of b lie on one side of the Nyquist term
+        const bool below = 2 * (i * nb + nb - 1) < NF, above = 2 * i * nb > NF;
+        const int k = b + i * nb;
+        const bool mir = above || (!below && 2 * k > NF);
+        x[i] = zval(ca, k, mir, (i == 0 && b == 0) || (!below && !above && 2 * k == NF), true);
+      }
+      dft_small<R, true>(x);
+      float2* d = rows + pk * st + fixed_freq2pos<NF>(b);
+#pragma unroll
+      for (int i = 0; i < R; ++i) d[i] = x[i];
+    }
+    __syncthreads();
+    constexpr int cnt = FixedFft<NF>::count;
+    pass_ct<NF, true, 1, true, 1, cnt - 1>(PassMap{1, lwp}, plan.tw, tid, nthr, at, at, sv);
+    if constexpr (cnt > 2) __syncthreads();
+    if (volume || bounded) {
+      pass_ct<NF, true, 1, false, cnt - 1, -1>(PassMap{np, 0}, plan.tw, tid, nthr, at, at, sv);
+    } else {
+      // A thread's items lie in increasing row pairs (nthr >= the butterflies
+      // of a row), and an item's values are taken in increasing index: the
+      // first of equal values is the one met first.
+      constexpr int R0 = FixedFft<NF>::r[0], m = NF / R0;
+      static_assert(m <= 128, "a block has at least 128 threads");
+      for (int it = tid; it < np * m; it += nthr) {
+        const int pk = it / m, j2 = it - pk * m;
+        const float2* row = rows + pk * st + j2;
+        float2 x[R0];
+#pragma unroll
+        for (int j = 0; j < R0; ++j) x[j] = row[j * m];
+#pragma unroll
+        for (int k = 1; k < R0; ++k) x[k] = cmul(x[k], cconj(__ldg(plan.tw + j2 * k)));
+        dft_small<R0, true>(x);
+        const uint32_t idx = (uint32_t)((r0 + 2 * pk) * NF + j2);
+        if (fi == 0xffffffffu) {
+          fi = idx;
+          fv = x[0].x;
+        }
+#pragma unroll
+        for (int j = 0; j < R0; ++j)
+          if (x[j].x > bv) {
+            bv = x[j].x;
+            bi = idx + j * m;
+          }
+#pragma unroll
+        for (int j = 0; j < R0; ++j)
+          if (x[j].y > bv) {
+            bv = x[j].y;
+            bi = idx + NF + j * m;
+          }
+      }
     }
   } else {
-    // tiles start at ky0 (multiple of Wt) in rows padded to 8 complex: load two
-    // complex per 16-byte access
-    const int half = Wt >> 1;
-    for (int e = threadIdx.x; e < N * A * half; e += kFuseZThreads) {
-      const int z = e / (A * half), rem = e - z * (A * half), ar = rem / half, t2 = rem - ar * half;
-      // arrays: f channels 0..C-1 then g channels; plain mode uses channel 0 of
-      // each side, the low-pass mode channel 1
-      const int src = a.laplace ? ar : (ar == 0 ? a.lowpass : C + a.lowpass);
-      const float4 v = *reinterpret_cast<const float4*>(
-          a.spec + (size_t)src * plane + ((size_t)z * N + xp) * H2p + ky0 + 2 * t2);
-      float2* d = tile + (size_t)z * rowlen + ar * Wt + 2 * t2;
-      d[0] = make_float2(v.x, v.y);
-      d[1] = make_float2(v.z, v.w);
+    float4* cs = reinterpret_cast<float4*>(rows + (size_t)kInvPairs * st);
+    int* pos = reinterpret_cast<int*>(cs + kMaxGenericRadix);
+    for (int k = tid; k < n; k += nthr) pos[k] = freq2pos<NF>(k, plan);
+    __syncthreads();
+    for (int pk = tid >> 5; pk < np; pk += nthr >> 5) {
+      const float2* ca = cspec + (size_t)(r0 + 2 * pk) * H2p;
+      const bool two = r0 + 2 * pk + 1 < nrows;
+      for (int k = tid & 31; k < n; k += 32) rows[pk * st + pos[k]] = zval(ca, k, 2 * k > n, k == 0 || 2 * k == n, two);
+    }
+    __syncthreads();
+    pass_rt<true, 1, true>(plan, PassMap{1, lwp}, PassMap{1, lwp}, PassMap{np, 0}, cs, tid, nthr, at, at, sv);
+  }
+  if (bi == 0xffffffffu) {
+    bi = fi;
+    bv = fv;
+  }
+  // + 0: a negative zero orders as zero
+  warp_argmax_commit(bi == 0xffffffffu ? 0ull : pack_argmax(bv + 0.0f, bi), argmax);
+}
+
+// ---------------------------------------------------------------- columns (x)
+struct ColArgs {
+  int N;
+  float2* spec;  // [channel][z][x][H2p]
+  size_t spec_stride;
+  const uint8_t* rowmask;  // forward: [N (z)][N (x)] rows that hold a voxel, the others are taken as zero; null: all
+  uint8_t* slab_live;      // forward: [N] set to whether any row of the slab holds a voxel
+  int write_empty;         // forward: empty slabs are written as zeros (else left alone)
+  FftPlan plan;
+};
+
+// In-place transform along x of a tile of 2^LW ky columns at one z of CC
+// arrays (forward: every channel of a side, which share the row flags, the
+// index arithmetic and the twiddles).  Forward: x natural in, digit-reversed
+// out; inverse: the reverse.  The first stage reads and the last stage writes
+// global memory directly.  Slabs without a voxel are left alone: the z pass
+// does not read them.
+constexpr int kXThreads = 320;
+template <int NF, bool INV, int CC, int LW>
+__global__ void __launch_bounds__(kXThreads, NF > 0 ? 4 : 2) k_fft_x(const __grid_constant__ ColArgs a) {
+  extern __shared__ __align__(16) float2 tile[];  // [CC][n][W] | float4 cs[] (runtime plans) | uint8 live[n]
+  __shared__ uint16_t s_mask[(INV || NF == 0) ? 1 : NF / 2];
+  constexpr int W = 1 << LW;
+  const int n = NF > 0 ? NF : a.N;
+  const int H2 = n / 2 + 1, H2p = spatial_h2p(n);
+  const int tid = threadIdx.x, nthr = blockDim.x;
+  const int z = blockIdx.y, ky0 = blockIdx.x * W, wt = min(W, H2 - ky0);
+  const int slot = n * W;
+  float4* cs = reinterpret_cast<float4*>(tile + (size_t)CC * slot);
+  uint8_t* s_live = reinterpret_cast<uint8_t*>(cs + (NF > 0 ? 0 : kMaxGenericRadix));
+  const size_t stride = a.spec_stride;
+  if constexpr (!INV) {
+    int any = 0;
+    for (int x = tid; x < n; x += nthr) {
+      const uint8_t f = a.rowmask ? a.rowmask[(size_t)z * n + x] : 1;
+      s_live[x] = f;
+      any |= f;
+    }
+    any = __syncthreads_or(any);
+    if (blockIdx.x == 0 && tid == 0) a.slab_live[z] = any ? 1 : 0;
+    if (!any && !a.write_empty) return;
+  }
+  float2* base = a.spec + (size_t)z * n * H2p + ky0;
+  auto at = [=](int, int t, int i, int m) { return SmemCursor{tile + i * W + t, m * W, slot}; };
+  auto sv = [=](int, int t, int i, int m) {
+    float2* p = base + i * H2p + t;
+    const bool ok = t < wt;
+    const int js = m * H2p;
+    return [=](int c, int j, float2 v) {
+      if (ok) p[c * stride + j * js] = v;
+    };
+  };
+  const PassMap map{1, LW};
+  if constexpr (NF > 0 && !INV) {
+    // which of the R rows of each first-stage butterfly are live
+    constexpr int R = FixedFft<NF>::r[0], m0 = NF / R;
+    for (int i = tid; i < m0; i += nthr) {
+      unsigned k = 0;
+#pragma unroll
+      for (int j = 0; j < R; ++j) k |= (s_live[i + j * m0] ? 1u : 0u) << j;
+      s_mask[i] = (uint16_t)k;
+    }
+    __syncthreads();
+    const uint16_t* mask = s_mask;
+    auto ld = [=](int, int t, int i, int m) {
+      const float2* p = base + i * H2p + t;
+      const unsigned k = t < wt ? mask[i] : 0u;
+      const int js = m * H2p;
+      return [=](int c, int j) { return (k >> j) & 1u ? p[c * stride + j * js] : make_float2(0.f, 0.f); };
+    };
+    pass_ct<NF, false, CC, true, 0, -1>(map, a.plan.tw, tid, nthr, ld, at, sv);
+  } else {
+    auto ld = [=](int, int t, int i, int m) {
+      const float2* p = base + i * H2p + t;
+      const bool ok = t < wt;
+      const int js = m * H2p;
+      const uint8_t* l = s_live + i;
+      return [=](int c, int j) {
+        bool take = ok;
+        if constexpr (!INV) take = take && l[j * m];
+        return take ? p[c * stride + j * js] : make_float2(0.f, 0.f);
+      };
+    };
+    if constexpr (NF > 0)
+      pass_ct<NF, true, CC, true, 0, -1>(map, a.plan.tw, tid, nthr, ld, at, sv);
+    else
+      pass_rt<INV, CC, false>(a.plan, map, map, map, cs, tid, nthr, ld, at, sv);
+  }
+}
+
+// ---------------------------------------------------------------- z, fusion
+// For one x position (digit-reversed) and a tile of ky: forward z transform of
+// all channels of both clouds, channel fusion, cross power and the inverse z
+// transform of the product.
+//
+// The sides follow one another through one set of C channel slots (slot C
+// holds the fused target, then the product), so a block of 3 channels keeps
+// 4 n W complex values rather than 6, and four blocks fit on an SM at N = 200.
+// With a compile-time plan the last forward stage, the fusion and the first
+// inverse stage run in registers: the last stage of a forward transform and
+// the first of an inverse one join the same R neighbouring positions, so a
+// thread transforms its R positions of every channel, keeps the running
+// fusion, and hands the product to the inverse butterfly without a shared
+// round trip.  Slabs without a point (slab_live) are not read.
+
+// Where the fusion rule is one rule over a run of positions [p0, p1]: no band
+// edge lies in (p0, p1].
+__device__ __forceinline__ bool fusion_uniform(uint32_t p0, uint32_t p1, const FusionBands& b) {
+  uint32_t off = 0;
+  bool same = p0 <= p1;
+  for (int l = 0; l < b.levels; ++l) {
+    const uint32_t e0 = off + b.lb[l], e1 = off + b.eub[l], e2 = off + b.sub[l];
+    same = same && !(p0 < e0 && e0 <= p1) && !(p0 < e1 && e1 <= p1) && !(p0 < e2 && e2 <= p1);
+    off = e0;
+  }
+  return same;
+}
+
+constexpr int kFuseMixed = 3;  // the rule varies over the tile's ky at this position
+
+// Shared-memory element of position i: one extra column group after every
+// R_last positions when R_last is even, so the butterflies of neighbouring
+// position groups start on different banks.
+template <int NF>
+__host__ __device__ constexpr int z_pad() {
+  if constexpr (NF > 0) {
+    constexpr int R = FixedFft<NF>::r[FixedFft<NF>::count - 1];
+    return R % 2 == 0 ? R : 0;
+  } else {
+    return 0;
+  }
+}
+template <int NF>
+__host__ __device__ constexpr int z_off(int i) {
+  if constexpr (z_pad<NF>() > 0)
+    return i + i / z_pad<NF>();
+  else
+    return i;
+}
+
+constexpr int kFuseZMaxThreads = 320;
+// LW >= 0: the tile is 2^LW columns wide; LW < 0: 2^lw_arg.
+template <int NF, int CC, int LW>
+__global__ void __launch_bounds__(kFuseZMaxThreads, NF > 0 ? 4 : 1) k_fuse_z(const __grid_constant__ SpatialArgs a, const __grid_constant__ FftPlan plan, int lw_arg) {
+  // [CC + 1][z_off(n)][W] | float4 cs[] (runtime plans) | int16 kz[n], uint16 mask[n], uint8 live[2 n], op[n], gop[n]
+  extern __shared__ __align__(16) float2 tile[];
+  __shared__ FusionBands s_bands;
+  const int n = NF > 0 ? NF : a.N;
+  const int H2 = n / 2 + 1, H2p = spatial_h2p(n);
+  const int lw = LW >= 0 ? LW : lw_arg;
+  const int W = 1 << lw;
+  const int tid = threadIdx.x, nthr = blockDim.x;
+  const int ky0 = blockIdx.x * W, wt = min(W, H2 - ky0);
+  const int xp = blockIdx.y;
+  const size_t plane = (size_t)n * n * H2p;
+  const int slot = z_off<NF>(n) * W;
+  const int kx = pos2freq<NF>(xp, plan);
+  const uint32_t nv = (uint32_t)n * n * n;
+  float4* cs = reinterpret_cast<float4*>(tile + (size_t)(CC + 1) * slot);
+  short* s_kz = reinterpret_cast<short*>(cs + (NF > 0 ? 0 : kMaxGenericRadix));
+  uint16_t* s_mask = reinterpret_cast<uint16_t*>(s_kz + n);
+  uint8_t* s_live = reinterpret_cast<uint8_t*>(s_mask + n);
+  uint8_t *s_op = s_live + 2 * n, *s_gop = s_op + n;
+  if (tid == 0) s_bands = a.bands;
+  // the inverse that follows on the stream finds an empty argmax
+  if (tid == 0 && blockIdx.x == 0 && blockIdx.y == 0) *a.argmax = 0ull;
+  constexpr int R = NF > 0 ? FixedFft<NF == 0 ? 64 : NF>::r[FixedFft<NF == 0 ? 64 : NF>::count - 1] : 1;
+  for (int g = tid; g < n / R; g += nthr) s_gop[g] = 0;
+  __syncthreads();
+  auto shifted = [&](int kz, int t) -> uint32_t {  // (klin + nv / 2) mod nv with klin < nv
+    const uint32_t klin = ((uint32_t)kz * n + (uint32_t)kx) * (uint32_t)H2 + (uint32_t)(ky0 + t);
+    uint32_t p = klin + (nv >> 1);
+    if (p >= nv || p < klin) p -= nv;
+    return p;
+  };
+  for (int zp = tid; zp < n; zp += nthr) {
+    const int kz = pos2freq<NF>(zp, plan);
+    s_kz[zp] = (short)kz;
+    s_live[zp] = a.slab_live[zp];
+    s_live[n + zp] = a.slab_live[n + zp];
+    if (a.laplace) {
+      const uint32_t p0 = shifted(kz, 0), p1 = shifted(kz, wt - 1);
+      const int op = fusion_uniform(p0, p1, s_bands) ? fusion_op(p0, s_bands) : kFuseMixed;
+      s_op[zp] = (uint8_t)op;
+      if (op != kFuseMax) s_gop[zp / R] = 1;
     }
   }
   __syncthreads();
-  if constexpr (CA > 0)
-    fixed_cols_ct<NF, false, CA * CW, CA * CW, kFuseZThreads, false>(tile, plan.tw, 0);
-  else
-    fft_any_cols<NF, false>(tile, rowlen, rowlen, plan);
-  const int kx = x_natural ? xp : pos2freq<NF>(xp, plan);
-  const uint32_t nv = (uint32_t)N * (uint32_t)N * (uint32_t)N;
+  if constexpr (NF > 0) {
+    // which of the R slabs of each first-stage butterfly are live
+    constexpr int R0 = FixedFft<NF>::r[0], m0 = NF / R0;
+    for (int i = tid; i < 2 * m0; i += nthr) {
+      const uint8_t* l = s_live + (i < m0 ? i : n + i - m0);
+      unsigned k = 0;
+#pragma unroll
+      for (int j = 0; j < R0; ++j) k |= (l[j * m0] ? 1u : 0u) << j;
+      s_mask[i] = (uint16_t)k;
+    }
+    __syncthreads();
+  }
   // MEAN divides by the total channel count: a product with the reciprocal,
   // exact for the reference's 4 channels (within one rounding otherwise)
   const float inv_total = 1.0f / (float)a.n_total_ch;
-  // Wt is a power of two (fuse_z_tile_ok): shifts, not a runtime division per element
-  const int lwt = __ffs(Wt) - 1;
-  // With Wt = 8 a half-warp covers two rows whose slots start on the same
-  // banks (a row is A * 64 bytes): odd rows load their two sides in the
-  // opposite order (conflict-free when the slots of a channel's sides are an
-  // odd number of slots apart) and keep the product in slot 1 instead of 0,
-  // which the inverse transform and the store follow.
-  const int podd = (NF > 0 && Wt == 8) ? Wt : 0;
-  for (int e = threadIdx.x; e < N * Wt; e += kFuseZThreads) {
-    const int zp = e >> lwt, t = e & (Wt - 1);
-    const bool odd = podd && (zp & 1);
-    float2* row = tile + (size_t)zp * rowlen;
-    float2 F, G;
-    if (CA == 0 && !a.laplace) {
-      const float2 p0 = row[(odd ? Wt : 0) + t], p1 = row[(odd ? 0 : Wt) + t];
-      F = odd ? p1 : p0;
-      G = odd ? p0 : p1;
-      if (a.lowpass) {
-        // keep the products whose FFT-shifted index p = (i N + j) + N^2 k has
-        // i, j, k in [lp_lo, lp_hi]
-        const int kz = s_kz[zp];
-        const uint32_t klin = ((uint32_t)kz * N + (uint32_t)kx) * (uint32_t)H2 + (uint32_t)(ky0 + t);
-        uint32_t p = klin + (nv >> 1);
-        if (p >= nv || p < klin) p -= nv;
-        const uint32_t n2 = (uint32_t)N * (uint32_t)N, kk = p / n2, rem = p - kk * n2;
-        const uint32_t ii = rem / (uint32_t)N, jj = rem - ii * (uint32_t)N;
-        if (ii < a.lp_lo || ii > a.lp_hi || jj < a.lp_lo || jj > a.lp_hi || kk < a.lp_lo || kk > a.lp_hi) {
-          F = make_float2(0.f, 0.f);
-          G = F;
+  auto val = [&](int c, int t, int i) -> float2& { return tile[c * slot + z_off<NF>(i) * W + t]; };
+  // z_off(r0 + j m) is linear in j: m is a multiple of the pad's period, or m = 1 within one period
+  auto at = [=](int c, int t, int i, int m) {
+    return SmemCursor{tile + c * slot + z_off<NF>(i) * W + t, (m == 1 ? 1 : z_off<NF>(m)) * W, slot};
+  };
+  // low-pass: keep the products whose FFT-shifted index p = (i N + j) + N^2 k
+  // has i, j, k in [lp_lo, lp_hi]
+  auto passed = [&](int i, int t) -> bool {
+    if (!a.lowpass) return true;
+    const uint32_t p = shifted(s_kz[i], t), n2 = (uint32_t)n * (uint32_t)n, kk = p / n2, rem = p - kk * n2;
+    const uint32_t ii = rem / (uint32_t)n, jj = rem - ii * (uint32_t)n;
+    return !(ii < a.lp_lo || ii > a.lp_hi || jj < a.lp_lo || jj > a.lp_hi || kk < a.lp_lo || kk > a.lp_hi);
+  };
+  // the fused value at a position whose channels are in the slots
+  auto fused_at = [&](int t, int i) -> float2 {
+    if (!a.laplace) return passed(i, t) ? val(0, t, i) : make_float2(0.f, 0.f);
+    int op = s_op[i];
+    if (op == kFuseMixed) op = fusion_op(shifted(s_kz[i], t), s_bands);
+    float2 sum = make_float2(0.f, 0.f), mx = sum;
+    float best = -1.f;
+#pragma unroll
+    for (int c = 0; c < CC; ++c) {
+      const float2 u = val(c, t, i);
+      sum = cadd(sum, u);
+      const float e = u.x * u.x + u.y * u.y;
+      mx = e > best ? u : mx;
+      best = e > best ? e : best;
+    }
+    return op == kFuseMax ? mx
+                          : (op == kFuseMean ? make_float2(sum.x * inv_total, sum.y * inv_total) : make_float2(0.f, 0.f));
+  };
+  // complexMulSeq: C = F * conj(G)
+  auto cross = [](float2 F, float2 G) { return make_float2(F.x * G.x - F.y * (-G.y), F.x * (-G.y) + F.y * G.x); };
+  for (int side = 0; side < 2; ++side) {
+    // plain correlation: channel 0 of each side, low-pass: channel 1
+    const float2* src = a.spec + (size_t)(side * a.n_data_ch + (a.laplace ? 0 : a.lowpass)) * plane +
+                        (size_t)xp * H2p + ky0;
+    const int zs = n * H2p;
+    if constexpr (NF > 0) {
+      constexpr int cnt = FixedFft<NF>::count;
+      const uint16_t* mask = s_mask + side * (NF / FixedFft<NF>::r[0]);
+      auto ld = [=](int, int t, int i, int m) {
+        const float2* p = src + (size_t)i * zs + t;
+        const unsigned k = t < wt ? mask[i] : 0u;
+        const size_t js = (size_t)m * zs;
+        return [=](int c, int j) { return (k >> j) & 1u ? __ldg(p + c * plane + j * js) : make_float2(0.f, 0.f); };
+      };
+      pass_ct<NF, false, CC, true, 0, cnt - 1>(PassMap{1, lw}, plan.tw, tid, nthr, ld, at, at);
+      __syncthreads();
+      for (int it = tid; it < (n / R) << lw; it += nthr) {
+        const int t = it & (W - 1), g = it >> lw, i0 = g * R;
+        float2 F[R];
+        float2* row = tile + z_off<NF>(i0) * W + t;
+        if (!a.laplace || s_gop[g]) {
+          // rare: rules other than the maximum near the spectrum's centre, or the plain and low-pass modes
+#pragma unroll 1
+          for (int c = 0; c < CC; ++c) {
+            float2 x[R];
+#pragma unroll
+            for (int j = 0; j < R; ++j) x[j] = row[c * slot + j * W];
+            dft_small<R, false>(x);
+#pragma unroll
+            for (int j = 0; j < R; ++j) row[c * slot + j * W] = x[j];
+          }
+#pragma unroll
+          for (int j = 0; j < R; ++j) F[j] = fused_at(t, i0 + j);
+        } else {
+          // the first channel of largest energy
+          float best[R];
+#pragma unroll
+          for (int j = 0; j < R; ++j) {
+            F[j] = make_float2(0.f, 0.f);
+            best[j] = -1.f;
+          }
+#pragma unroll
+          for (int c = 0; c < CC; ++c) {
+            float2 x[R];
+#pragma unroll
+            for (int j = 0; j < R; ++j) x[j] = row[c * slot + j * W];
+            dft_small<R, false>(x);
+#pragma unroll
+            for (int j = 0; j < R; ++j) {
+              const float e = x[j].x * x[j].x + x[j].y * x[j].y;
+              F[j] = e > best[j] ? x[j] : F[j];
+              best[j] = e > best[j] ? e : best[j];
+            }
+          }
         }
+        row += CC * slot;
+        if (side == 1) {
+          float2 x[R];
+#pragma unroll
+          for (int j = 0; j < R; ++j) x[j] = cross(row[j * W], F[j]);
+          dft_small<R, true>(x);
+#pragma unroll
+          for (int j = 0; j < R; ++j) F[j] = x[j];
+        }
+#pragma unroll
+        for (int j = 0; j < R; ++j) row[j * W] = F[j];
       }
     } else {
-      const int kz = s_kz[zp];
-      const uint32_t klin = ((uint32_t)kz * N + (uint32_t)kx) * (uint32_t)H2 + (uint32_t)(ky0 + t);
-      // (klin + nv/2) mod nv with klin < nv
-      uint32_t p = klin + (nv >> 1);
-      if (p >= nv || p < klin) p -= nv;
-      const int op = fusion_op(p, *s_bands);
-      // one branch-free pass serves every rule (a divergent switch between
-      // the rules cost more than the arithmetic): channel sums for MEAN, the
-      // first channel of largest energy for MAX
-      float2 sf, sg, mf, mg;
-      if constexpr (CA > 0)
-        fuse_sides<CA / 2>(row, C, Wt, t, odd, sf, sg, mf, mg);
-      else if (C == 3)  // range, intensity, reflectivity: the loop unrolled
-        fuse_sides<3>(row, 3, Wt, t, odd, sf, sg, mf, mg);
-      else
-        fuse_sides<0>(row, C, Wt, t, odd, sf, sg, mf, mg);
-      const float inv = inv_total;
-      F = op == kFuseMax ? mf : (op == kFuseMean ? make_float2(sf.x * inv, sf.y * inv) : make_float2(0.f, 0.f));
-      G = op == kFuseMax ? mg : (op == kFuseMean ? make_float2(sg.x * inv, sg.y * inv) : make_float2(0.f, 0.f));
+      const PassMap map{1, lw};
+      const uint8_t* live = s_live + side * n;
+      auto ld = [=](int, int t, int i, int m) {
+        const float2* p = src + (size_t)i * zs + t;
+        const bool ok = t < wt;
+        const size_t js = (size_t)m * zs;
+        const uint8_t* l = live + i;
+        return [=](int c, int j) { return ok && l[j * m] ? __ldg(p + c * plane + j * js) : make_float2(0.f, 0.f); };
+      };
+      pass_rt<false, CC, false>(plan, map, map, map, cs, tid, nthr, ld, at, at);
+      __syncthreads();
+      for (int it = tid; it < n << lw; it += nthr) {
+        const int t = it & (W - 1), i = it >> lw;
+        const float2 v = fused_at(t, i);
+        float2& o = val(CC, t, i);
+        o = side == 0 ? v : cross(o, v);
+      }
     }
-    // complexMulSeq: C = F * conj(G); only this thread touches position (zp, t)
-    row[(odd ? Wt : 0) + t] = make_float2(F.x * G.x - F.y * (-G.y), F.x * (-G.y) + F.y * G.x);
+    __syncthreads();
   }
-  __syncthreads();
-  if constexpr (CA > 0) {
-    fixed_cols_ct<NF, true, CW, CA * CW, kFuseZThreads, true>(tile, plan.tw, CW);
-  } else if constexpr (NF > 0) {
-    if (podd)
-      fft_fixed_cols_podd<NF, true>(tile, Wt, rowlen, podd, plan.tw);
-    else
-      fft_any_cols<NF, true>(tile, Wt, rowlen, plan);
+  float2* dst = a.cspec + (size_t)xp * H2p + ky0;
+  auto pat = [=](int, int t, int i, int m) { return at(CC, t, i, m); };
+  auto sv = [=](int, int t, int i, int m) {
+    float2* p = dst + (size_t)i * n * H2p + t;
+    const bool ok = t < wt;
+    const size_t js = (size_t)m * n * H2p;
+    return [=](int, int j, float2 v) {
+      if (ok) p[j * js] = v;
+    };
+  };
+  if constexpr (NF > 0) {
+    pass_ct<NF, true, 1, true, 1, -1>(PassMap{1, lw}, plan.tw, tid, nthr, pat, pat, sv);
   } else {
-    fft_any_cols<NF, true>(tile, Wt, rowlen, plan);
+    const PassMap map{1, lw};
+    pass_rt<true, 1, true>(plan, map, map, map, cs, tid, nthr, pat, pat, sv);
   }
-  for (int e = threadIdx.x; e < N * Wt; e += kFuseZThreads) {
-    const int z = e >> lwt, t = e & (Wt - 1);
-    if (t < wt) a.cspec[((size_t)z * N + xp) * H2p + ky0 + t] = tile[(size_t)z * rowlen + ((z & 1) ? podd : 0) + t];
-  }
-}
-
-// ---------------------------------------------------------------- C2
-// Real inverse over y of kRowsR2C rows with first-occurrence argmax.  A
-// half-complex inverse reads only the real parts of the ky = 0 and ky = N/2
-// terms, so each row is made exactly Hermitian that way, and rows are
-// inverted two at a time as Z = X0 + i X1 (output x0 = Re, x1 = Im).
-template <int NF>
-__global__ void k_c2r_y(int N, const float2* __restrict__ cspec, FftPlan plan,
-                        unsigned long long* __restrict__ argmax, float* __restrict__ volume, uint32_t limit) {
-  extern __shared__ float2 rows[];  // [kRowsR2C / 2][n] packed rows, then int pos[n]
-  constexpr int R = kRowsR2C;
-  const int n = NF > 0 ? NF : N;
-  const int H2 = n / 2 + 1;
-  const int H2p = spatial_h2p(n);
-  int* pos = reinterpret_cast<int*>(rows + (size_t)(R / 2) * n);
-  const size_t nrows = (size_t)n * n;
-  const size_t r0 = (size_t)blockIdx.x * R;
-  for (int k = threadIdx.x; k < n; k += blockDim.x) pos[k] = freq2pos<NF>(k, plan);
-  __syncthreads();
-  const int hmax = (n - 1) / 2;  // last ky with a mirrored partner
-  for (int e = threadIdx.x; e < (R / 2) * H2; e += blockDim.x) {
-    const int pk = e / H2, ky = e - pk * H2;
-    const size_t ra = r0 + 2 * pk, rb = ra + 1;
-    float2 a = ra < nrows ? cspec[ra * H2p + ky] : make_float2(0.f, 0.f);
-    float2 b = rb < nrows ? cspec[rb * H2p + ky] : make_float2(0.f, 0.f);
-    if (ky == 0 || 2 * ky == n) {
-      a.y = 0.f;
-      b.y = 0.f;
-    }
-    float2* Z = rows + (size_t)pk * n;
-    Z[pos[ky]] = make_float2(a.x - b.y, a.y + b.x);                                // a + i b
-    if (ky >= 1 && ky <= hmax) Z[pos[n - ky]] = make_float2(a.x + b.y, b.x - a.y);  // conj a + i conj b
-  }
-  __syncthreads();
-  fft_any<NF, true>(rows, R / 2, n, 1, plan);
-  unsigned long long best = 0ull;
-  for (int e = threadIdx.x; e < R * n; e += blockDim.x) {
-    const int rr = e / n, y = e - rr * n;
-    const size_t r = r0 + rr;
-    if (r < nrows) {
-      const float2 z = rows[(size_t)(rr >> 1) * n + y];
-      const float v = (rr & 1) ? z.y : z.x;
-      const uint32_t idx = (uint32_t)(r * n + y);
-      const unsigned long long key = idx < limit ? pack_argmax(v, idx) : 0ull;
-      best = key > best ? key : best;
-      if (volume) volume[idx] = v;
-    }
-  }
-  warp_argmax_commit(best, argmax);
-}
-
-// ---------------------------------------------------------------- z-slab
-// Fused forward r2c over (x, y) of one z-slab of one channel (NF even, the
-// slab of NF/2 x NF complex fits in shared memory).  Rows x = 2r and 2r+1 are
-// packed as real and imaginary parts of one complex row; FFT over y (NF
-// points), FFT over r (NF/2 points), then the two real spectra are separated
-// in the 2-D frequency domain,
-//   A = (W[ky][k] + conj W[-ky][-k]) / 2,  B = (W[ky][k] - conj W[-ky][-k]) / 2i,
-// and combined over the even/odd x split,
-//   X[k][ky] = A + w_N^k B,  X[k + N/2][ky] = A - w_N^k B.
-// Output rows are in natural kx order.  Shared rows have the odd stride N + 1.
-
-
-template <int NF>
-__global__ void __launch_bounds__(tail_threads<NF>()) k_slab_fwd(const float* __restrict__ grids, size_t grid_cstride,
-                                                   const float* __restrict__ count,
-                                                   const uint8_t* __restrict__ rowlive, float2* __restrict__ spec,
-                                                   size_t spec_cstride, FftPlan pN, FftPlan pH,
-                                                   uint8_t* __restrict__ slab_nz) {
-  constexpr int N = NF, NH = NF / 2, H2 = NF / 2 + 1, Q = NF / 4, S = NF + 1;
-  constexpr int T = tail_threads<NF>();  // the launch's block size
-  const int H2p = spatial_h2p(N);
-  extern __shared__ float2 W[];  // [NH][S]
-  __shared__ int s_flag[NH];      // packed row r may hold a point (row flags), else all zero
-  __shared__ int s_live[NH];      // packed row r holds a non-zero value
-  __shared__ int s_rows[NH];      // compact list of those rows
-  __shared__ int s_nrows;
-  __shared__ int s_posN[N], s_posH[NH];  // digit-reversed positions of frequencies
-  const int z = blockIdx.x, c = blockIdx.y;
-  const float* g = grids + (size_t)c * grid_cstride + (size_t)z * N * N;
-  const float* cnt = count ? count + (size_t)z * N * N : nullptr;
-  // slab_nz[c][z]: 0 when this slab of spectrum array c is known to hold zeros
-  uint8_t* nz = slab_nz ? slab_nz + (size_t)c * N + z : nullptr;
-  const int held_nonzero = nz ? *nz : 1;
-  int any_flag = 0;
-  for (int r = threadIdx.x; r < NH; r += T) {
-    s_live[r] = 0;
-    s_flag[r] = rowlive ? (rowlive[z * N + 2 * r] | rowlive[z * N + 2 * r + 1]) : 1;
-    any_flag |= s_flag[r];
-  }
-  // a slab without a flagged row transforms to zero: nothing to do where the
-  // array already holds zeros there (about half the slabs of a room scan, so
-  // they leave before any other set-up)
-  if (!__syncthreads_or(any_flag) && !held_nonzero) return;
-  for (int r = threadIdx.x; r < NH; r += T) s_posH[r] = fixed_freq2pos<NH>(r);
-  for (int k = threadIdx.x; k < N; k += T) s_posN[k] = fixed_freq2pos<N>(k);
-  for (int e = threadIdx.x; e < NH * Q; e += T) {
-    const int r = e / Q, y4 = (e - r * Q) * 4;
-    if (!s_flag[r]) {  // no point in either row: skip the loads
-      float2* d = W + r * S + y4;
-      d[0] = d[1] = d[2] = d[3] = make_float2(0.f, 0.f);
-      continue;
-    }
-    float4 a = *reinterpret_cast<const float4*>(g + (size_t)(2 * r) * N + y4);
-    float4 b = *reinterpret_cast<const float4*>(g + (size_t)(2 * r + 1) * N + y4);
-    if (cnt) {
-      const float4 ca = *reinterpret_cast<const float4*>(cnt + (size_t)(2 * r) * N + y4);
-      const float4 cb = *reinterpret_cast<const float4*>(cnt + (size_t)(2 * r + 1) * N + y4);
-      a = make_float4(voxel_mean(a.x, ca.x), voxel_mean(a.y, ca.y), voxel_mean(a.z, ca.z), voxel_mean(a.w, ca.w));
-      b = make_float4(voxel_mean(b.x, cb.x), voxel_mean(b.y, cb.y), voxel_mean(b.z, cb.z), voxel_mean(b.w, cb.w));
-    }
-    float2* d = W + r * S + y4;
-    d[0] = make_float2(a.x, b.x);
-    d[1] = make_float2(a.y, b.y);
-    d[2] = make_float2(a.z, b.z);
-    d[3] = make_float2(a.w, b.w);
-    if ((a.x != 0.f) | (a.y != 0.f) | (a.z != 0.f) | (a.w != 0.f) | (b.x != 0.f) | (b.y != 0.f) | (b.z != 0.f) |
-        (b.w != 0.f))
-      s_live[r] = 1;
-  }
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    int base = 0;
-    for (int r0 = 0; r0 < NH; r0 += 32) {
-      const bool live = r0 + (int)threadIdx.x < NH && s_live[r0 + threadIdx.x];
-      const unsigned m = __ballot_sync(0xffffffffu, live);
-      if (live) s_rows[base + __popc(m & ((1u << threadIdx.x) - 1u))] = r0 + threadIdx.x;
-      base += __popc(m);
-    }
-    if (threadIdx.x == 0) s_nrows = base;
-  }
-  __syncthreads();
-  const int nrows = s_nrows;
-  float2* out = spec + (size_t)c * spec_cstride + (size_t)z * N * H2p;
-  if (nrows == 0) {  // empty slab: its 2-D spectrum is zero
-    for (int e = threadIdx.x; e < N * H2; e += T) {
-      const int k = e / H2, ky = e - k * H2;
-      out[(size_t)k * H2p + ky] = make_float2(0.f, 0.f);
-    }
-    if (nz && threadIdx.x == 0) *nz = 0;  // every thread read it before the barrier above
-    return;
-  }
-  if (nz && threadIdx.x == 0) *nz = 1;
-  // rows that are all zero stay zero under the y transform
-  fft_tail<N, false, false, true, tail_threads<NF>()>(W, nrows, S, pN.tw, s_rows);  // over y, live rows
-  fft_tail<NH, false, true, true, tail_threads<NF>()>(W, N, S, pH.tw);               // over r, columns
-  for (int e = threadIdx.x; e < NH * H2; e += T) {
-    const int k = e / H2, ky = e - k * H2;
-    const float2 w1 = W[s_posH[k] * S + s_posN[ky]];
-    const float2 w2 = W[s_posH[k == 0 ? 0 : NH - k] * S + s_posN[ky == 0 ? 0 : N - ky]];
-    const float2 A = make_float2(0.5f * (w1.x + w2.x), 0.5f * (w1.y - w2.y));
-    const float2 B = make_float2(0.5f * (w1.y + w2.y), -0.5f * (w1.x - w2.x));  // (w1 - conj w2) / 2i
-    const float2 tB = cmul(__ldg(&pN.tw[k]), B);
-    out[(size_t)k * H2p + ky] = cadd(A, tB);
-    out[(size_t)(k + NH) * H2p + ky] = csub(A, tB);
-  }
-}
-
-// Fused inverse of one z-slab: inverse over x and the real inverse over y of
-// the product spectrum (natural kx), first-occurrence argmax of the signed
-// output.  The ky = 0 and ky = N/2 columns are first projected onto their
-// x-Hermitian parts, which is what a half-complex inverse reads (only the real
-// parts of its DC and Nyquist terms after the inverse over x).
-template <int NF>
-__global__ void __launch_bounds__(tail_threads<NF>()) k_slab_inv(const float2* __restrict__ cspec, FftPlan pN,
-                                                   FftPlan pH, unsigned long long* __restrict__ argmax,
-                                                   float* __restrict__ volume, uint32_t limit) {
-  constexpr int N = NF, NH = NF / 2, H2 = NF / 2 + 1, S = NF + 1;
-  constexpr int T = tail_threads<NF>();  // the launch's block size
-  const int H2p = spatial_h2p(N);
-  extern __shared__ float2 W[];  // [NH][S]
-  __shared__ int s_posN[N], s_posH[NH];  // digit-reversed positions of frequencies
-  const int z = blockIdx.x;
-  const float2* X = cspec + (size_t)z * N * H2p;
-  for (int k = threadIdx.x; k < N; k += T) {
-    s_posN[k] = fixed_freq2pos<N>(k);
-    if (k < NH) s_posH[k] = fixed_freq2pos<NH>(k);
-  }
-  __syncthreads();
-  // four elements' loads in flight per thread
-  constexpr int U = 4;
-  for (int e0 = threadIdx.x; e0 < NH * H2; e0 += U * T) {
-    float2 x0u[U], x1u[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int e = e0 + u * T;
-      const int k = e / H2, ky = e - k * H2;
-      const bool ok = e < NH * H2;
-      x0u[u] = ok ? X[(size_t)k * H2p + ky] : make_float2(0.f, 0.f);
-      x1u[u] = ok ? X[(size_t)(k + NH) * H2p + ky] : make_float2(0.f, 0.f);
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-    const int e = e0 + u * T;
-    if (e >= NH * H2) break;
-    const int k = e / H2, ky = e - k * H2;
-    float2 x0 = x0u[u], x1 = x1u[u];
-    if (ky == 0 || ky == NH) {
-      const float2 m0 = X[(size_t)(k == 0 ? 0 : N - k) * H2p + ky];  // kx = -k
-      const float2 m1 = X[(size_t)(NH - k) * H2p + ky];               // kx = -(k + N/2)
-      x0 = make_float2(0.5f * (x0.x + m0.x), 0.5f * (x0.y - m0.y));
-      x1 = make_float2(0.5f * (x1.x + m1.x), 0.5f * (x1.y - m1.y));
-    }
-    const float2 A = make_float2(0.5f * (x0.x + x1.x), 0.5f * (x0.y + x1.y));
-    const float2 B = cmul(make_float2(0.5f * (x0.x - x1.x), 0.5f * (x0.y - x1.y)), cconj(__ldg(&pN.tw[k])));
-    // W = A + i B at (k, ky); its mirror (-k, -ky) holds conj(A) + i conj(B)
-    W[s_posH[k] * S + s_posN[ky]] = make_float2(A.x - B.y, A.y + B.x);
-    if (ky >= 1 && ky < NH) W[s_posH[k == 0 ? 0 : NH - k] * S + s_posN[N - ky]] = make_float2(A.x + B.y, -A.y + B.x);
-    }
-  }
-  __syncthreads();
-  fft_tail<NH, true, true, true, tail_threads<NF>()>(W, N, S, pH.tw);    // over r, columns
-  fft_tail<N, true, false, true, tail_threads<NF>()>(W, NH, S, pN.tw);   // over y, rows
-  // per thread: the largest value, the lowest index among equal ones (the
-  // reference's first occurrence, whatever order the thread visits them in)
-  float bv = -INFINITY;
-  uint32_t bi = 0xffffffffu;
-  for (int e = threadIdx.x; e < NH * N; e += T) {
-    const int r = e / N, y = e - r * N;
-    const float2 v = W[r * S + y];
-    const float a0 = 2.0f * v.x, a1 = 2.0f * v.y;
-    const uint32_t i0 = (uint32_t)(((size_t)z * N + 2 * r) * N + y);
-    const uint32_t i1 = i0 + N;
-    if (i0 < limit && (a0 > bv || (a0 == bv && i0 < bi) || bi == 0xffffffffu)) {
-      bv = a0;
-      bi = i0;
-    }
-    if (i1 < limit && (a1 > bv || (a1 == bv && i1 < bi) || bi == 0xffffffffu)) {
-      bv = a1;
-      bi = i1;
-    }
-    if (volume) {
-      volume[i0] = a0;
-      volume[i1] = a1;
-    }
-  }
-  warp_argmax_commit(bi == 0xffffffffu ? 0ull : pack_argmax(bv, bi), argmax);
 }
 
 // ---------------------------------------------------------------- launchers
@@ -682,169 +773,166 @@ static cudaError_t allow_max_smem(const void* fn) {
   return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem - (int)fa.sharedSizeBytes);
 }
 
+// The z pass of C channels per side with tiles of wt columns: the width is a
+// compile-time constant (4 or 8) for the compile-time lengths.
+using FuseZFn = void (*)(const SpatialArgs, const FftPlan, int);
+template <int NF, int LW>
+static FuseZFn fuse_z_channels(int C) {
+  return C == 1 ? k_fuse_z<NF, 1, LW> : (C == 2 ? k_fuse_z<NF, 2, LW> : (C == 3 ? k_fuse_z<NF, 3, LW> : k_fuse_z<NF, 4, LW>));
+}
+template <int NF>
+static FuseZFn fuse_z_kernel(int C, int wt) {
+  if constexpr (NF > 0)
+    return wt >= 8 ? fuse_z_channels<NF, 3>(C) : fuse_z_channels<NF, 2>(C);
+  else
+    return fuse_z_channels<0, -1>(C);
+}
+
+// The forward x pass of C channels: tiles of 8 columns (64-byte rows), so four
+// or more blocks fit on an SM at N = 200 with three channels.
+constexpr int kXFwdLog2 = 3, kXInvLog2 = 4;
+using FftXFn = void (*)(const ColArgs);
+template <int NF>
+static FftXFn fft_x_forward(int C) {
+  return C == 1 ? k_fft_x<NF, false, 1, kXFwdLog2>
+                : (C == 2 ? k_fft_x<NF, false, 2, kXFwdLog2>
+                          : (C == 3 ? k_fft_x<NF, false, 3, kXFwdLog2> : k_fft_x<NF, false, 4, kXFwdLog2>));
+}
+
 template <int NF>
 static cudaError_t set_attrs() {
-  cudaError_t e = allow_max_smem((const void*)k_fuse_z<NF>);
-  if constexpr (NF > 0)
-    if (e == cudaSuccess) e = allow_max_smem((const void*)k_fuse_z<NF, 6, 8>);
-  if (e == cudaSuccess) e = allow_max_smem((const void*)k_r2c_y<NF>);
-  if (e == cudaSuccess) e = allow_max_smem((const void*)k_fft_x<NF, false>);
-  if (e == cudaSuccess) e = allow_max_smem((const void*)k_fft_x<NF, true>);
-  if (e == cudaSuccess) e = allow_max_smem((const void*)k_c2r_y<NF>);
-  return e;
-}
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFn encode_tiled() {
-  static EncodeTiledFn fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      p = nullptr;
-    return reinterpret_cast<EncodeTiledFn>(p);
-  }();
-  return fn;
-}
-
-cudaError_t spatial_init_attributes() {
   cudaError_t e = cudaSuccess;
-  for (int n : {64, 128, 200, 256, 320, 512, 0}) {  // every length PHGPU_DISPATCH_N instantiates
-    cudaError_t r = cudaSuccess;
-    PHGPU_DISPATCH_N(n, r = set_attrs<NF>());
-    if (r != cudaSuccess) e = r;
-  }
-  for (auto fn : {(const void*)k_slab_fwd<64>, (const void*)k_slab_fwd<128>, (const void*)k_slab_fwd<200>,
-                  (const void*)k_slab_inv<64>, (const void*)k_slab_inv<128>, (const void*)k_slab_inv<200>}) {
-    cudaError_t r = allow_max_smem(fn);
-    if (r != cudaSuccess) e = r;
-  }
-  // look the tensor-map encoder up now, not first inside a stream capture
-  encode_tiled();
+  for (auto fn : {(const void*)k_r2c_rows<NF>, (const void*)k_c2r_rows<NF>, (const void*)k_fft_x<NF, true, 1, 4>})
+    if (e == cudaSuccess) e = allow_max_smem(fn);
+  for (int C = 1; C <= 4; ++C)
+    if (e == cudaSuccess) e = allow_max_smem((const void*)fft_x_forward<NF>(C));
+  for (int C = 1; C <= 4; ++C)
+    for (int wt : {4, 8})
+      if (e == cudaSuccess) e = allow_max_smem((const void*)fuse_z_kernel<NF>(C, wt));
   return e;
 }
 
-bool spatial_slab_path(int N) { return N == 64 || N == 128 || N == 200; }
-
-#define PHGPU_DISPATCH_SLAB(n, ...) \
-  switch (n) {                      \
-    case 64: {                      \
-      constexpr int NF = 64;        \
-      __VA_ARGS__;                  \
-    } break;                        \
-    case 128: {                     \
-      constexpr int NF = 128;       \
-      __VA_ARGS__;                  \
-    } break;                        \
-    default: {                      \
-      constexpr int NF = 200;       \
-      __VA_ARGS__;                  \
-    } break;                        \
-  }
-
-// Tile width of the z pass: as many ky columns as fit (<= 8) in shared memory.
-static size_t fuse_z_smem(int N, int A, int wt) {
-  const int chunks = (N + 255) / 256;
-  const size_t rows = (size_t)chunks * ((N + chunks - 1) / chunks);
-  return rows * A * wt * sizeof(float2) + 16 + sizeof(FusionBands) + (size_t)N * sizeof(int);
+cudaError_t spatial_init_attributes(int N, int M) {
+  cudaError_t e = cudaSuccess;
+  PHGPU_DISPATCH_N(N, e = set_attrs<NF>());
+  if (e == cudaSuccess && M != N) PHGPU_DISPATCH_N(M, e = set_attrs<NF>());
+  for (auto fn : {(const void*)k_scan_rows<1>, (const void*)k_scan_rows<2>, (const void*)k_scan_rows<3>,
+                  (const void*)k_scan_rows<4>})
+    if (e == cudaSuccess) e = allow_max_smem(fn);
+  return e;
 }
+
+// Whether PHGPU_DISPATCH_N gives N a compile-time plan.
+static bool fixed_length(int N) {
+  bool fixed = false;
+  PHGPU_DISPATCH_N(N, fixed = NF > 0);
+  return fixed;
+}
+
+// Shared memory of the prime-radix scratch of runtime plans.
+static size_t prime_scratch(int N) { return fixed_length(N) ? 0 : kMaxGenericRadix * sizeof(float4); }
+
+static size_t fuse_z_smem(int N, int C, int wt) {
+  int rows = N;
+  PHGPU_DISPATCH_N(N, rows = z_off<NF>(N));
+  return (size_t)(C + 1) * rows * wt * sizeof(float2) + prime_scratch(N) + 8 * (size_t)N;
+}
+
+constexpr size_t kFuseZStatic = 2 * 1024;  // the kernel's static and the system's shared memory, rounded up
 
 bool fuse_z_tile_ok(int N, int A, int wt) {
-  return (wt == 2 || wt == 4 || wt == 8 || wt == 16) && fuse_z_smem(N, A, wt) <= (size_t)kMaxSmem;
+  return (wt == 2 || wt == 4 || wt == 8 || wt == 16) && fuse_z_smem(N, A / 2, wt) + kFuseZStatic <= (size_t)kMaxSmem;
 }
 
-static int fuse_z_tile(int N, int A) {
-  // >= 2: the loader moves two complex per 16-byte access, and a bulk copy's
-  // innermost extent must be a multiple of 16 bytes
+// Tile width of the z pass: the widest (<= 8: 64-byte rows) of which two
+// blocks fit on an SM, since the blocks hide one another's barriers and loads.
+static int fuse_z_tile(int N, int C) {
   int wt = 8;
-  const int chunks = (N + 255) / 256;                       // bulk copies of <= 256 z rows
-  const size_t rows = (size_t)chunks * ((N + chunks - 1) / chunks);
-  const size_t extra = 16 + sizeof(FusionBands) + (size_t)N * sizeof(int);
-  // narrower tiles until two blocks fit on an SM (one block cannot overlap
-  // its bulk load with its own transforms), at least until the limit is met
-  while (wt > 2 && rows * A * wt * sizeof(float2) + extra > (size_t)kMaxSmem / 2) wt >>= 1;
+  while (wt > 2 && fuse_z_smem(N, C, wt) + kFuseZStatic > (size_t)kMaxSmem / 2) wt >>= 1;
   return wt;
 }
 
-// cuTensorMapEncodeTiled through the runtime (no link against the driver
-// library); null when unavailable, in which case the element loader is used.
+// Threads of a z-pass block: the least idle time over its stages (an item
+// carries the C channels of a side; the fused middle stage; the product's
+// inverse).
+static int fuse_z_threads(const FftPlan& p, int C, int wt) {
+  int best = 256;
+  double best_cost = 1e300;
+  const int lo = std::min(192, (wt * p.n / std::max(1, p.nstage ? p.radix[0] : 1) + 31) / 32 * 32);
+  for (int t = std::max(lo, 64); t <= kFuseZMaxThreads; t += 32) {
+    auto rounds = [&](int items) { return (double)((items + t - 1) / t) * t; };
+    double cost = 0.0;
+    for (int s = 0; s < p.nstage; ++s) {
+      const int R = p.radix[s], nb = p.n / R;
+      cost += R * (2.0 * C + 1.0) * rounds(wt * nb);
+    }
+    if (cost <= best_cost * 1.0001) {
+      best_cost = cost;
+      best = t;
+    }
+  }
+  return best;
+}
+
 cudaError_t launch_spatial_forward(const SpatialArgs& a, int side, cudaStream_t st) {
   const int N = a.N, H2 = N / 2 + 1;
   const size_t nv = (size_t)N * N * N;
   const size_t plane = (size_t)N * N * spatial_h2p(N);
-  const float* grids = side == 0 ? a.grids_f : a.grids_g;
+  float* grids = side == 0 ? a.grids_f : a.grids_g;
   const int nch = a.laplace ? a.n_data_ch : (a.lowpass ? 2 : 1);
-  const float* count = a.grids_are_means ? nullptr : grids + (size_t)a.n_data_ch * nv;
-  if (spatial_slab_path(N) && a.plan_half) {
-    float2* spec = a.spec + (size_t)(side * a.n_data_ch) * plane;
-    dim3 g(N, nch);
-    const size_t sm = (size_t)(N / 2) * (N + 1) * sizeof(float2);
-    const uint8_t* rowlive = side == 0 ? a.rowlive_f : a.rowlive_g;
-    uint8_t* nz = a.slab_nz ? a.slab_nz + (size_t)(side * a.n_data_ch) * N : nullptr;
-    PHGPU_DISPATCH_SLAB(N, k_slab_fwd<NF><<<g, tail_threads<NF>(), sm, st>>>(grids, nv, count, rowlive, spec, plane,
-                                                                             *a.plan, *a.plan_half, nz));
+  float2* spec = a.spec + (size_t)(side * a.n_data_ch) * plane;
+  const ColArgs c{N, spec, plane, a.grids_are_means ? nullptr : a.rowmask + (size_t)side * N * N,
+                  a.slab_live + (size_t)side * N, a.full_spec, *a.plan};
+  if (a.grids_are_means) {
+    const dim3 gr((N * N + 2 * kRowPairs - 1) / (2 * kRowPairs), nch);
+    const size_t smr = (size_t)kRowPairs * row_stride(N) * sizeof(float2) + prime_scratch(N);
+    const int tr = pass_threads(*a.plan, kRowPairs, 1, 128, 320);
+    PHGPU_DISPATCH_N(N, k_r2c_rows<NF><<<gr, tr, smr, st>>>(N, grids, nv, spec, plane, *a.plan));
+  } else {
+    const ScanRowArgs r{N, grids, reinterpret_cast<const float*>(a.plan->tw), (size_t)a.count_plane * nv, a.rowlive[side],
+                        a.rowmask + (size_t)side * N * N, spec, plane, a.clear};
+    const dim3 gr(N, (N + kRowsBlock - 1) / kRowsBlock);
+    const size_t smr = scan_rows_smem(N);
+    if (nch == 1)
+      k_scan_rows<1><<<gr, kRowsWarps * 32, smr, st>>>(r);
+    else if (nch == 2)
+      k_scan_rows<2><<<gr, kRowsWarps * 32, smr, st>>>(r);
+    else if (nch == 3)
+      k_scan_rows<3><<<gr, kRowsWarps * 32, smr, st>>>(r);
+    else
+      k_scan_rows<4><<<gr, kRowsWarps * 32, smr, st>>>(r);
+  }
+  // channels of one launch: as many as leave two blocks an SM's shared memory
+  const size_t per = (size_t)N * (1 << kXFwdLog2) * sizeof(float2), extra = prime_scratch(N) + (size_t)N;
+  int cc = nch;
+  while (cc > 1 && cc * per + extra + 2048 > (size_t)kMaxSmem / 2) --cc;
+  const dim3 gx((H2 + (1 << kXFwdLog2) - 1) >> kXFwdLog2, N);
+  for (int ch = 0; ch < nch; ch += cc) {
+    ColArgs cx = c;
+    cx.spec += (size_t)ch * plane;
+    const int k = std::min(cc, nch - ch);
+    const int tx = pass_threads(*a.plan, 1 << kXFwdLog2, k, 160, kXThreads);
+    FftXFn fn = nullptr;
+    PHGPU_DISPATCH_N(N, fn = fft_x_forward<NF>(k));
+    fn<<<gx, tx, k * per + extra, st>>>(cx);
     count_launches(1);
-    return cudaGetLastError();
   }
-  const int nrowblk = (int)((nv / N + kRowsR2C - 1) / kRowsR2C);
-  for (int c = 0; c < nch; ++c) {
-    float2* spec = a.spec + (size_t)(side * a.n_data_ch + c) * plane;
-    const float* g = grids + (size_t)c * nv;
-    dim3 gx((H2 + 15) / 16, N, 1);
-    const uint8_t* rowlive = side == 0 ? a.rowlive_f : a.rowlive_g;
-    const size_t smr = (size_t)(kRowsR2C / 2) * N * sizeof(float2) + (size_t)N * sizeof(int);
-    PHGPU_DISPATCH_N(N,
-        k_r2c_y<NF><<<nrowblk, 256, smr, st>>>(N, g, count, rowlive, spec, *a.plan);
-        k_fft_x<NF, false><<<gx, 256, (size_t)N * 16 * sizeof(float2), st>>>(N, spec, *a.plan));
-    count_launches(2);
-  }
+  count_launches(1);
   return cudaGetLastError();
 }
 
 cudaError_t launch_spatial_fuse_z(const SpatialArgs& a, cudaStream_t st) {
   const int N = a.N, H2 = N / 2 + 1;
-  const int A = a.laplace ? 2 * a.n_data_ch : 2;
-  const int wt = fuse_z_tile_ok(N, A, a.fuse_tile) ? a.fuse_tile : fuse_z_tile(N, A);
-  // bulk tensor copies of the [z][array][ky] tile (element = one complex)
-  CUtensorMap tmap;
-  memset(&tmap, 0, sizeof(tmap));
-  FuseZTma tma{0, N, 1};
-  if (EncodeTiledFn enc = encode_tiled()) {
-    const size_t plane = (size_t)N * N * spatial_h2p(N);
-    const int chunks = (N + 255) / 256;
-    const int zbox = (N + chunks - 1) / chunks;
-    const cuuint64_t dims[4] = {(cuuint64_t)spatial_h2p(N), (cuuint64_t)A, (cuuint64_t)N, (cuuint64_t)N};
-    const cuuint64_t strides[3] = {(cuuint64_t)(a.laplace ? plane : plane * a.n_data_ch) * sizeof(float2),
-                                   (cuuint64_t)spatial_h2p(N) * sizeof(float2),
-                                   (cuuint64_t)N * spatial_h2p(N) * sizeof(float2)};
-    const cuuint32_t box[4] = {(cuuint32_t)wt, (cuuint32_t)A, 1u, (cuuint32_t)zbox};
-    const cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
-    void* base = (void*)(a.spec + (a.laplace ? 0 : (size_t)a.lowpass * plane));
-    if (enc(&tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, base, dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS)
-      tma = FuseZTma{1, zbox, chunks};
-  }
-  const size_t rows = (size_t)tma.zbox * tma.chunks;
-  const size_t smB = rows * A * wt * sizeof(float2) + 16 + sizeof(FusionBands) + (size_t)N * sizeof(int);
-  if (smB > (size_t)kMaxSmem) return cudaErrorInvalidConfiguration;
-  dim3 gB((H2 + wt - 1) / wt, N);
-  const int xnat = (spatial_slab_path(N) && a.plan_half) ? 1 : 0;
-  // the bench shape (Laplace fusion of three channels, tile width 8) has its
-  // own instantiation with the tile shape known at compile time
-  const bool shape68 = A == 6 && wt == 8;
-  PHGPU_DISPATCH_N(N, {
-    bool done = false;
-    if constexpr (NF > 0) {
-      if (shape68) {
-        k_fuse_z<NF, 6, 8><<<gB, kFuseZThreads, smB, st>>>(a, *a.plan, wt, xnat, tmap, tma);
-        done = true;
-      }
-    }
-    if (!done) k_fuse_z<NF><<<gB, kFuseZThreads, smB, st>>>(a, *a.plan, wt, xnat, tmap, tma);
-  });
+  const int C = a.laplace ? a.n_data_ch : 1;
+  int wt = fuse_z_tile_ok(N, 2 * C, a.fuse_tile) ? a.fuse_tile : fuse_z_tile(N, C);
+  if (fixed_length(N)) wt = wt >= 8 ? 8 : 4;  // the widths built for compile-time lengths
+  const size_t sm = fuse_z_smem(N, C, wt);
+  if (sm + kFuseZStatic > (size_t)kMaxSmem) return cudaErrorInvalidConfiguration;
+  const dim3 g((H2 + wt - 1) / wt, N);
+  const int lw = wt == 16 ? 4 : (wt == 8 ? 3 : (wt == 4 ? 2 : 1));
+  FuseZFn fn = nullptr;
+  PHGPU_DISPATCH_N(N, fn = fuse_z_kernel<NF>(C, wt));
+  fn<<<g, fuse_z_threads(*a.plan, C, wt), sm, st>>>(a, *a.plan, lw);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -852,27 +940,17 @@ cudaError_t launch_spatial_fuse_z(const SpatialArgs& a, cudaStream_t st) {
 cudaError_t launch_spatial_inverse(const SpatialArgs& a, cudaStream_t st) {
   const int N = a.N, H2 = N / 2 + 1;
   const uint32_t limit = a.argmax_limit ? a.argmax_limit : 0xffffffffu;
-  if (spatial_slab_path(N) && a.plan_half) {
-    const size_t sm = (size_t)(N / 2) * (N + 1) * sizeof(float2);
-    PHGPU_DISPATCH_SLAB(N, k_slab_inv<NF><<<N, tail_threads<NF>(), sm, st>>>(a.cspec, *a.plan, *a.plan_half, a.argmax,
-                                                                             a.volume, limit));
-    count_launches(1);
-    return cudaGetLastError();
-  }
-  dim3 gC((H2 + 15) / 16, N, 1);
-  const int nrowblk = (int)(((size_t)N * N + kRowsR2C - 1) / kRowsR2C);
-  PHGPU_DISPATCH_N(N,
-      k_fft_x<NF, true><<<gC, 256, (size_t)N * 16 * sizeof(float2), st>>>(N, a.cspec, *a.plan);
-      k_c2r_y<NF><<<nrowblk, 256, (size_t)(kRowsR2C / 2) * N * sizeof(float2) + (size_t)N * sizeof(int), st>>>(
-          N, a.cspec, *a.plan, a.argmax, a.volume, limit));
+  const ColArgs c{N, a.cspec, 0, nullptr, nullptr, 1, *a.plan};
+  const dim3 gx((H2 + (1 << kXInvLog2) - 1) >> kXInvLog2, N);
+  const size_t smx = (size_t)N * (1 << kXInvLog2) * sizeof(float2) + prime_scratch(N);
+  const int nblk = (N * N + 2 * kInvPairs - 1) / (2 * kInvPairs);
+  const size_t smr = (size_t)kInvPairs * row_stride(N) * sizeof(float2) +
+                     (fixed_length(N) ? 0 : prime_scratch(N) + (size_t)N * sizeof(int) + 16);
+  const int tr = pass_threads(*a.plan, kInvPairs, 1, 128, 320), tx = pass_threads(*a.plan, 1 << kXInvLog2, 1, 160, kXThreads);
+  PHGPU_DISPATCH_N(N, k_fft_x<NF, true, 1, kXInvLog2><<<gx, tx, smx, st>>>(c);
+                   k_c2r_rows<NF><<<nblk, tr, smr, st>>>(N, a.cspec, *a.plan, a.argmax, a.volume, limit));
   count_launches(2);
   return cudaGetLastError();
-}
-
-cudaError_t launch_spatial_combine(const SpatialArgs& a, cudaStream_t st) {
-  cudaError_t e = launch_spatial_fuse_z(a, st);
-  if (e == cudaSuccess) e = launch_spatial_inverse(a, st);
-  return e;
 }
 
 }  // namespace phgpu

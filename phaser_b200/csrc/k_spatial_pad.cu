@@ -71,7 +71,7 @@ __device__ __forceinline__ float2 spec_at(const float2* __restrict__ arr, uint32
   const uint32_t kz = flat / (N * H), rem = flat - kz * N * H;
   const uint32_t kx = rem / H, ky = rem - kx * H;
   const int zp = fft_freq2pos((int)kz, a.planN);
-  const int xp = a.x_natural_N ? (int)kx : fft_freq2pos((int)kx, a.planN);
+  const int xp = fft_freq2pos((int)kx, a.planN);
   return arr[((size_t)zp * N + (size_t)xp) * spatial_h2p(a.N) + ky];
 }
 
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(256) k_pad_fuse(PadArgs a) {
   const uint32_t kz = y / (M * HM), rem = y - kz * M * HM;
   const uint32_t kx = rem / HM, ky = rem - kx * HM;
   const int zp = fft_freq2pos((int)kz, a.planM);
-  const int xp = a.x_natural_M ? (int)kx : fft_freq2pos((int)kx, a.planM);
+  const int xp = fft_freq2pos((int)kx, a.planM);
   a.cspec[((size_t)zp * M + (size_t)xp) * spatial_h2p(a.M) + ky] = c;
 }
 

@@ -92,9 +92,11 @@ struct FuseS2Args {
   FusionBands bands;      // for n = B^2
   const float2* coef;     // [2][n_data_ch][B][B]   (side-major)
   float2* fused;          // [2][B (l)][2B-1 (m + B - 1)]
+  unsigned long long* argmax;  // rotation argmax, reset here for the transform that follows
   int count = 0;          // > 0: requests of one launch, coef_b / fused_b per request (else coef / fused)
   const float2* coef_b[32];
   float2* fused_b[32];
+  unsigned long long* argmax_b[32];  // each request's rotation argmax, reset here
 };
 cudaError_t launch_fuse_s2(const FuseS2Args& a, cudaStream_t st);
 // out[side][k] = 0.6 * intensity + 0.4 * range of samples [side][c][n] (n = 4B^2)
@@ -126,7 +128,7 @@ struct So3Args {
 bool so3_beta_tile_ok(int bw_out, int wt);
 cudaError_t launch_so3_synth(const So3Args& a, cudaStream_t st);  // coefficient product + FP32 Wigner synthesis
 cudaError_t launch_so3_fft(const So3Args& a, cudaStream_t st);    // alpha FFT + gamma C2R + argmax
-cudaError_t so3_init_attributes();  // once per device
+cudaError_t so3_init_attributes(int n);  // once per context: length n = 2 bw_out
 void so3_beta_table(int bw_out, double* host_tab);  // fills the [3][2 bw_out] beta_tab on the host
 void so3_wigner_table(int bw_in, std::vector<double>& host_tab);  // recurrence tables of the synthesis
 
@@ -178,11 +180,6 @@ struct VoxelArgs {
   const uint32_t* n_dev = nullptr;  // when set: the point count is read from device memory (n_points = capacity)
 };
 cudaError_t launch_voxelize(const VoxelArgs& a, cudaStream_t st);
-// Zeroes what one voxelisation wrote: planes [0, n_planes) at every point's
-// voxel (lin[i] != 0xffffffff) and the point's row flag.
-cudaError_t launch_clear_voxels(const uint32_t* lin, int n_points, float* grids, size_t nv, int n_planes,
-                                uint8_t* rowlive, int N, cudaStream_t st, const uint32_t* n_dev = nullptr);
-
 struct SpatialArgs {
   int N;
   int n_data_ch;          // channels per side with data
@@ -191,31 +188,31 @@ struct SpatialArgs {
   int lowpass;            // 1 (with laplace 0): channel 1, products outside the shifted cube zeroed
   uint32_t lp_lo, lp_hi;  // cube [lp_lo, lp_hi]^3 of subscripts
   FusionBands bands;      // for n = N^3
-  const float* grids_f;   // [n_data_ch + 1][N^3] target sums + count (normalised here)
-  const float* grids_g;   // source
+  float* grids_f;         // target grids: voxel sums, counts in plane count_plane (or values)
+  float* grids_g;         // source
+  int count_plane;        // plane of the point counts in the grids
   int grids_are_means;    // 1: grids already hold values (no count plane)
-  const uint8_t* rowlive_f;  // optional row flags of the grids (rows never flagged are all zero)
-  const uint8_t* rowlive_g;
-  uint8_t* slab_nz;       // optional [2 n_data_ch][N] per spectrum array: 0 where the z-slab is known
-                          // to hold zeros (the z-slab forward then skips a slab that stays zero,
-                          // and keeps the flags); null: every slab is written
+  int clear;              // 1: the forward zeroes the voxels and row flags it read
+  uint8_t* rowlive[2];    // [N (z)][N (x)] rows that hold a point, per side
+  uint8_t* rowmask;       // [2][N (z)][N (x)]: written by the forward of a voxelised side (the row flags, which
+                          // `clear` resets)
+  uint8_t* slab_live;     // [2][N]: written by the forward, 1 where the side's z-slab holds a point; the z
+                          // pass reads no other slab's spectrum
+  int full_spec;          // 1: empty slabs are written as zeros too (the padded product reads them)
   float2* spec;           // [2 n_data_ch][N (z)][N (x)][H2p (ky)]
   float2* cspec;          // [N][N][H2p]
   const FftPlan* plan;    // length N
-  const FftPlan* plan_half;  // length N/2 (z-slab kernels), may be null
-  unsigned long long* argmax;
+  unsigned long long* argmax;  // reset by the z pass, taken by the inverse
   float* volume;          // optional N^3 correlation, [z][x][y]
-  unsigned long long* status;  // bit 0: a bulk-copy wait gave up (result invalid)
   uint32_t argmax_limit = 0;   // argmax over indices < limit (0: all)
-  int fuse_tile = 0;           // ky columns per k_fuse_z block (2, 4, 8, 16; 0 = widest with two blocks per SM): tuned
+  int fuse_tile = 0;           // ky columns per k_fuse_z block (2, 4, 8, 16; 0 = the widest up to 8 with two blocks per SM): tuned
 };
 // Whether a k_fuse_z tile of wt ky columns fits shared memory for N and A arrays.
 bool fuse_z_tile_ok(int N, int A, int wt);
 cudaError_t launch_spatial_forward(const SpatialArgs& a, int side, cudaStream_t st);
-cudaError_t launch_spatial_combine(const SpatialArgs& a, cudaStream_t st);
 cudaError_t launch_spatial_fuse_z(const SpatialArgs& a, cudaStream_t st);   // z FFTs + fusion + cross power
 cudaError_t launch_spatial_inverse(const SpatialArgs& a, cudaStream_t st);  // inverse x + C2R y + argmax
-cudaError_t spatial_init_attributes();  // once per device
+cudaError_t spatial_init_attributes(int N, int M);  // once per context: lengths N and M
 // ------------------------------------------------------------ zero-padded translation
 // The reference's padded spatial correlation (spatial-correlation.cc:11-45,
 // 142-161,223-230): the product of the (fused) N-sized spectra is scattered
@@ -228,12 +225,10 @@ struct PadArgs {
   int n_spec;             // channels with spectra in spec (mode 1; the others are zero)
   int spec_ch;            // channels per side in the spec layout
   int first_ch;           // spec channel read by modes 0 and 2
-  const float2* spec;     // [2][spec_ch][N (z pos)][N (x pos)][H2p]: full 3-D spectra
+  const float2* spec;     // [2][spec_ch][N (z pos)][N (x pos)][H2p]: full 3-D spectra (x, z digit-reversed)
   const float2* prev_f;   // last channel of the previous call (mode 1), null = zero
   const float2* prev_g;
-  int x_natural_N;        // spec x positions: 1 natural, 0 digit-reversed
-  int x_natural_M;        // cspec_pad x positions expected by the inverse at M
-  FftPlan planN, planM;   // z positions (both digit-reversed)
+  FftPlan planN, planM;   // x and z positions
   FusionBands bands;      // n = N^3
   uint32_t lp_lo, lp_hi;  // mode 2 index cube
   float inv_total;        // 1 / channel count (MEAN)
@@ -247,7 +242,5 @@ cudaError_t launch_pad_fuse(const PadArgs& a, cudaStream_t st);
 
 // Row length of the half spectra: N/2 + 1 rounded up to 8 complex (64 B).
 __host__ __device__ inline int spatial_h2p(int N) { return ((N / 2 + 1) + 7) / 8 * 8; }
-// True when the fused z-slab kernels handle this N (the slab fits in shared memory).
-bool spatial_slab_path(int N);
 
 }  // namespace phgpu

@@ -87,7 +87,7 @@ uint64_t estimate_slot_bytes(const phgpu_params& p, uint32_t max_points) {
   uint64_t b = 0;
   b += 4 * 4 * bw * bw * 2 + 8 * bw * bw * 8 + 8 * bw * 2 * bw * 8;  // samples, coefficients, SHT scratch
   b += 8 * bo * bo * bo;                                           // S
-  b += 2 * 5 * nv * 4 + 9 * H * 8;                                 // grids, spectra
+  b += 2 * 5 * nv * 4 + 9 * H * 8 + 4 * N * N;                     // grids, spectra, row flags
   b += bw * bw * (bw + 1) * 4;                                     // Legendre table
   if (p.flags & PHGPU_FLAG_KEEP_VOLUMES || p.rot_peak_neighbors) b += 8 * bo * bo * bo * 4;
   if (p.flags & PHGPU_FLAG_KEEP_VOLUMES || p.trans_peak_neighbors) b += nv * 4;

@@ -30,13 +30,14 @@ bool compile_time_length(int n) {
 bool has_runtime_plan(const phgpu_ctx* c) {
   if (!compile_time_length(2 * c->bw) || !compile_time_length(2 * c->bw_out) || !compile_time_length(c->N))
     return true;
-  if (c->has_sp_half && !compile_time_length(c->N / 2)) return true;
-  return c->pad && (!compile_time_length(c->M) || (c->has_pad_half && !compile_time_length(c->M / 2)));
+  return c->pad && !compile_time_length(c->M);
 }
 
 void apply_radix_order(phgpu_ctx* c, int order) {
-  for (FftPlan* p : {&c->plan_s2, &c->plan_so3, &c->plan_sp, &c->plan_sp_half, &c->plan_pad, &c->plan_pad_half}) {
-    if (p->n < 1) continue;
+  for (FftPlan* p : {&c->plan_s2, &c->plan_so3, &c->plan_sp, &c->plan_pad}) {
+    // compile-time lengths keep the order their kernels are built for (the
+    // padded product maps frequencies to positions by the plan)
+    if (p->n < 1 || compile_time_length(p->n)) continue;
     FftPlan q = *p;
     if (fft_plan_radices(p->n, order, &q)) *p = q;
   }

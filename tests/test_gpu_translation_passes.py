@@ -1,0 +1,89 @@
+"""The translation passes over voxelised clouds (row sums, x, z and inverse
+passes) against the FP64 oracle at lengths where they can go wrong: the
+shortest transforms, odd and prime lengths, prime factors at both ends of the
+generic stage, the compile-time lengths and their neighbours, tiles with a
+remainder; with one row and one slab filled, the rest nearly empty; two, three
+and four channels; a cloud outside the grid.  The bar is the repository's
+relative L2 of 1e-5 for correlation volumes."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from test_gpu_parity import REL_L2, tie_masked_rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def nat():
+    from phaser_b200 import native
+    native.load()
+    return native
+
+
+def cloud(rng, N, half, n=400):
+    """Points at random, along one whole row (every y) and over one z slab."""
+    edges = np.linspace(-half, half, N, dtype=np.float32)
+    step = edges[1] - edges[0] if N > 1 else np.float32(half)
+    p = rng.uniform(-half, half, (n, 3)).astype(np.float32)
+    k = np.arange(N)
+    row = np.stack([np.full(N, edges[N // 3]), edges[k], np.full(N, edges[N // 2])], 1) + 0.4 * step
+    m = min(N * N // 2, 3000)
+    slab = np.stack([edges[rng.integers(0, N, m)], edges[rng.integers(0, N, m)], np.full(m, edges[N // 4])], 1) + 0.4 * step
+    xyz = np.concatenate([p, row, slab]).astype(np.float32)
+    xyz = np.clip(xyz, -half, half)
+    w = rng.uniform(0.1, 1.0, (len(xyz), 3)).astype(np.float32)
+    return np.concatenate([xyz, w[:, :1]], 1), w[:, 1].copy(), w[:, 2].copy()
+
+
+@pytest.mark.parametrize("N,channels", [(2, 3), (3, 2), (4, 4), (7, 3), (8, 2), (11, 3), (13, 4), (22, 3), (31, 2), (35, 3),
+                                        (64, 4), (66, 3), (67, 3), (97, 2), (100, 3), (121, 3), (127, 2), (128, 2),
+                                        (130, 3), (200, 2)])
+def test_voxelised_translation_vs_oracle(nat, N, channels):
+    rng = np.random.default_rng(1000 * N + channels)
+    half = 10
+    clouds = [cloud(rng, N, half) for _ in range(2)]
+    c = nat.Context(spherical_bandwidth=2, spatial_n_voxels=N, spatial_discretize_lower=-half,
+                    spatial_discretize_upper=half, flags=nat.PHGPU_FLAG_KEEP_VOLUMES)
+    grids = []
+    for side, (xyzi, refl, amb) in enumerate(clouds):
+        args = (xyzi, refl if channels > 2 else None, amb if channels > 3 else None)
+        c.voxelize(*args, side=side)
+        grids.append(O.discretize(*args, N, -half, half).reshape(4, -1))
+    c.spatial_correlate_voxelized()
+    vox, peak, vol = c.spatial_result(volume=True)
+    ref = O.spatial_correlation(grids[0], grids[1], N, laplace=True)
+    err, _ = tie_masked_rel_l2(vol, ref, grids[0], grids[1], N)
+    assert err <= REL_L2
+    # the same grids again (they are kept), then a far cloud: everything zero, the first voxel wins
+    c.spatial_correlate_voxelized()
+    again = c.spatial_result(volume=True)
+    assert again[0] == vox and np.array_equal(again[2], vol)
+    far = clouds[1][0].copy()
+    far[:, 2] += 1000.0 * half
+    lin = O.voxel_index(far, N, -half, half)
+    c.voxelize(far, clouds[1][1] if channels > 2 else None, clouds[1][2] if channels > 3 else None, side=1)
+    c.spatial_correlate_voxelized()
+    vox, peak, vol = c.spatial_result(volume=True)
+    if (lin == 0xffffffff).all():
+        assert vox == 0 and peak == 0.0 and not vol.any()
+
+
+@pytest.mark.parametrize("N", [1, 2, 9, 64, 101, 169, 200])
+def test_host_grids_translation_vs_oracle(nat, N):
+    rng = np.random.default_rng(N)
+    f, g = rng.standard_normal((2, 2, N ** 3))
+    c = nat.Context(spherical_bandwidth=2, spatial_n_voxels=N, flags=nat.PHGPU_FLAG_KEEP_VOLUMES)
+    c.spatial_correlate(list(f), list(g))
+    _, _, vol = c.spatial_result(volume=True)
+    ref = O.spatial_correlation(f, g, N, laplace=True)
+    err, _ = tie_masked_rel_l2(vol, ref, f, g, N)
+    assert err <= REL_L2
+
+
+def test_fast_division_is_exact():
+    """fast_div(x, ceil(2^32 / d)) == x // d over the passes' ranges (x d < 2^32)."""
+    x = np.arange(1 << 18, dtype=np.uint64)
+    for d in [*range(2, 130), 201, 255, 256, 257, 511, 512, 513, 1000, 1023, 1024]:
+        mul = np.uint64(0xffffffff // d + 1)
+        assert np.array_equal((x * mul) >> np.uint64(32), x // np.uint64(d)), d
