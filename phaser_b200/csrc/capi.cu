@@ -469,14 +469,15 @@ static int ensure_cloud_capacity(phgpu_ctx* ctx, uint32_t n) {
     dfree(ctx, ctx->d_xyzi[s]);
     dfree(ctx, ctx->d_refl[s]);
     dfree(ctx, ctx->d_amb[s]);
-    dfree(ctx, ctx->d_sample_scratch[s]);
     dfree(ctx, ctx->d_lin[s]);
     CKV(dalloc(ctx, &ctx->d_xyzi[s], sizeof(float4) * cap));
     CKV(dalloc(ctx, &ctx->d_refl[s], sizeof(float) * cap));
     CKV(dalloc(ctx, &ctx->d_amb[s], sizeof(float) * cap));
-    CKV(dalloc(ctx, &ctx->d_sample_scratch[s], sampler_scratch_bytes((int)cap, 4 * ctx->bw * ctx->bw)));
     CKV(dalloc(ctx, &ctx->d_lin[s], sizeof(uint32_t) * cap));
   }
+  dfree(ctx, ctx->d_sample_scratch);
+  ctx->sample_scratch_stride = (sampler_scratch_bytes((int)cap, 4 * ctx->bw * ctx->bw) + 255) & ~(size_t)255;
+  CKV(dalloc(ctx, &ctx->d_sample_scratch, 2 * ctx->sample_scratch_stride));
   ctx->cap_points = cap;
   return PHGPU_OK;
 }
@@ -729,27 +730,32 @@ int phgpu_upload_cloud(phgpu_ctx* ctx, const phgpu_cloud* c, int side, cudaStrea
   return PHGPU_OK;
 }
 
-static int run_sample(phgpu_ctx* ctx, int side, cudaStream_t st) {
-  SampleArgs a;
-  a.xyzi = ctx->d_xyzi[side];
-  a.refl = ctx->has_refl[side] ? ctx->d_refl[side] : nullptr;
-  a.amb = ctx->has_amb[side] ? ctx->d_amb[side] : nullptr;
-  a.n_points = ctx->dev_counts ? (int)ctx->cap_points : (int)ctx->np[side];
-  a.n_dev = ctx->dev_counts ? ctx->d_np + side : nullptr;
-  a.max_points = (int)ctx->cap_points;
-  a.grid = ctx->d_grid;
-  a.n_queries = 4 * ctx->bw * ctx->bw;
-  a.n2b = 2 * ctx->bw;
-  a.max_sq = ctx->max_sq;
-  a.n_out_ch = 4;
-  a.out = ctx->d_samples + (size_t)side * 4 * a.n_queries;
-  a.nn_idx = ctx->d_nn[side];
-  a.scratch = ctx->d_sample_scratch[side];
+// Samples sides [first, first + n) in one set of launches.
+static int run_sample(phgpu_ctx* ctx, int first, int n, cudaStream_t st) {
+  SampleArgs args[2];
+  for (int i = 0; i < n; ++i) {
+    const int side = first + i;
+    SampleArgs& a = args[i];
+    a.xyzi = ctx->d_xyzi[side];
+    a.refl = ctx->has_refl[side] ? ctx->d_refl[side] : nullptr;
+    a.amb = ctx->has_amb[side] ? ctx->d_amb[side] : nullptr;
+    a.n_points = ctx->dev_counts ? (int)ctx->cap_points : (int)ctx->np[side];
+    a.n_dev = ctx->dev_counts ? ctx->d_np + side : nullptr;
+    a.max_points = (int)ctx->cap_points;
+    a.grid = ctx->d_grid;
+    a.n_queries = 4 * ctx->bw * ctx->bw;
+    a.n2b = 2 * ctx->bw;
+    a.max_sq = ctx->max_sq;
+    a.n_out_ch = 4;
+    a.out = ctx->d_samples + (size_t)side * 4 * a.n_queries;
+    a.nn_idx = ctx->d_nn[side];
+    a.scratch = (char*)ctx->d_sample_scratch + side * ctx->sample_scratch_stride;
+  }
   {
     ProfScope ps(ctx, st, PS_SAMPLE);
-    CK(launch_sample(a, st));
+    CK(launch_sample(args, n, st));
   }
-  ctx->sampled[side] = true;
+  for (int i = 0; i < n; ++i) ctx->sampled[first + i] = true;
   return PHGPU_OK;
 }
 
@@ -757,7 +763,7 @@ int phgpu_sample_s2(phgpu_ctx* ctx, const phgpu_cloud* cloud, int side) {
   if (!ctx || !cloud || side < 0 || side > 1) return PHGPU_ERR_INVALID;
   cudaSetDevice(ctx->prm.device);
   CKV(phgpu_upload_cloud(ctx, cloud, side, ctx->s0));
-  CKV(run_sample(ctx, side, ctx->s0));
+  CKV(run_sample(ctx, side, 1, ctx->s0));
   CK(cudaStreamSynchronize(ctx->s0));
   return PHGPU_OK;
 }
@@ -1278,8 +1284,7 @@ int phgpu_pair_front(phgpu_ctx* ctx, const PairPlan& pp, bool until_phi) {
   voxels_cleared(ctx, 0);
   CK(cudaEventRecord(ctx->ev_b, s1));
   // rotation up to the fused spectra
-  CKV(run_sample(ctx, 0, s0));
-  CKV(run_sample(ctx, 1, s0));
+  CKV(run_sample(ctx, 0, 2, s0));
   const bool mix = ctx->prm.spherical_fusion == PHGPU_FUSION_MIX;
   if (until_phi) {
     CKV(phgpu_run_sph_phi(ctx, pp.laplace_s2 ? pp.nd_s2 : 1, s0, mix));

@@ -51,7 +51,8 @@ struct phgpu_ctx {
   float4* d_xyzi[2] = {nullptr, nullptr};
   float* d_refl[2] = {nullptr, nullptr};
   float* d_amb[2] = {nullptr, nullptr};
-  void* d_sample_scratch[2] = {nullptr, nullptr};
+  void* d_sample_scratch = nullptr;  // both sides, sample_scratch_stride bytes apart
+  size_t sample_scratch_stride = 0;
   uint32_t* d_lin[2] = {nullptr, nullptr};
   uint32_t np[2] = {0, 0};
   int has_refl[2] = {0, 0}, has_amb[2] = {0, 0};

@@ -40,7 +40,8 @@ struct SampleArgs {
   const uint32_t* n_dev = nullptr;  // when set: the point count is read from device memory (n_points = capacity)
 };
 size_t sampler_scratch_bytes(int max_points, int max_queries);
-cudaError_t launch_sample(const SampleArgs& a, cudaStream_t st);
+// One or two clouds of one grid in one set of launches, each with its own scratch.
+cudaError_t launch_sample(const SampleArgs* a, int n_clouds, cudaStream_t st);
 
 // ------------------------------------------------------------ forward SHT
 // Legendre table: for m in [0,B), l in [m,B), k in [0,2B):

@@ -122,5 +122,5 @@ int phgpu_sample_s2_noalloc(const phgpu_params* params, const phgpu_cloud* cloud
   a.out = values_dev;
   a.nn_idx = nn_index_dev;
   a.scratch = scratch + kGridBytes;
-  return launch_sample(a, st) == cudaSuccess ? PHGPU_OK : PHGPU_ERR_CUDA;
+  return launch_sample(&a, 1, st) == cudaSuccess ? PHGPU_OK : PHGPU_ERR_CUDA;
 }
