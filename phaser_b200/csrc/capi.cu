@@ -470,6 +470,7 @@ static int ensure_cloud_capacity(phgpu_ctx* ctx, uint32_t n) {
     dfree(ctx, ctx->d_refl[s]);
     dfree(ctx, ctx->d_amb[s]);
     dfree(ctx, ctx->d_lin[s]);
+    ctx->lin_points[s] = -1;
     CKV(dalloc(ctx, &ctx->d_xyzi[s], sizeof(float4) * cap));
     CKV(dalloc(ctx, &ctx->d_refl[s], sizeof(float) * cap));
     CKV(dalloc(ctx, &ctx->d_amb[s], sizeof(float) * cap));
@@ -1020,11 +1021,18 @@ static int sp_channels(int has_refl, int has_amb) { return has_amb ? 4 : (has_re
 int phgpu_run_voxelize(phgpu_ctx* ctx, int side, const float* T12, int n_data, cudaStream_t st,
                        const float* T_dev) {
   const size_t nv = (size_t)ctx->N * ctx->N * ctx->N;
-  if (ctx->clean_planes[side] < n_data + 1) {
-    CK(cudaMemsetAsync(ctx->d_grids[side], 0, sizeof(float) * (n_data + 1) * nv, st));
-    CK(cudaMemsetAsync(ctx->d_rowlive[side], 0, (size_t)ctx->N * ctx->N, st));
+  float4* sums = reinterpret_cast<float4*>(ctx->d_grids[side]);
+  float* counts = ctx->d_grids[side] + 4 * nv;
+  if (!ctx->grids_clean[side]) {
+    if (ctx->lin_points[side] >= 0) {
+      CK(launch_clear_voxels(ctx->d_lin[side], (int)ctx->lin_points[side], sums, counts, ctx->d_rowlive[side], ctx->N,
+                             st));
+    } else {
+      CK(cudaMemsetAsync(ctx->d_grids[side], 0, sizeof(float) * 5 * nv, st));
+      CK(cudaMemsetAsync(ctx->d_rowlive[side], 0, (size_t)ctx->N * ctx->N, st));
+    }
   }
-  ctx->clean_planes[side] = 0;
+  ctx->grids_clean[side] = false;
   VoxelArgs v;
   v.xyzi = ctx->d_xyzi[side];
   v.refl = ctx->has_refl[side] ? ctx->d_refl[side] : nullptr;
@@ -1036,7 +1044,8 @@ int phgpu_run_voxelize(phgpu_ctx* ctx, int side, const float* T12, int n_data, c
   v.has_T = T12 ? 1 : 0;
   for (int i = 0; i < 12; ++i) v.T[i] = T12 ? T12[i] : 0.0f;
   v.n_data_ch = n_data;
-  v.grids = ctx->d_grids[side];
+  v.sums = sums;
+  v.counts = counts;
   v.lin_out = ctx->d_lin[side];
   v.rowlive = ctx->d_rowlive[side];
   v.T_dev = T_dev;
@@ -1044,7 +1053,9 @@ int phgpu_run_voxelize(phgpu_ctx* ctx, int side, const float* T12, int n_data, c
     ProfScope ps(ctx, st, PS_VOXELIZE);
     CK(launch_voxelize(v, st));
   }
+  ctx->lin_points[side] = ctx->dev_counts ? -1 : (int64_t)ctx->np[side];
   ctx->vox_ch[side] = n_data;
+  ctx->vox_data[side] = sp_channels(ctx->has_refl[side], ctx->has_amb[side]);
   ctx->voxelized[side] = true;
   ctx->grids_live[side] = true;
   return PHGPU_OK;
@@ -1054,7 +1065,7 @@ int phgpu_run_voxelize(phgpu_ctx* ctx, int side, const float* T12, int n_data, c
 // voxelised side zeroes what the voxelisation wrote (SpatialArgs::clear), so the
 // next voxelisation of this side needs no full-grid memset.
 static void voxels_cleared(phgpu_ctx* ctx, int side) {
-  ctx->clean_planes[side] = ctx->vox_ch[side] + 1;
+  ctx->grids_clean[side] = true;
   ctx->grids_live[side] = false;
 }
 
@@ -1092,7 +1103,6 @@ static SpatialArgs spatial_args(phgpu_ctx* ctx, int n_data, int n_total, int lap
   a.bands = ctx->bands_sp;
   a.grids_f = ctx->d_grids[0];
   a.grids_g = ctx->d_grids[1];
-  a.count_plane = n_data;
   a.grids_are_means = means;
   a.clear = clear;
   for (int s = 0; s < 2; ++s) a.rowlive[s] = ctx->d_rowlive[s];
@@ -1207,7 +1217,8 @@ int phgpu_spatial_correlate(phgpu_ctx* ctx, const double* const* f, const double
   const int laplace = ctx->prm.spatial_fusion == PHGPU_FUSION_LAPLACE ? 1 : 0;
   std::vector<float> tmp(nv);
   for (int side = 0; side < 2; ++side) {
-    ctx->clean_planes[side] = 0;
+    ctx->grids_clean[side] = false;
+    ctx->lin_points[side] = -1;
     ctx->grids_live[side] = false;
     const double* const* src = side == 0 ? f : g;
     for (uint32_t c = 0; c < C; ++c) {
@@ -1228,7 +1239,10 @@ int phgpu_spatial_correlate_voxelized(phgpu_ctx* ctx) {
   }
   cudaSetDevice(ctx->prm.device);
   const int laplace = ctx->prm.spatial_fusion == PHGPU_FUSION_LAPLACE ? 1 : 0;
-  CKV(phgpu_run_spatial(ctx, ctx->vox_ch[0], (int)ctx->prm.n_channels, laplace, 0, ctx->s0));
+  // channels without data on either side are zero: they neither win the
+  // channel maximum nor change the mean's sum
+  const int n_data = std::max(ctx->vox_data[0], ctx->vox_data[1]);
+  CKV(phgpu_run_spatial(ctx, n_data, (int)ctx->prm.n_channels, laplace, 0, ctx->s0));
   CK(cudaStreamSynchronize(ctx->s0));
   return PHGPU_OK;
 }

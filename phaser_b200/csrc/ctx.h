@@ -71,13 +71,17 @@ struct phgpu_ctx {
   size_t* d_class_off = nullptr; // per-class offsets into d_wtable
   float* d_rotvol = nullptr;
   // translation
-  float* d_grids[2] = {nullptr, nullptr};  // [(C+1)][N^3]
+  float* d_grids[2] = {nullptr, nullptr};  // float4 [N^3] channel sums + [N^3] counts, or values [C][N^3] handed in
   uint8_t* d_rowlive[2] = {nullptr, nullptr};  // [N][N] rows holding a point of the last voxelisation
   uint8_t* d_slab_live = nullptr;              // [2][N] z-slabs holding a point of the last forward transform
   uint8_t* d_rowmask = nullptr;  // [2][N][N] row flags of the last forward transform
-  // leading grid planes (and row flags) known to be zero: a voxelisation whose
-  // transform cleared its voxels leaves them zero, so the next one needs no memset
-  int clean_planes[2] = {0, 0};
+  // the grids (and row flags) are known to be zero: a voxelisation whose
+  // transform cleared its voxels leaves them so, and the next one needs no memset
+  bool grids_clean[2] = {false, false};
+  // points of the voxelisation the grids hold, whose indices d_lin still has
+  // (-1: unknown): the next one clears those voxels instead of the whole grid
+  int64_t lin_points[2] = {-1, -1};
+  int vox_data[2] = {0, 0};  // channels that carry data in the last voxelisation
   bool grids_live[2] = {false, false};  // grids hold the last voxelisation (not yet cleared)
   float2* d_spec = nullptr;
   float2* d_cspec = nullptr;

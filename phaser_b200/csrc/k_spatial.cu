@@ -49,55 +49,112 @@ __device__ __forceinline__ int histc_bin(float x, const float* __restrict__ E, i
   return (x == E[l + 1]) ? l + 1 : l;
 }
 
-__global__ void k_voxelize(VoxelArgs a) {
+// A voxel's channel sums lie together (one 16-byte vector atomic per update,
+// one load per voxel later), the point counts in an array of their own (which
+// the row sums scan).  Neighbouring points of a scan mostly share a voxel --
+// near the sensor dozens do, and their atomics on one address serialised (28 us
+// of a sparse scan's 8 us kernel) -- so a warp sums each run of equal voxels
+// with shuffles and the run's last lane issues the atomics.
+__global__ void k_voxelize(const __grid_constant__ VoxelArgs a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int np = a.n_dev ? (int)*a.n_dev : a.n_points;
-  if (i >= np) return;
-  const float4 p = a.xyzi[i];
-  float x = p.x, y = p.y, z = p.z;
-  if (a.has_T || a.T_dev) {
-    // PCL 1.8 transformPointCloud order ((T0 x + T1 y) + T2 z) + T3
-    float Tl[12];
-    if (a.T_dev) {
+  const int lane = threadIdx.x & 31;
+  if (i - lane >= np) return;  // whole warps
+  uint32_t lin = 0xffffffffu;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (i < np) {
+    const float4 p = a.xyzi[i];
+    float x = p.x, y = p.y, z = p.z;
+    if (a.has_T || a.T_dev) {
+      // PCL 1.8 transformPointCloud order ((T0 x + T1 y) + T2 z) + T3
+      float Tl[12];
+      if (a.T_dev) {
 #pragma unroll
-      for (int k = 0; k < 12; ++k) Tl[k] = __ldg(&a.T_dev[k]);
-    } else {
+        for (int k = 0; k < 12; ++k) Tl[k] = __ldg(&a.T_dev[k]);
+      } else {
 #pragma unroll
-      for (int k = 0; k < 12; ++k) Tl[k] = a.T[k];
+        for (int k = 0; k < 12; ++k) Tl[k] = a.T[k];
+      }
+      const float* T = Tl;
+      const float nx = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(T[0], x), __fmul_rn(T[1], y)), __fmul_rn(T[2], z)), T[3]);
+      const float ny = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(T[4], x), __fmul_rn(T[5], y)), __fmul_rn(T[6], z)), T[7]);
+      const float nz = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(T[8], x), __fmul_rn(T[9], y)), __fmul_rn(T[10], z)), T[11]);
+      x = nx;
+      y = ny;
+      z = nz;
     }
-    const float* T = Tl;
-    const float nx = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(T[0], x), __fmul_rn(T[1], y)), __fmul_rn(T[2], z)), T[3]);
-    const float ny = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(T[4], x), __fmul_rn(T[5], y)), __fmul_rn(T[6], z)), T[7]);
-    const float nz = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(T[8], x), __fmul_rn(T[9], y)), __fmul_rn(T[10], z)), T[11]);
-    x = nx;
-    y = ny;
-    z = nz;
+    const uint32_t N = (uint32_t)a.N;
+    const float e0 = __ldg(&a.edges[0]), e1 = __ldg(&a.edges[a.N - 1]);
+    const float inv = a.N > 1 ? (float)(a.N - 1) / (e1 - e0) : 0.0f;
+    const uint32_t bx = (uint32_t)histc_bin(x, a.edges, a.N, e0, e1, inv);
+    const uint32_t by = (uint32_t)histc_bin(y, a.edges, a.N, e0, e1, inv);
+    const uint32_t bz = (uint32_t)histc_bin(z, a.edges, a.N, e0, e1, inv);
+    lin = (bx * N + by) + (N * N * bz);
+    if (lin >= N * N * N) lin = 0xffffffffu;
+    if (a.lin_out) a.lin_out[i] = lin;
+    if (lin != 0xffffffffu) {
+      v.x = p.w;
+      v.y = sqrtf(__fadd_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)), __fmul_rn(z, z)));
+      if (a.n_data_ch > 2 && a.refl) v.z = a.refl[i];
+      if (a.n_data_ch > 3 && a.amb) v.w = a.amb[i];
+    }
   }
-  const uint32_t N = (uint32_t)a.N;
-  const float e0 = __ldg(&a.edges[0]), e1 = __ldg(&a.edges[a.N - 1]);
-  const float inv = a.N > 1 ? (float)(a.N - 1) / (e1 - e0) : 0.0f;
-  const uint32_t bx = (uint32_t)histc_bin(x, a.edges, a.N, e0, e1, inv);
-  const uint32_t by = (uint32_t)histc_bin(y, a.edges, a.N, e0, e1, inv);
-  const uint32_t bz = (uint32_t)histc_bin(z, a.edges, a.N, e0, e1, inv);
-  const uint32_t lin = (bx * N + by) + (N * N * bz);
-  const uint32_t nv = N * N * N;
-  const bool ok = lin < nv;
-  if (a.lin_out) a.lin_out[i] = ok ? lin : 0xffffffffu;
-  if (!ok) return;
+  // runs of equal voxels: sums up to each lane from its run's first lane
+  const uint32_t prev = __shfl_up_sync(0xffffffffu, lin, 1);
+  const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || lin != prev);
+  const int first = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+  if (heads != 0xffffffffu) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float ux = __shfl_up_sync(0xffffffffu, v.x, o), uy = __shfl_up_sync(0xffffffffu, v.y, o);
+      const bool add = lane - o >= first;
+      v.x += add ? ux : 0.f;
+      v.y += add ? uy : 0.f;
+      if (a.n_data_ch > 2) {
+        const float uz = __shfl_up_sync(0xffffffffu, v.z, o);
+        v.z += add ? uz : 0.f;
+      }
+      if (a.n_data_ch > 3) {
+        const float uw = __shfl_up_sync(0xffffffffu, v.w, o);
+        v.w += add ? uw : 0.f;
+      }
+    }
+  }
+  const bool last = lane == 31 || ((heads >> (lane + 1)) & 1u);
+  if (!last || lin == 0xffffffffu) return;
   // the row of lin, not (bz, bx): an out-of-range bin (-1) wraps into another row
-  if (a.rowlive) a.rowlive[lin / N] = 1;
-  float* g = a.grids;
-  atomicAdd(&g[lin], p.w);
-  const float r = sqrtf(__fadd_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)), __fmul_rn(z, z)));
-  atomicAdd(&g[(size_t)nv + lin], r);
-  if (a.n_data_ch > 2) atomicAdd(&g[(size_t)2 * nv + lin], a.refl ? a.refl[i] : 0.0f);
-  if (a.n_data_ch > 3) atomicAdd(&g[(size_t)3 * nv + lin], a.amb ? a.amb[i] : 0.0f);
-  atomicAdd(&g[(size_t)a.n_data_ch * nv + lin], 1.0f);
+  if (a.rowlive) a.rowlive[lin / (uint32_t)a.N] = 1;
+  if (a.n_data_ch > 2)
+    atomicAdd(&a.sums[lin], v);
+  else
+    atomicAdd(reinterpret_cast<float2*>(&a.sums[lin]), make_float2(v.x, v.y));
+  atomicAdd(&a.counts[lin], (float)(lane - first + 1));
 }
 
 cudaError_t launch_voxelize(const VoxelArgs& a, cudaStream_t st) {
   if (a.n_points > 0) {
     k_voxelize<<<(a.n_points + 255) / 256, 256, 0, st>>>(a);
+    count_launches(1);
+  }
+  return cudaGetLastError();
+}
+
+// Zeroes what the voxelisation that left these indices wrote.
+__global__ void k_clear_voxels(const uint32_t* __restrict__ lin, int n_points, float4* __restrict__ sums,
+                               float* __restrict__ counts, uint8_t* __restrict__ rowlive, int N) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_points) return;
+  const uint32_t l = lin[i];
+  if (l == 0xffffffffu || (i > 0 && lin[i - 1] == l)) return;
+  sums[l] = make_float4(0.f, 0.f, 0.f, 0.f);
+  counts[l] = 0.f;
+  rowlive[l / (uint32_t)N] = 0;
+}
+
+cudaError_t launch_clear_voxels(const uint32_t* lin, int n_points, float4* sums, float* counts, uint8_t* rowlive, int N,
+                                cudaStream_t st) {
+  if (n_points > 0) {
+    k_clear_voxels<<<(n_points + 255) / 256, 256, 0, st>>>(lin, n_points, sums, counts, rowlive, N);
     count_launches(1);
   }
   return cudaGetLastError();
@@ -126,9 +183,9 @@ constexpr int kRowsWarps = 4;
 
 struct ScanRowArgs {
   int N;
-  float* grids;         // [channel][N^3] sums
-  const float* tw;      // N complex twiddles
-  size_t count_plane;   // offset of the point counts
+  float4* sums;         // [N^3] channel sums
+  float* counts;        // [N^3] points
+  const float2* tw;     // N twiddles
   uint8_t* rowlive;     // [N (z)][N (x)] rows that hold a point
   uint8_t* rowmask;     // [N][N]: the flags again, kept for the x transform
   float2* spec;         // [channel][z][x][H2p]
@@ -145,7 +202,6 @@ __global__ void __launch_bounds__(kRowsWarps * 32) k_scan_rows(const ScanRowArgs
   constexpr int U = 8, Q = 4;
   const int n = a.N, H2 = n / 2 + 1, H2p = spatial_h2p(n);
   const int z = blockIdx.x, x0 = blockIdx.y * kRowsBlock, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const size_t nv = (size_t)n * n * n;
   const bool mine = lane < kRowsBlock && x0 + lane < n;
   const bool live_l = mine && a.rowlive[(size_t)z * n + x0 + lane];
   const unsigned live = __ballot_sync(0xffffffffu, live_l);  // every warp: the block's rows
@@ -154,7 +210,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32) k_scan_rows(const ScanRowArgs
   float4* s_val = s_mem + (size_t)warp * n;
   float2* s_tw = reinterpret_cast<float2*>(s_mem + (size_t)kRowsWarps * n);
   uint16_t* s_y = reinterpret_cast<uint16_t*>(s_tw + n) + (size_t)warp * n;
-  for (int i = threadIdx.x; i < n; i += kRowsWarps * 32) s_tw[i] = __ldg(reinterpret_cast<const float2*>(a.tw) + i);
+  for (int i = threadIdx.x; i < n; i += kRowsWarps * 32) s_tw[i] = __ldg(a.tw + i);
   __syncthreads();
   if (a.clear && warp == 0 && live_l) a.rowlive[(size_t)z * n + x0 + lane] = 0;
   const uint32_t mul = fast_div_mul(n);
@@ -162,18 +218,16 @@ __global__ void __launch_bounds__(kRowsWarps * 32) k_scan_rows(const ScanRowArgs
   for (unsigned todo = live; todo; todo &= todo - 1) {
     if ((seen++ & (kRowsWarps - 1)) != warp) continue;
     const size_t row = (size_t)z * n + x0 + __ffs(todo) - 1;
-    float* c = a.grids + a.count_plane + row * n;
-    float* g = a.grids + row * n;
+    float* c = a.counts + row * n;
+    float4* g = a.sums + row * n;
     int cnt = 0;
     for (int y0 = 0; y0 < n; y0 += 32 * U) {
       float q[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) q[u] = y0 + 32 * u + lane < n ? c[y0 + 32 * u + lane] : 0.f;
-      float v[CC][U];
+      float4 v[U];
 #pragma unroll
-      for (int ch = 0; ch < CC; ++ch)
-#pragma unroll
-        for (int u = 0; u < U; ++u) v[ch][u] = q[u] > 0.f ? g[ch * nv + y0 + 32 * u + lane] : 0.f;
+      for (int u = 0; u < U; ++u) v[u] = q[u] > 0.f ? g[y0 + 32 * u + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const bool occ = q[u] > 0.f;
@@ -182,12 +236,10 @@ __global__ void __launch_bounds__(kRowsWarps * 32) k_scan_rows(const ScanRowArgs
           const int y = y0 + 32 * u + lane, at = cnt + __popc(m & ((1u << lane) - 1u));
           const float inv = __frcp_rn(q[u]);  // mean = sum * (1 / count)
           s_y[at] = (uint16_t)y;
-          s_val[at] = make_float4(v[0][u] * inv, CC > 1 ? v[CC > 1 ? 1 : 0][u] * inv : 0.f,
-                                  CC > 2 ? v[CC > 2 ? 2 : 0][u] * inv : 0.f, CC > 3 ? v[CC > 3 ? 3 : 0][u] * inv : 0.f);
+          s_val[at] = make_float4(v[u].x * inv, v[u].y * inv, v[u].z * inv, v[u].w * inv);
           if (a.clear) {
             c[y] = 0.f;
-#pragma unroll
-            for (int ch = 0; ch < CC; ++ch) g[ch * nv + y] = 0.f;
+            g[y] = make_float4(0.f, 0.f, 0.f, 0.f);
           }
         }
         cnt += __popc(m);
@@ -889,7 +941,7 @@ cudaError_t launch_spatial_forward(const SpatialArgs& a, int side, cudaStream_t 
     const int tr = pass_threads(*a.plan, kRowPairs, 1, 128, 320);
     PHGPU_DISPATCH_N(N, k_r2c_rows<NF><<<gr, tr, smr, st>>>(N, grids, nv, spec, plane, *a.plan));
   } else {
-    const ScanRowArgs r{N, grids, reinterpret_cast<const float*>(a.plan->tw), (size_t)a.count_plane * nv, a.rowlive[side],
+    const ScanRowArgs r{N, reinterpret_cast<float4*>(grids), grids + 4 * nv, a.plan->tw, a.rowlive[side],
                         a.rowmask + (size_t)side * N * N, spec, plane, a.clear};
     const dim3 gr(N, (N + kRowsBlock - 1) / kRowsBlock);
     const size_t smr = scan_rows_smem(N);

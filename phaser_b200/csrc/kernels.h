@@ -174,13 +174,18 @@ struct VoxelArgs {
   int has_T;
   float T[12];            // 3x4 row-major, applied in PCL order
   int n_data_ch;          // channels accumulated (1..4) in order {int, range, refl, amb}
-  float* grids;           // [n_data_ch + 1][N^3] sums, last = count
+  float4* sums;           // [N^3] sums of {intensity, range, reflectivity, ambient}
+  float* counts;          // [N^3] points
   uint32_t* lin_out;      // optional per-point linear index (or 0xffffffff)
   uint8_t* rowlive;       // optional [N (z)][N (x)]: set to 1 for every row a point lands in
   const float* T_dev = nullptr;     // when set: the 3x4 transform is read from device memory (has_T ignored)
   const uint32_t* n_dev = nullptr;  // when set: the point count is read from device memory (n_points = capacity)
 };
 cudaError_t launch_voxelize(const VoxelArgs& a, cudaStream_t st);
+// Zeroes what one voxelisation wrote: every point's voxel (lin[i] !=
+// 0xffffffff) and row flag.
+cudaError_t launch_clear_voxels(const uint32_t* lin, int n_points, float4* sums, float* counts, uint8_t* rowlive, int N,
+                                cudaStream_t st);
 struct SpatialArgs {
   int N;
   int n_data_ch;          // channels per side with data
@@ -189,10 +194,9 @@ struct SpatialArgs {
   int lowpass;            // 1 (with laplace 0): channel 1, products outside the shifted cube zeroed
   uint32_t lp_lo, lp_hi;  // cube [lp_lo, lp_hi]^3 of subscripts
   FusionBands bands;      // for n = N^3
-  float* grids_f;         // target grids: voxel sums, counts in plane count_plane (or values)
+  float* grids_f;         // target: float4 [N^3] voxel sums, then [N^3] counts (or values [channel][N^3])
   float* grids_g;         // source
-  int count_plane;        // plane of the point counts in the grids
-  int grids_are_means;    // 1: grids already hold values (no count plane)
+  int grids_are_means;    // 1: the grids hold values, channel by channel
   int clear;              // 1: the forward zeroes the voxels and row flags it read
   uint8_t* rowlive[2];    // [N (z)][N (x)] rows that hold a point, per side
   uint8_t* rowmask;       // [2][N (z)][N (x)]: written by the forward of a voxelised side (the row flags, which

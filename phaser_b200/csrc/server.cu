@@ -265,7 +265,7 @@ struct phgpu_server {
           destroy_exec(e);
           return PHGPU_ERR_CUDA;
         }
-        c->clean_planes[s] = 5;
+        c->grids_clean[s] = true;
       }
     }
     if (cudaStreamCreateWithFlags(&e->st, cudaStreamNonBlocking) != cudaSuccess ||

@@ -87,3 +87,28 @@ def test_fast_division_is_exact():
     for d in [*range(2, 130), 201, 255, 256, 257, 511, 512, 513, 1000, 1023, 1024]:
         mul = np.uint64(0xffffffff // d + 1)
         assert np.array_equal((x * mul) >> np.uint64(32), x // np.uint64(d)), d
+
+
+def test_voxels_of_a_smaller_cloud_are_cleared(nat):
+    """A context whose buffers grow between voxelisations, and one that goes from
+    the voxelisation calls to whole registrations and back, must not keep voxels
+    of an earlier cloud."""
+    rng = np.random.default_rng(5)
+    small, large = cloud(rng, 40, 10, n=5), cloud(rng, 40, 10, n=3000)
+    kw = dict(spherical_bandwidth=8, spatial_n_voxels=40, spatial_discretize_lower=-10, spatial_discretize_upper=10,
+              flags=nat.PHGPU_FLAG_KEEP_VOLUMES)
+
+    def volume(c, a, b):
+        c.voxelize(*a, side=0)
+        c.voxelize(*b, side=1)
+        c.spatial_correlate_voxelized()
+        return c.spatial_result(volume=True)[2]
+
+    fresh = volume(nat.Context(**kw), small, large)
+    c = nat.Context(max_points=8, **kw)
+    for a, b in ((small, small), (large, small), (small, large)):
+        vol = volume(c, a, b)
+    np.testing.assert_allclose(vol, fresh, rtol=0, atol=1e-6 * np.abs(fresh).max())
+    c.register_pair(large[:2], small[:2])
+    vol = volume(c, small, large)
+    np.testing.assert_allclose(vol, fresh, rtol=0, atol=1e-6 * np.abs(fresh).max())
