@@ -514,9 +514,9 @@ __global__ void __launch_bounds__(kXThreads, NF > 0 ? 4 : 2) k_fft_x(const __gri
     if (!any && !a.write_empty) return;
   }
   float2* base = a.spec + (size_t)z * n * H2p + ky0;
-  auto at = [=](int, int t, int i, int m) { return SmemCursor{tile + i * W + t, m * W, slot}; };
-  auto sv = [=](int, int t, int i, int m) {
-    float2* p = base + i * H2p + t;
+  auto at = [=](int c, int t, int i, int m) { return SmemCursor{tile + c * slot + i * W + t, m * W, slot}; };
+  auto sv = [=](int g, int t, int i, int m) {
+    float2* p = base + g * stride + i * H2p + t;
     const bool ok = t < wt;
     const int js = m * H2p;
     return [=](int c, int j, float2 v) {
@@ -543,8 +543,8 @@ __global__ void __launch_bounds__(kXThreads, NF > 0 ? 4 : 2) k_fft_x(const __gri
     };
     pass_ct<NF, false, CC, true, 0, -1>(map, a.plan.tw, tid, nthr, ld, at, sv);
   } else {
-    auto ld = [=](int, int t, int i, int m) {
-      const float2* p = base + i * H2p + t;
+    auto ld = [=](int g, int t, int i, int m) {
+      const float2* p = base + g * stride + i * H2p + t;
       const bool ok = t < wt;
       const int js = m * H2p;
       const uint8_t* l = s_live + i;
@@ -556,8 +556,10 @@ __global__ void __launch_bounds__(kXThreads, NF > 0 ? 4 : 2) k_fft_x(const __gri
     };
     if constexpr (NF > 0)
       pass_ct<NF, true, CC, true, 0, -1>(map, a.plan.tw, tid, nthr, ld, at, sv);
-    else
-      pass_rt<INV, CC, false>(a.plan, map, map, map, cs, tid, nthr, ld, at, sv);
+    else {
+      const PassMap ch{CC, LW};  // the channels as groups of transforms
+      pass_rt<INV, 1, false>(a.plan, ch, ch, ch, cs, tid, nthr, ld, at, sv);
+    }
   }
 }
 
@@ -576,20 +578,24 @@ __global__ void __launch_bounds__(kXThreads, NF > 0 ? 4 : 2) k_fft_x(const __gri
 // fusion, and hands the product to the inverse butterfly without a shared
 // round trip.  Slabs without a point (slab_live) are not read.
 
-// Where the fusion rule is one rule over a run of positions [p0, p1]: no band
-// edge lies in (p0, p1].
-__device__ __forceinline__ bool fusion_uniform(uint32_t p0, uint32_t p1, const FusionBands& b) {
-  uint32_t off = 0;
-  bool same = p0 <= p1;
+constexpr int kFuseMixed = 3;  // the rule varies over the run of positions
+// The fusion rule of a run of positions [p0, p1] (p1 < p0: it wraps): one
+// descent of the levels with both ends, which stops at the first level that
+// keeps neither (about two on average).
+__device__ __forceinline__ int fusion_op_run(uint32_t p0, uint32_t p1, const FusionBands& b) {
+  if (p1 < p0) return kFuseMixed;
   for (int l = 0; l < b.levels; ++l) {
-    const uint32_t e0 = off + b.lb[l], e1 = off + b.eub[l], e2 = off + b.sub[l];
-    same = same && !(p0 < e0 && e0 <= p1) && !(p0 < e1 && e1 <= p1) && !(p0 < e2 && e2 <= p1);
-    off = e0;
+    const uint32_t lb = b.lb[l], eub = b.eub[l], sub = b.sub[l];
+    if (p0 >= lb && p1 < eub) {
+      p0 -= lb;
+      p1 -= lb;
+      continue;
+    }
+    if (p1 < lb || (p0 >= eub && p0 >= sub)) return kFuseMax;
+    return p0 >= eub && p1 < sub ? kFuseZero : kFuseMixed;
   }
-  return same;
+  return kFuseMean;
 }
-
-constexpr int kFuseMixed = 3;  // the rule varies over the tile's ky at this position
 
 // Shared-memory element of position i: one extra column group after every
 // R_last positions when R_last is even, so the butterflies of neighbouring
@@ -611,10 +617,23 @@ __host__ __device__ constexpr int z_off(int i) {
     return i;
 }
 
-constexpr int kFuseZMaxThreads = 320;
+// Blocks of up to 320 threads, four to an SM (three for plans that end in
+// radix 8, whose fused middle stage needs 64 registers); runtime plans two of
+// up to 384.
+template <int NF>
+constexpr int fuse_z_max_threads() {
+  return NF > 0 ? 320 : 384;
+}
+template <int NF>
+constexpr int fuse_z_blocks() {
+  if constexpr (NF > 0)
+    return FixedFft<NF>::r[FixedFft<NF>::count - 1] == 8 ? 3 : 4;
+  else
+    return 2;
+}
 // LW >= 0: the tile is 2^LW columns wide; LW < 0: 2^lw_arg.
 template <int NF, int CC, int LW>
-__global__ void __launch_bounds__(kFuseZMaxThreads, NF > 0 ? 4 : 1) k_fuse_z(const __grid_constant__ SpatialArgs a, const __grid_constant__ FftPlan plan, int lw_arg) {
+__global__ void __launch_bounds__(fuse_z_max_threads<NF>(), fuse_z_blocks<NF>()) k_fuse_z(const __grid_constant__ SpatialArgs a, const __grid_constant__ FftPlan plan, int lw_arg) {
   // [CC + 1][z_off(n)][W] | float4 cs[] (runtime plans) | int16 kz[n], uint16 mask[n], uint8 live[2 n], op[n], gop[n]
   extern __shared__ __align__(16) float2 tile[];
   __shared__ FusionBands s_bands;
@@ -653,7 +672,7 @@ __global__ void __launch_bounds__(kFuseZMaxThreads, NF > 0 ? 4 : 1) k_fuse_z(con
     s_live[n + zp] = a.slab_live[n + zp];
     if (a.laplace) {
       const uint32_t p0 = shifted(kz, 0), p1 = shifted(kz, wt - 1);
-      const int op = fusion_uniform(p0, p1, s_bands) ? fusion_op(p0, s_bands) : kFuseMixed;
+      const int op = fusion_op_run(p0, p1, s_bands);
       s_op[zp] = (uint8_t)op;
       if (op != kFuseMax) s_gop[zp / R] = 1;
     }
@@ -775,16 +794,17 @@ __global__ void __launch_bounds__(kFuseZMaxThreads, NF > 0 ? 4 : 1) k_fuse_z(con
         for (int j = 0; j < R; ++j) row[j * W] = F[j];
       }
     } else {
-      const PassMap map{1, lw};
+      // channels as groups of transforms: an item of one channel keeps to the registers of two blocks per SM
+      const PassMap map{CC, lw};
       const uint8_t* live = s_live + side * n;
-      auto ld = [=](int, int t, int i, int m) {
-        const float2* p = src + (size_t)i * zs + t;
+      auto ld = [=](int c, int t, int i, int m) {
+        const float2* p = src + (size_t)c * plane + (size_t)i * zs + t;
         const bool ok = t < wt;
         const size_t js = (size_t)m * zs;
         const uint8_t* l = live + i;
-        return [=](int c, int j) { return ok && l[j * m] ? __ldg(p + c * plane + j * js) : make_float2(0.f, 0.f); };
+        return [=](int, int j) { return ok && l[j * m] ? __ldg(p + j * js) : make_float2(0.f, 0.f); };
       };
-      pass_rt<false, CC, false>(plan, map, map, map, cs, tid, nthr, ld, at, at);
+      pass_rt<false, 1, false>(plan, map, map, map, cs, tid, nthr, ld, at, at);
       __syncthreads();
       for (int it = tid; it < n << lw; it += nthr) {
         const int t = it & (W - 1), i = it >> lw;
@@ -904,19 +924,19 @@ static int fuse_z_tile(int N, int C) {
   return wt;
 }
 
-// Threads of a z-pass block: the least idle time over its stages (an item
-// carries the C channels of a side; the fused middle stage; the product's
-// inverse).
+// Threads of a z-pass block: the least idle time over its stages.  With a
+// compile-time plan an item carries the C channels of a side; runtime plans
+// take the channels as transforms of their own.
 static int fuse_z_threads(const FftPlan& p, int C, int wt) {
+  if (!fixed_length(p.n)) return pass_threads(p, C * wt, 1, 192, fuse_z_max_threads<0>());
   int best = 256;
   double best_cost = 1e300;
-  const int lo = std::min(192, (wt * p.n / std::max(1, p.nstage ? p.radix[0] : 1) + 31) / 32 * 32);
-  for (int t = std::max(lo, 64); t <= kFuseZMaxThreads; t += 32) {
-    auto rounds = [&](int items) { return (double)((items + t - 1) / t) * t; };
+  const int lo = std::min(192, (wt * p.n / p.radix[0] + 31) / 32 * 32);
+  for (int t = std::max(lo, 64); t <= fuse_z_max_threads<64>(); t += 32) {
     double cost = 0.0;
     for (int s = 0; s < p.nstage; ++s) {
-      const int R = p.radix[s], nb = p.n / R;
-      cost += R * (2.0 * C + 1.0) * rounds(wt * nb);
+      const int items = wt * p.n / p.radix[s];
+      cost += p.radix[s] * (2.0 * C + 1.0) * ((items + t - 1) / t) * t;
     }
     if (cost <= best_cost * 1.0001) {
       best_cost = cost;
@@ -963,7 +983,8 @@ cudaError_t launch_spatial_forward(const SpatialArgs& a, int side, cudaStream_t 
     ColArgs cx = c;
     cx.spec += (size_t)ch * plane;
     const int k = std::min(cc, nch - ch);
-    const int tx = pass_threads(*a.plan, 1 << kXFwdLog2, k, 160, kXThreads);
+    const bool fixed = fixed_length(N);  // an item carries all channels, or one of them
+    const int tx = pass_threads(*a.plan, (1 << kXFwdLog2) * (fixed ? 1 : k), fixed ? k : 1, 160, kXThreads);
     FftXFn fn = nullptr;
     PHGPU_DISPATCH_N(N, fn = fft_x_forward<NF>(k));
     fn<<<gx, tx, k * per + extra, st>>>(cx);
