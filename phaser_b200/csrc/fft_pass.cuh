@@ -62,8 +62,9 @@ struct SmemCursor {
 };
 
 // One radix-R stage of NG * groups * 2^lw transforms.  The NG transforms of an
-// item share its index arithmetic and twiddles.
-template <int R, bool INV, int NG, bool ONE, class G, class Ld, class Sv>
+// item share its index arithmetic and twiddles.  PK: packed butterflies
+// (dft_small).
+template <int R, bool INV, int NG, bool ONE, bool PK = true, class G, class Ld, class Sv>
 __device__ __forceinline__ void pass_stage(const G g, PassMap map, const float2* __restrict__ tw, int tid, int nthr,
                                            Ld ld, Sv sv) {
   const int m = g.m();
@@ -100,9 +101,9 @@ __device__ __forceinline__ void pass_stage(const G g, PassMap map, const float2*
 #pragma unroll
           for (int k = 1; k < R; ++k) x[k] = twiddle(x[k], k);
         }
-        dft_small<R, true>(x);
+        dft_small<R, true, PK>(x);
       } else {
-        dft_small<R, false>(x);
+        dft_small<R, false, PK>(x);
         if (m > 1) {
 #pragma unroll
           for (int k = 1; k < R; ++k) x[k] = twiddle(x[k], k);
@@ -261,7 +262,7 @@ __device__ __noinline__ void pass_prime(const FftPlan& p, int s, PassMap map, fl
 // between goes through at (shared memory; ld / sv may be at as well).  I1 < 0:
 // up to the plan's last stage.  A barrier separates the stages; the caller
 // synchronises before reading what sv wrote.  ONE: map.groups = 1.
-template <int NF, bool INV, int NG, bool ONE, int I0, int I1, class Ld, class At, class Sv>
+template <int NF, bool INV, int NG, bool ONE, int I0, int I1, bool PK = true, class Ld, class At, class Sv>
 __device__ __forceinline__ void pass_ct(PassMap map, const float2* __restrict__ tw, int tid, int nthr, Ld ld, At at,
                                         Sv sv) {
   constexpr int cnt = FixedFft<NF>::count;
@@ -271,16 +272,16 @@ __device__ __forceinline__ void pass_ct(PassMap map, const float2* __restrict__ 
     using G = StageC<NF, S>;
     const G g;
     if constexpr (I0 == 0 && cnt == 1) {
-      pass_stage<G::R, INV, NG, ONE>(g, map, tw, tid, nthr, ld, sv);
+      pass_stage<G::R, INV, NG, ONE, PK>(g, map, tw, tid, nthr, ld, sv);
     } else if constexpr (I0 == 0) {
-      pass_stage<G::R, INV, NG, ONE>(g, map, tw, tid, nthr, ld, at);
+      pass_stage<G::R, INV, NG, ONE, PK>(g, map, tw, tid, nthr, ld, at);
     } else if constexpr (I0 == cnt - 1) {
-      pass_stage<G::R, INV, NG, ONE>(g, map, tw, tid, nthr, at, sv);
+      pass_stage<G::R, INV, NG, ONE, PK>(g, map, tw, tid, nthr, at, sv);
     } else {
-      pass_stage<G::R, INV, NG, ONE>(g, map, tw, tid, nthr, at, at);
+      pass_stage<G::R, INV, NG, ONE, PK>(g, map, tw, tid, nthr, at, at);
     }
     if constexpr (I0 + 1 < end) __syncthreads();
-    pass_ct<NF, INV, NG, ONE, I0 + 1, end>(map, tw, tid, nthr, ld, at, sv);
+    pass_ct<NF, INV, NG, ONE, I0 + 1, end, PK>(map, tw, tid, nthr, ld, at, sv);
   }
 }
 

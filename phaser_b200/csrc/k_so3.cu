@@ -27,7 +27,7 @@
 
 #include <vector>
 
-#include "fft2.cuh"
+#include "fft_pass.cuh"
 #include "kernels.h"
 #include "so3_common.cuh"
 
@@ -138,175 +138,176 @@ void so3_beta_table(int bw_out, double* tab) {
 }
 
 // Forward DFT over a (alpha) for one b and a tile of Wt = 2^LOG2W betas
-// (8, 16 or 32: a tuned parameter, 16 by default).
-constexpr int kSo3FftAThreads = 256;
+// (8, 16 or 32: a tuned parameter, 16 by default), in place.  The first stage
+// reads and the last writes S directly (fft_pass.cuh), so a tile crosses
+// shared memory four times instead of eight.  Per-component butterflies with
+// compile-time plans: packed ones round the SO(3) volume differently, and one
+// near-tied pair of the 256-pair batched workload then picked another bin under
+// the tf32x3 synthesis than under FP32 and the FP64 oracle.
+constexpr int kSo3FftAThreads = 320;
 template <int NF, int LOG2W>
-__global__ void k_so3_fft_a(int bw_in, int bw_out, So3Batch bt, FftPlan plan) {
-  extern __shared__ float2 tile[];  // [a][beta tile]
+__global__ void __launch_bounds__(kSo3FftAThreads, NF > 0 ? 4 : 2)
+    k_so3_fft_a(int bw_in, int bw_out, const __grid_constant__ So3Batch bt, const __grid_constant__ FftPlan plan) {
+  extern __shared__ __align__(16) float2 tile[];  // [a][beta tile] | float4 cs[] (runtime plans)
   constexpr int Wt = 1 << LOG2W;
   const int n = NF > 0 ? NF : 2 * bw_out;
   const int Bo = n / 2;
-  const int b = blockIdx.y;
-  const int k0 = blockIdx.x * Wt;
-  const int wt = min(Wt, n - k0);
-  float2* __restrict__ S = bt.out[blockIdx.z].S + (size_t)b * n + k0;
+  const int k0 = blockIdx.x * Wt, wt = min(Wt, n - k0);
+  float2* S = bt.out[blockIdx.z].S + (size_t)blockIdx.y * n + k0;
   const size_t astride = (size_t)Bo * n;
-  // four loads in flight per thread
-  for (int e0 = threadIdx.x; e0 < n * Wt; e0 += 4 * blockDim.x) {
-    float2 v[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int e = e0 + u * blockDim.x;
-      const int a = e / Wt, t = e % Wt;
-      // rows with |m1| >= bw_in are not synthesised: read them as zero
-      const bool row_ok = (a < bw_in) || (a > n - bw_in);
-      v[u] = (e < n * Wt && t < wt && row_ok) ? S[(size_t)a * astride + t] : make_float2(0.f, 0.f);
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (e0 + u * blockDim.x < n * Wt) tile[e0 + u * blockDim.x] = v[u];
-  }
-  __syncthreads();
-  // per-component butterflies (fixed_stage): the packed column-resident form
-  // ran about 1 % faster but rounds the SO(3) volume differently, and one
-  // near-tied pair of the 256-pair batched workload then picked another bin
-  // under the tf32x3 synthesis than under FP32 and the FP64 oracle
-  fft_any<NF, false, LOG2W>(tile, Wt, 1, Wt, plan);
-  for (int e = threadIdx.x; e < n * Wt; e += blockDim.x) {
-    const int a = e / Wt, t = e % Wt;
-    if (t < wt) S[(size_t)a * astride + t] = tile[e];
-  }
+  const int tid = threadIdx.x, nthr = blockDim.x;
+  auto at = [=](int, int t, int i, int m) { return SmemCursor{tile + i * Wt + t, m * Wt, 0}; };
+  auto ld = [=](int, int t, int i, int m) {
+    const float2* p = S + (size_t)i * astride + t;
+    const size_t js = (size_t)m * astride;
+    const bool ok = t < wt;
+    // rows with |m1| >= bw_in are not synthesised: read them as zero
+    return [=](int, int j) {
+      const int a = i + j * m;
+      return ok && (a < bw_in || a > n - bw_in) ? p[j * js] : make_float2(0.f, 0.f);
+    };
+  };
+  auto sv = [=](int, int t, int i, int m) {
+    float2* p = S + (size_t)i * astride + t;
+    const size_t js = (size_t)m * astride;
+    const bool ok = t < wt;
+    return [=](int, int j, float2 v) {
+      if (ok) p[j * js] = v;
+    };
+  };
+  const PassMap map{1, LOG2W};
+  if constexpr (NF > 0)
+    pass_ct<NF, false, 1, true, 0, -1, false>(map, plan.tw, tid, nthr, ld, at, sv);
+  else
+    pass_rt<false, 1, false>(plan, map, map, map, reinterpret_cast<float4*>(tile + (size_t)n * Wt), tid, nthr, ld, at, sv);
 }
 
 // Hermitian complex-to-real transform over gamma, |z|^2 and argmax: one alpha
-// row position and a tile of R betas, one beta per transform (lengths without
-// a register-tail plan).
+// row position and kSo3Pairs pairs of betas.  Betas k and k + 1 are inverted by
+// one complex transform of Z = X0 + i X1, whose output is x0 + i x1 since both
+// spectra are Hermitian: X[b] = conj(u_b), X[n - b] = u_b for 0 < b < n/2; the
+// DC term is taken real (its imaginary part only ever reaches the imaginary
+// output, which the real transform discards) and the Nyquist term is zero.  A
+// pair of betas is one 16-byte load.  The first inverse stage reads S directly
+// (neighbouring threads take neighbouring pairs, 256 contiguous bytes), the
+// last one's outputs go to the argmax without a shared round trip.
+constexpr int kSo3Pairs = 16;
+constexpr int kSo3C2rThreads = 320;
 template <int NF>
-__global__ void k_so3_c2r(int bw_in, int bw_out, So3Batch bt, FftPlan plan) {
-  extern __shared__ float2 rows[];  // [R][n]
-  constexpr int R = 16;
+__global__ void __launch_bounds__(kSo3C2rThreads, NF > 0 ? 3 : 2)
+    k_so3_c2r(int bw_in, int bw_out, const __grid_constant__ So3Batch bt, const __grid_constant__ FftPlan plan) {
+  extern __shared__ __align__(16) float2 zrow[];  // [kSo3Pairs][st] | float4 cs[] | int pos[n] (runtime plans)
   const int n = NF > 0 ? NF : 2 * bw_out;
-  const int Bo = n / 2;
-  const So3Out o = bt.out[blockIdx.z];
+  const int Bo = n / 2, st = n | 1;
+  const So3Out& o = bt.out[blockIdx.z];
   const int r = blockIdx.y;  // alpha row position of the alpha transform's output
-  const int k0 = blockIdx.x * R;
-  const int nk = min(R, n - k0);
-  int* pos = reinterpret_cast<int*>(rows + R * n);  // [n] positions of gamma frequencies
-  for (int e = threadIdx.x; e < R * n; e += blockDim.x) rows[e] = make_float2(0.f, 0.f);
-  for (int b = threadIdx.x; b < n; b += blockDim.x) pos[b] = freq2pos<NF>(b, plan);
-  __syncthreads();
+  const int k0 = blockIdx.x * 2 * kSo3Pairs;
+  const int np = min(kSo3Pairs, (n - k0) / 2);  // n is even
   const int alpha = pos2freq<NF>(r, plan);
-  const float2* __restrict__ Sr = o.S + (size_t)r * Bo * n + k0;
-  for (int e = threadIdx.x; e < Bo * R; e += blockDim.x) {
-    const int b = e / R, j = e - b * R;
-    if (j >= nk) continue;
-    float2* row = rows + j * n;
-    const float2 u = b < bw_in ? Sr[(size_t)b * n + j] : make_float2(0.f, 0.f);
-    row[pos[b]] = cconj(u);
-    if (b > 0) row[pos[n - b]] = u;
-  }
-  __syncthreads();
-  fft_any<NF, true>(rows, R, n, 1, plan);
+  const float2* Sr = o.S + (size_t)r * Bo * n + k0;
+  const int tid = threadIdx.x, nthr = blockDim.x;
+  // Z at gamma frequency k of beta pair pk (mir: k > n / 2, mirrored)
+  auto zval = [=](int pk, int k, bool mir) -> float2 {
+    const int b = mir ? n - k : k;
+    if (b >= bw_in || b == Bo) return make_float2(0.f, 0.f);
+    const float4 w = __ldg(reinterpret_cast<const float4*>(Sr + (size_t)b * n + 2 * pk));
+    if (b == 0) return make_float2(w.x, w.z);
+    return mir ? make_float2(w.x - w.w, w.y + w.z)   // u0 + i u1
+               : make_float2(w.x + w.w, w.z - w.y);  // conj(u0) + i conj(u1)
+  };
   const float K = (float)((1.0 / (double)n) * ((double)Bo / M_PI));
-  unsigned long long best = 0ull;
-  for (int e = threadIdx.x; e < R * n; e += blockDim.x) {
-    const int j = e / n, g = e - j * n;
-    if (j < nk) {
-      const float v = rows[e].x * K;
-      const float v2 = v * v;
-      const uint32_t idx = ((uint32_t)(k0 + j) * n + (uint32_t)alpha) * n + g;
-      const unsigned long long key = pack_argmax(v2, idx);
-      best = key > best ? key : best;
-      if (o.volume) o.volume[idx] = v2;
-    }
-  }
-  warp_argmax_commit(best, o.argmax);
-}
-
-// Betas of one block of the packed transform: two Hermitian sequences per
-// complex transform.
-template <int NF>
-constexpr int c2r_pair_rows() {
-  return (NF % 40 == 0) ? 40 : 32;
-}
-
-// The same C2R for lengths with a register-tail plan: betas k and k + 1 of
-// one alpha are inverted by one complex transform of Z = X0 + i X1, whose
-// output is x0 + i x1 since both spectra are Hermitian.  Sequence X holds
-// X[b] = conj(u_b), X[n - b] = u_b for 0 < b < n/2; its DC term is taken real
-// (its imaginary part only ever reaches the imaginary output, which the real
-// transform discards) and the Nyquist term is zero, as the one-sequence-per-
-// transform kernel above fills it.  A pair of betas is one 16-byte load.
-// Four blocks per SM (64 registers) rather than the three that 74 registers
-// allowed: 0.0488 vs 0.0511 ms for the SO(3) angle transforms at B = 100.
-constexpr int kSo3TailThreads = 256;
-template <int NF>
-__global__ void __launch_bounds__(kSo3TailThreads, 4) k_so3_c2r_tail(int bw_in, So3Batch bt, FftPlan plan) {
-  constexpr int n = NF, Bo = NF / 2, RB = c2r_pair_rows<NF>(), ST = NF + 1;
-  extern __shared__ float2 zrow[];  // [RB / 2][ST]: one beta pair per complex transform
-  __shared__ int s_pos[NF];
-  const So3Out o = bt.out[blockIdx.z];
-  const int r = blockIdx.y;
-  const int k0 = blockIdx.x * RB;
-  const int nk = min(RB, n - k0);
-  const int np = (nk + 1) >> 1;
-  for (int b = threadIdx.x; b < n; b += blockDim.x) s_pos[b] = fixed_freq2pos<NF>(b);
-  __syncthreads();
-  const int alpha = fixed_pos2freq<NF>(r);
-  const float2* __restrict__ Sr = o.S + (size_t)r * Bo * n + k0;
-  constexpr int U = 2;  // loads in flight per thread
-  for (int e0 = threadIdx.x; e0 < np * Bo; e0 += U * blockDim.x) {
-    float4 w[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int e = e0 + u * blockDim.x;
-      const int b = e / np, pp = e - b * np;
-      const bool ok = e < np * Bo && b < bw_in;
-      w[u] = ok ? *reinterpret_cast<const float4*>(Sr + (size_t)b * n + 2 * pp) : make_float4(0.f, 0.f, 0.f, 0.f);
-      if (ok && 2 * pp + 1 >= nk) w[u].z = w[u].w = 0.f;
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int e = e0 + u * blockDim.x;
-      if (e >= np * Bo) continue;
-      const int b = e / np, pp = e - b * np;
-      const float2 u0 = make_float2(w[u].x, w[u].y), u1 = make_float2(w[u].z, w[u].w);
-      float2* z = zrow + pp * ST;
-      if (b == 0) {
-        z[s_pos[0]] = make_float2(u0.x, u1.x);
-        z[s_pos[Bo]] = make_float2(0.f, 0.f);
-      } else {
-        z[s_pos[b]] = make_float2(u0.x + u1.y, u1.x - u0.y);      // conj(u0) + i conj(u1)
-        z[s_pos[n - b]] = make_float2(u0.x - u1.y, u0.y + u1.x);  // u0 + i u1
-      }
-    }
-  }
-  __syncthreads();
-  fft_tail<NF, true, false, true, kSo3TailThreads>(zrow, np, ST, plan.tw);
-  const float K = (float)((1.0 / (double)n) * ((double)Bo / M_PI));
+  float* volume = o.volume;
   // per thread: the largest value, the lowest index among equal ones
   float bv = -1.0f;
   uint32_t bi = 0xffffffffu;
-  for (int e = threadIdx.x; e < np * n; e += blockDim.x) {
-    const int pp = e / n, g = e - pp * n;
-    const float2 z = zrow[pp * ST + g];
+  if constexpr (NF > 0) {
+    constexpr int cnt = FixedFft<NF>::count;
+    constexpr int R = FixedFft<NF>::r[cnt - 1], nb = NF / R;
+    for (int it = tid; it < kSo3Pairs * nb; it += nthr) {
+      const int pk = it % kSo3Pairs, b = it / kSo3Pairs;
+      if (pk >= np) continue;
+      float2 x[R];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int j = 2 * pp + h;
-      if (j < nk) {
-        const float v = (h ? z.y : z.x) * K;
-        const float v2 = v * v;
-        const uint32_t idx = ((uint32_t)(k0 + j) * n + (uint32_t)alpha) * n + g;
-        if (v2 > bv || (v2 == bv && idx < bi)) {
-          bv = v2;
-          bi = idx;
-        }
-        if (o.volume) o.volume[idx] = v2;
+      for (int i = 0; i < R; ++i) {
+        const bool below = 2 * (i * nb + nb - 1) < NF, above = 2 * i * nb > NF;
+        const int k = b + i * nb;
+        x[i] = zval(pk, k, above || (!below && 2 * k > NF));
       }
+      dft_small<R, true>(x);
+      float2* d = zrow + pk * st + fixed_freq2pos<NF>(b);
+#pragma unroll
+      for (int i = 0; i < R; ++i) d[i] = x[i];
     }
+    __syncthreads();
+    const int lwp = 32 - __clz(np - 1);
+    auto at = [=](int g, int t, int i, int m) { return SmemCursor{zrow + (g + t) * st + i, m, 0}; };
+    pass_ct<NF, true, 1, true, 1, cnt - 1>(PassMap{1, lwp}, plan.tw, tid, nthr, at, at, at);
+    if constexpr (cnt > 2) __syncthreads();
+    constexpr int R0 = FixedFft<NF>::r[0], m = NF / R0;
+    for (int it = tid; it < np * m; it += nthr) {
+      const int pk = it / m, j2 = it - pk * m;
+      const float2* row = zrow + pk * st + j2;
+      float2 x[R0];
+#pragma unroll
+      for (int j = 0; j < R0; ++j) x[j] = row[j * m];
+#pragma unroll
+      for (int k = 1; k < R0; ++k) x[k] = cmul(x[k], cconj(__ldg(plan.tw + j2 * k)));
+      dft_small<R0, true>(x);
+      const uint32_t idx = ((uint32_t)(k0 + 2 * pk) * n + (uint32_t)alpha) * n + j2;
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int j = 0; j < R0; ++j) {
+          const float v = (h ? x[j].y : x[j].x) * K, v2 = v * v;
+          const uint32_t id = idx + h * (uint32_t)(n * n) + j * m;
+          if (v2 > bv || (v2 == bv && id < bi)) {
+            bv = v2;
+            bi = id;
+          }
+          if (volume) volume[id] = v2;
+        }
+    }
+  } else {
+    float4* cs = reinterpret_cast<float4*>(zrow + (size_t)kSo3Pairs * st);
+    int* pos = reinterpret_cast<int*>(cs + kMaxGenericRadix);
+    for (int k = tid; k < n; k += nthr) pos[k] = freq2pos<NF>(k, plan);
+    __syncthreads();
+    for (int it = tid; it < kSo3Pairs * (Bo + 1); it += nthr) {
+      const int pk = it % kSo3Pairs, b = it / kSo3Pairs;
+      if (pk >= np) continue;
+      zrow[pk * st + pos[b]] = zval(pk, b, false);
+      if (b > 0 && b < Bo) zrow[pk * st + pos[n - b]] = zval(pk, n - b, true);
+    }
+    __syncthreads();
+    const int lwp = 32 - __clz(np - 1);
+    auto at = [=](int g, int t, int i, int m) { return SmemCursor{zrow + (g + t) * st + i, m, 0}; };
+    auto sv = [=, &bv, &bi](int g, int t, int i, int m) {
+      const uint32_t idx = ((uint32_t)(k0 + 2 * (g + t)) * n + (uint32_t)alpha) * n + i;
+      return [=, &bv, &bi](int, int j, float2 z) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float v = (h ? z.y : z.x) * K, v2 = v * v;
+          const uint32_t id = idx + h * (uint32_t)(n * n) + j * m;
+          if (v2 > bv || (v2 == bv && id < bi)) {
+            bv = v2;
+            bi = id;
+          }
+          if (volume) volume[id] = v2;
+        }
+      };
+    };
+    pass_rt<true, 1, true>(plan, PassMap{1, lwp}, PassMap{1, lwp}, PassMap{np, 0}, cs, tid, nthr, at, at, sv);
   }
   warp_argmax_commit(bi == 0xffffffffu ? 0ull : pack_argmax(bv, bi), o.argmax);
 }
+
+static bool so3_fixed_length(int n) {
+  bool fixed = false;
+  PHGPU_DISPATCH_N(n, fixed = NF > 0);
+  return fixed;
+}
+// Shared memory beyond the tile: the prime-radix scratch of runtime plans.
+static size_t so3_prime_scratch(int n) { return so3_fixed_length(n) ? 0 : kMaxGenericRadix * sizeof(float4); }
 
 template <int NF>
 static cudaError_t so3_attrs() {
@@ -315,11 +316,6 @@ static cudaError_t so3_attrs() {
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_so3_fft_a<NF, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, m);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_so3_fft_a<NF, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, m);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_so3_c2r<NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, m);
-  if constexpr (Tail<NF>::ok) {
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_so3_c2r_tail<NF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (c2r_pair_rows<NF>() / 2) * (NF + 1) * (int)sizeof(float2));
-  }
   return e;
 }
 
@@ -342,36 +338,31 @@ cudaError_t launch_so3_synth(const So3Args& a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// The gamma transform: packed pairs on the register-tail engine where the
-// length has a tail plan, one sequence per transform otherwise.
 template <int NF>
 static void launch_so3_c2r(const So3Args& a, int n, cudaStream_t st) {
-  if constexpr (Tail<NF>::ok) {
-    constexpr int RB = c2r_pair_rows<NF>();
-    dim3 g((n + RB - 1) / RB, n, a.batch.count);
-    k_so3_c2r_tail<NF><<<g, kSo3TailThreads, (size_t)(RB / 2) * (NF + 1) * sizeof(float2), st>>>(a.bw_in, a.batch,
-                                                                                               *a.plan);
-  } else {
-    dim3 g((n + 15) / 16, n, a.batch.count);
-    k_so3_c2r<NF><<<g, 256, (size_t)16 * n * sizeof(float2) + (size_t)n * sizeof(int), st>>>(a.bw_in, a.bw_out,
-                                                                                            a.batch, *a.plan);
-  }
+  const dim3 g((n + 2 * kSo3Pairs - 1) / (2 * kSo3Pairs), n, a.batch.count);
+  size_t sm = (size_t)kSo3Pairs * (n | 1) * sizeof(float2);
+  if (NF == 0) sm += so3_prime_scratch(n) + (size_t)n * sizeof(int);
+  k_so3_c2r<NF><<<g, pass_threads(*a.plan, kSo3Pairs, 1, 160, kSo3C2rThreads), sm, st>>>(a.bw_in, a.bw_out, a.batch,
+                                                                                        *a.plan);
 }
 
 template <int NF>
 static void launch_so3_fft_a(const So3Args& a, int n, int wt, cudaStream_t st) {
-  dim3 g((n + wt - 1) / wt, a.bw_in, a.batch.count);
-  const size_t sm = (size_t)n * wt * sizeof(float2);
+  const dim3 g((n + wt - 1) / wt, a.bw_in, a.batch.count);
+  const size_t sm = (size_t)n * wt * sizeof(float2) + so3_prime_scratch(n);
+  const int thr = pass_threads(*a.plan, wt, 1, 160, kSo3FftAThreads);
   if (wt == 8)
-    k_so3_fft_a<NF, 3><<<g, kSo3FftAThreads, sm, st>>>(a.bw_in, a.bw_out, a.batch, *a.plan);
+    k_so3_fft_a<NF, 3><<<g, thr, sm, st>>>(a.bw_in, a.bw_out, a.batch, *a.plan);
   else if (wt == 32)
-    k_so3_fft_a<NF, 5><<<g, kSo3FftAThreads, sm, st>>>(a.bw_in, a.bw_out, a.batch, *a.plan);
+    k_so3_fft_a<NF, 5><<<g, thr, sm, st>>>(a.bw_in, a.bw_out, a.batch, *a.plan);
   else
-    k_so3_fft_a<NF, 4><<<g, kSo3FftAThreads, sm, st>>>(a.bw_in, a.bw_out, a.batch, *a.plan);
+    k_so3_fft_a<NF, 4><<<g, thr, sm, st>>>(a.bw_in, a.bw_out, a.batch, *a.plan);
 }
 
 bool so3_beta_tile_ok(int bw_out, int wt) {
-  return (wt == 8 || wt == 16 || wt == 32) && (size_t)2 * bw_out * wt * sizeof(float2) <= 227u * 1024u;
+  return (wt == 8 || wt == 16 || wt == 32) &&
+         (size_t)2 * bw_out * wt * sizeof(float2) + so3_prime_scratch(2 * bw_out) <= 227u * 1024u;
 }
 
 cudaError_t launch_so3_fft(const So3Args& a, cudaStream_t st) {

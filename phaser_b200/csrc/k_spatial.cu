@@ -740,7 +740,15 @@ __global__ void __launch_bounds__(fuse_z_max_threads<NF>(), fuse_z_blocks<NF>())
         const size_t js = (size_t)m * zs;
         return [=](int c, int j) { return (k >> j) & 1u ? __ldg(p + c * plane + j * js) : make_float2(0.f, 0.f); };
       };
-      pass_ct<NF, false, CC, true, 0, cnt - 1>(PassMap{1, lw}, plan.tw, tid, nthr, ld, at, at);
+      // the first stage's items are one channel's (they are the fewest: n / R0 butterflies a column), the others'
+      // all channels'
+      auto ld1 = [=](int c, int t, int i, int m) {
+        const auto f = ld(0, t, i, m);
+        return [=](int, int j) { return f(c, j); };
+      };
+      pass_ct<NF, false, 1, false, 0, 1>(PassMap{CC, lw}, plan.tw, tid, nthr, ld1, at, at);
+      if constexpr (cnt > 2) __syncthreads();
+      pass_ct<NF, false, CC, true, 1, cnt - 1>(PassMap{1, lw}, plan.tw, tid, nthr, at, at, at);
       __syncthreads();
       for (int it = tid; it < (n / R) << lw; it += nthr) {
         const int t = it & (W - 1), g = it >> lw, i0 = g * R;
