@@ -466,6 +466,11 @@ static int ensure_cloud_capacity(phgpu_ctx* ctx, uint32_t n) {
   if (n <= ctx->cap_points) return PHGPU_OK;
   uint32_t cap = std::max<uint32_t>(n, ctx->cap_points * 2);
   for (int s = 0; s < 2; ++s) {
+    // what the kernels read follows the context's own buffers (a server's slots are captured before their first
+    // upload); a caller's cloud taken in place stays
+    const bool own_xyzi = !ctx->use_xyzi[s] || ctx->use_xyzi[s] == ctx->d_xyzi[s];
+    const bool own_refl = !ctx->use_refl[s] || ctx->use_refl[s] == ctx->d_refl[s];
+    const bool own_amb = !ctx->use_amb[s] || ctx->use_amb[s] == ctx->d_amb[s];
     dfree(ctx, ctx->d_xyzi[s]);
     dfree(ctx, ctx->d_refl[s]);
     dfree(ctx, ctx->d_amb[s]);
@@ -475,6 +480,9 @@ static int ensure_cloud_capacity(phgpu_ctx* ctx, uint32_t n) {
     CKV(dalloc(ctx, &ctx->d_refl[s], sizeof(float) * cap));
     CKV(dalloc(ctx, &ctx->d_amb[s], sizeof(float) * cap));
     CKV(dalloc(ctx, &ctx->d_lin[s], sizeof(uint32_t) * cap));
+    if (own_xyzi) ctx->use_xyzi[s] = ctx->d_xyzi[s];
+    if (own_refl) ctx->use_refl[s] = ctx->d_refl[s];
+    if (own_amb) ctx->use_amb[s] = ctx->d_amb[s];
   }
   dfree(ctx, ctx->d_sample_scratch);
   ctx->sample_scratch_stride = (sampler_scratch_bytes((int)cap, 4 * ctx->bw * ctx->bw) + 255) & ~(size_t)255;
@@ -711,16 +719,39 @@ int phgpu_ctx_destroy(phgpu_ctx* ctx) {
 
 // ------------------------------------------------------------------ stages
 
+// Whether a kernel of this context may read `p` in place: memory of its own
+// device, aligned for the loads.
+static bool readable_in_place(const phgpu_ctx* ctx, const void* p, size_t align) {
+  if ((reinterpret_cast<uintptr_t>(p) & (align - 1)) != 0) return false;
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeDevice && at.device == ctx->prm.device;
+}
+
+// Makes a cloud readable by the kernels of a call: host memory (and device
+// memory of another GPU) is copied into the context's buffers; a device cloud
+// is read where it lies, since the calls that take one return only when they
+// have finished with it.  A server's slots always copy (their captured graphs
+// read fixed addresses).
 int phgpu_upload_cloud(phgpu_ctx* ctx, const phgpu_cloud* c, int side, cudaStream_t st) {
   CKV(ensure_cloud_capacity(ctx, c->n_points));
   const cudaMemcpyKind kind = c->on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-  if (c->n_points) {
-    CK(cudaMemcpyAsync(ctx->d_xyzi[side], c->xyzi, sizeof(float4) * c->n_points, kind, st));
-    if (c->reflectivity)
-      CK(cudaMemcpyAsync(ctx->d_refl[side], c->reflectivity, sizeof(float) * c->n_points, kind, st));
-    if (c->ambient)
-      CK(cudaMemcpyAsync(ctx->d_amb[side], c->ambient, sizeof(float) * c->n_points, kind, st));
-  }
+  auto bring = [&](const float* from, void* own, size_t floats, size_t align, const void** use) -> int {
+    *use = own;
+    if (!from || !c->n_points) return PHGPU_OK;
+    if (c->on_device && !ctx->dev_counts && readable_in_place(ctx, from, align)) {
+      *use = from;
+      return PHGPU_OK;
+    }
+    CK(cudaMemcpyAsync(own, from, sizeof(float) * floats * c->n_points, kind, st));
+    return PHGPU_OK;
+  };
+  CKV(bring(c->xyzi, ctx->d_xyzi[side], 4, 16, (const void**)&ctx->use_xyzi[side]));
+  CKV(bring(c->reflectivity, ctx->d_refl[side], 1, 4, (const void**)&ctx->use_refl[side]));
+  CKV(bring(c->ambient, ctx->d_amb[side], 1, 4, (const void**)&ctx->use_amb[side]));
   ctx->np[side] = c->n_points;
   ctx->has_refl[side] = c->reflectivity != nullptr;
   ctx->has_amb[side] = c->ambient != nullptr;
@@ -737,9 +768,9 @@ static int run_sample(phgpu_ctx* ctx, int first, int n, cudaStream_t st) {
   for (int i = 0; i < n; ++i) {
     const int side = first + i;
     SampleArgs& a = args[i];
-    a.xyzi = ctx->d_xyzi[side];
-    a.refl = ctx->has_refl[side] ? ctx->d_refl[side] : nullptr;
-    a.amb = ctx->has_amb[side] ? ctx->d_amb[side] : nullptr;
+    a.xyzi = ctx->use_xyzi[side];
+    a.refl = ctx->has_refl[side] ? ctx->use_refl[side] : nullptr;
+    a.amb = ctx->has_amb[side] ? ctx->use_amb[side] : nullptr;
     a.n_points = ctx->dev_counts ? (int)ctx->cap_points : (int)ctx->np[side];
     a.n_dev = ctx->dev_counts ? ctx->d_np + side : nullptr;
     a.max_points = (int)ctx->cap_points;
@@ -762,6 +793,7 @@ static int run_sample(phgpu_ctx* ctx, int first, int n, cudaStream_t st) {
 
 int phgpu_sample_s2(phgpu_ctx* ctx, const phgpu_cloud* cloud, int side) {
   if (!ctx || !cloud || side < 0 || side > 1) return PHGPU_ERR_INVALID;
+  ChainScope chain(true);
   cudaSetDevice(ctx->prm.device);
   CKV(phgpu_upload_cloud(ctx, cloud, side, ctx->s0));
   CKV(run_sample(ctx, side, 1, ctx->s0));
@@ -956,6 +988,7 @@ int phgpu_sph_correlate(phgpu_ctx* ctx, const double* const* f, const double* co
     if (ctx) ctx->err = "phgpu_sph_correlate: 1..4 channels required";
     return PHGPU_ERR_INVALID;
   }
+  ChainScope chain(true);
   cudaSetDevice(ctx->prm.device);
   const size_t nq = (size_t)4 * ctx->bw * ctx->bw;
   std::vector<float> tmp(2 * 4 * nq, 0.0f);
@@ -977,6 +1010,7 @@ int phgpu_sph_correlate_sampled(phgpu_ctx* ctx) {
     ctx->err = "both sides must be sampled first";
     return PHGPU_ERR_STATE;
   }
+  ChainScope chain(true);
   cudaSetDevice(ctx->prm.device);
   const int nd = std::max(ctx->has_amb[0] || ctx->has_amb[1] ? 4 : 0,
                           ctx->has_refl[0] || ctx->has_refl[1] ? 3 : 2);
@@ -1034,9 +1068,9 @@ int phgpu_run_voxelize(phgpu_ctx* ctx, int side, const float* T12, int n_data, c
   }
   ctx->grids_clean[side] = false;
   VoxelArgs v;
-  v.xyzi = ctx->d_xyzi[side];
-  v.refl = ctx->has_refl[side] ? ctx->d_refl[side] : nullptr;
-  v.amb = ctx->has_amb[side] ? ctx->d_amb[side] : nullptr;
+  v.xyzi = ctx->use_xyzi[side];
+  v.refl = ctx->has_refl[side] ? ctx->use_refl[side] : nullptr;
+  v.amb = ctx->has_amb[side] ? ctx->use_amb[side] : nullptr;
   v.n_points = ctx->dev_counts ? (int)ctx->cap_points : (int)ctx->np[side];
   v.n_dev = ctx->dev_counts ? ctx->d_np + side : nullptr;
   v.N = ctx->N;
@@ -1071,6 +1105,7 @@ static void voxels_cleared(phgpu_ctx* ctx, int side) {
 
 int phgpu_voxelize(phgpu_ctx* ctx, const phgpu_cloud* cloud, int side, const float* T12) {
   if (!ctx || !cloud || side < 0 || side > 1) return PHGPU_ERR_INVALID;
+  ChainScope chain(true);
   cudaSetDevice(ctx->prm.device);
   CKV(phgpu_upload_cloud(ctx, cloud, side, ctx->s0));
   CKV(phgpu_run_voxelize(ctx, side, T12, 4, ctx->s0));
@@ -1212,6 +1247,7 @@ int phgpu_spatial_correlate(phgpu_ctx* ctx, const double* const* f, const double
     ctx->err = "the low-pass spatial correlation uses channel 1: at least 2 channels required";
     return PHGPU_ERR_INVALID;
   }
+  ChainScope chain(true);
   cudaSetDevice(ctx->prm.device);
   const size_t nv = (size_t)ctx->N * ctx->N * ctx->N;
   const int laplace = ctx->prm.spatial_fusion == PHGPU_FUSION_LAPLACE ? 1 : 0;
@@ -1237,6 +1273,7 @@ int phgpu_spatial_correlate_voxelized(phgpu_ctx* ctx) {
     ctx->err = "both sides must be voxelised (phgpu_voxelize) with the same channel count first";
     return PHGPU_ERR_STATE;
   }
+  ChainScope chain(true);
   cudaSetDevice(ctx->prm.device);
   const int laplace = ctx->prm.spatial_fusion == PHGPU_FUSION_LAPLACE ? 1 : 0;
   // channels without data on either side are zero: they neither win the
@@ -1411,10 +1448,13 @@ bool pair_device_pose(const phgpu_ctx* ctx) { return ctx->prm.rot_peak_neighbors
 int phgpu_register_pair(phgpu_ctx* ctx, const phgpu_cloud* target, const phgpu_cloud* source,
                         phgpu_pose* out) {
   if (!ctx || !target || !source || !out) return PHGPU_ERR_INVALID;
+  ChainScope chain(true);
   cudaSetDevice(ctx->prm.device);
   cudaStream_t s0 = ctx->s0;
   {
     ProfScope ps(ctx, s0, PS_UPLOAD);
+    // room for both first: growing for the source would lose the uploaded target
+    CKV(ensure_cloud_capacity(ctx, std::max(target->n_points, source->n_points)));
     CKV(phgpu_upload_cloud(ctx, target, 0, s0));
     CKV(phgpu_upload_cloud(ctx, source, 1, s0));
   }

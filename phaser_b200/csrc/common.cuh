@@ -78,6 +78,15 @@ __device__ __forceinline__ void warp_argmax_commit(unsigned long long key, unsig
   if ((threadIdx.x & 31) == 0) atomicMax(dst, key);
 }
 
+// First statement of every kernel of the registration chain: lets the next
+// kernel of the stream be set up while this one runs, and waits until the
+// kernels before it have finished (with all their writes).  Without the
+// launch attribute (launch_kernel in kernels.h) both do nothing.
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Complex sums as packed FP32 pairs (one FADD2 / FFMA2 for both components).
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }

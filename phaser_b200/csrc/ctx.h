@@ -51,6 +51,10 @@ struct phgpu_ctx {
   float4* d_xyzi[2] = {nullptr, nullptr};
   float* d_refl[2] = {nullptr, nullptr};
   float* d_amb[2] = {nullptr, nullptr};
+  // what the running call's kernels read: the buffers above, or a caller's device cloud in place
+  const float4* use_xyzi[2] = {nullptr, nullptr};
+  const float* use_refl[2] = {nullptr, nullptr};
+  const float* use_amb[2] = {nullptr, nullptr};
   void* d_sample_scratch = nullptr;  // both sides, sample_scratch_stride bytes apart
   size_t sample_scratch_stride = 0;
   uint32_t* d_lin[2] = {nullptr, nullptr};

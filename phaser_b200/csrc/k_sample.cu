@@ -71,6 +71,7 @@ struct CloudPair {
 
 // Projection of every point, its bin and the per-bin and per-row counts.
 __global__ void k_project(const __grid_constant__ CloudPair pr, int n2b) {
+  chain_begin();
   const CloudView& v = pr.c[blockIdx.y];
   float4* __restrict__ proj = v.proj;
   double* __restrict__ range = v.range;
@@ -135,6 +136,7 @@ constexpr int kMaxGridSide = 1024;  // 2B for B <= 512
 // (hav_tab[0] = 0), stq_tab[i] = sin((i + 1/2) w) - 1e-5 (clamped at 0) for the
 // direction rows, w = pi / 2B.
 __global__ void __launch_bounds__(kBinScanThreads) k_bin_scan(int n2b, const __grid_constant__ CloudPair pr) {
+  chain_begin();
   const CloudView& v0 = pr.c[blockIdx.y];
   const uint32_t* __restrict__ bin_count = v0.bin_count;
   const uint32_t* __restrict__ row_count = v0.row_count;
@@ -221,6 +223,7 @@ __global__ void __launch_bounds__(kBinScanThreads) k_bin_scan(int n2b, const __g
 
 // Counting-sort scatter: sorted[k] = {x, y, z, point index (bits)}.
 __global__ void k_bin_scatter(const __grid_constant__ CloudPair pr) {
+  chain_begin();
   const CloudView& v = pr.c[blockIdx.y];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (v.P_dev ? (int)*v.P_dev : v.P)) return;
@@ -385,6 +388,7 @@ constexpr int kQueryThreads = 256;
 // clouds: 70 -> 22 us.
 __global__ void __launch_bounds__(kQueryThreads, 6)
 k_nn_rows(int n2b, uint32_t mul_n2b, const __grid_constant__ CloudPair pr) {
+  chain_begin();
   const CloudView& v = pr.c[blockIdx.y];
   const float4* __restrict__ sorted = v.sorted;
   const uint32_t* __restrict__ bin_start = v.bin_start;
@@ -459,6 +463,7 @@ k_nn_rows(int n2b, uint32_t mul_n2b, const __grid_constant__ CloudPair pr) {
 
 std::atomic<unsigned long long> g_launch_count{0};
 thread_local int g_capture_depth = 0;
+thread_local bool g_chain_launch = false;
 
 namespace {
 int grid_side(int max_queries) {
@@ -539,17 +544,17 @@ cudaError_t launch_sample(const SampleArgs* args, int n_clouds, cudaStream_t st)
   int launched = 0;
   const dim3 gp((P + 255) / 256, n_clouds);
   if (P > 0) {
-    k_project<<<gp, 256, 0, st>>>(pr, n2b);
+    launch_kernel(k_project, dim3(gp), dim3(256), 0, st, pr, n2b);
     ++launched;
   }
-  k_bin_scan<<<dim3(n2b, n_clouds), kBinScanThreads, 0, st>>>(n2b, pr);
+  launch_kernel(k_bin_scan, dim3(n2b, n_clouds), dim3(kBinScanThreads), 0, st, n2b, pr);
   ++launched;
   if (P > 0) {
-    k_bin_scatter<<<gp, 256, 0, st>>>(pr);
+    launch_kernel(k_bin_scatter, dim3(gp), dim3(256), 0, st, pr);
     ++launched;
   }
   const size_t q_threads = nbins * kGroup;
-  k_nn_rows<<<dim3((unsigned)((q_threads + kQueryThreads - 1) / kQueryThreads), n_clouds), kQueryThreads, 0, st>>>(
+  launch_kernel(k_nn_rows, dim3((unsigned)((q_threads + kQueryThreads - 1) / kQueryThreads), n_clouds), dim3(kQueryThreads), 0, st, 
       n2b, fast_div_mul((uint32_t)n2b), pr);
   ++launched;
   count_launches(launched);

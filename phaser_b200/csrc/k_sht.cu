@@ -102,6 +102,7 @@ template <int NF>
 __global__ void __launch_bounds__(kPhiThreads) k_sht_phi(int bw, int n_data, size_t side_stride,
                                                          const float* __restrict__ sig, FftPlan plan,
                                                          float2* __restrict__ fphi) {
+  chain_begin();
   extern __shared__ float2 zr[];  // [kPhiRows / 2][n] packed row pairs
   const int n = 2 * bw;
   const int s = blockIdx.y, side = s / n_data, c = s - side * n_data;
@@ -162,6 +163,7 @@ __device__ __forceinline__ void cp_async_wait() {
 __global__ void __launch_bounds__(kLegThreads) k_sht_leg(int bw, int n_data, int cr, int nslot,
                                                          const float* __restrict__ table,
                                                          const float2* __restrict__ fphi, float2* __restrict__ coef) {
+  chain_begin();
   extern __shared__ float2 sh[];
   const int n = 2 * bw;
   const int rs = n + 2;  // table row stride in shared memory (8-byte aligned, conflict-free 8-byte reads)
@@ -298,7 +300,7 @@ cudaError_t launch_sht_phi(const ShtArgs& a, cudaStream_t st) {
   if (a.plan->n != n) return cudaErrorInvalidValue;
   dim3 g1((n + kPhiRows - 1) / kPhiRows, 2 * a.n_data);
   const size_t sm1 = (size_t)(kPhiRows / 2) * n * sizeof(float2);
-  PHGPU_DISPATCH_N(n, k_sht_phi<NF><<<g1, kPhiThreads, sm1, st>>>(a.bw, a.n_data, a.side_stride, a.signal,
+  PHGPU_DISPATCH_N(n, launch_kernel(k_sht_phi<NF>, dim3(g1), dim3(kPhiThreads), sm1, st, a.bw, a.n_data, a.side_stride, a.signal,
                                                                    *a.plan, a.fphi));
   count_launches(1);
   return cudaGetLastError();
@@ -319,7 +321,7 @@ cudaError_t launch_sht(const ShtArgs& a, cudaStream_t st) {
     return launch_sht_leg_tc(a.bw, a.n_data, b, a.table_tc, a.precision, a.tc_chunk, a.status, st);
   }
   dim3 g2((a.bw + 1) / 2, 2);
-  k_sht_leg<<<g2, kLegThreads, sm, st>>>(a.bw, a.n_data, cr, nslot, a.table, a.fphi, a.coef);
+  launch_kernel(k_sht_leg, dim3(g2), dim3(kLegThreads), sm, st, a.bw, a.n_data, cr, nslot, a.table, a.fphi, a.coef);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -425,6 +427,7 @@ struct LegendreGemm {
 
 template <int PREC>
 __global__ void __launch_bounds__(kTcThreads, kTcCtasPerSm) k_sht_leg_tc(TcGemmArgs g, LegendreGemm prob) {
+  chain_begin();
   tc_class_gemm<PREC>(g, prob);
 }
 
@@ -451,9 +454,9 @@ cudaError_t launch_sht_leg_tc(int bw, int n_data, const ShtBatch& b, const float
   prob.b = b;
   const int grid = bw < sms * g.ctas_per_sm ? bw : sms * g.ctas_per_sm;
   if (precision == kSo3Tf32x3)
-    k_sht_leg_tc<kSo3Tf32x3><<<grid, kTcThreads, g.smem, st>>>(g, prob);
+    launch_kernel(k_sht_leg_tc<kSo3Tf32x3>, dim3(grid), dim3(kTcThreads), g.smem, st, g, prob);
   else
-    k_sht_leg_tc<kSo3Bf16x3><<<grid, kTcThreads, g.smem, st>>>(g, prob);
+    launch_kernel(k_sht_leg_tc<kSo3Bf16x3>, dim3(grid), dim3(kTcThreads), g.smem, st, g, prob);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -473,6 +476,7 @@ __device__ __forceinline__ float2 coef_at(const float2* __restrict__ c, int bw, 
 
 // One thread per (l, m) with |m| <= l; both sides; request blockIdx.y.
 __global__ void k_fuse_s2(FuseS2Args a) {
+  chain_begin();
   const int bw = a.bw;
   const float2* __restrict__ coef = a.coef_b[blockIdx.y];
   float2* __restrict__ fused = a.fused_b[blockIdx.y];
@@ -522,6 +526,7 @@ __global__ void k_fuse_s2(FuseS2Args a) {
 // 0.6 * intensity + 0.4 * range of every direction, in double, for both
 // sides; samples [side][c][n] with channels {range, intensity, ...}.
 __global__ void k_mix_signal(const float* __restrict__ samples, size_t side_stride, int n, float* __restrict__ out) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= 2 * n) return;
   const int side = i / n, k = i - side * n;
@@ -530,7 +535,7 @@ __global__ void k_mix_signal(const float* __restrict__ samples, size_t side_stri
 }
 
 cudaError_t launch_mix_signal(const float* samples, size_t side_stride, int n, float* out, cudaStream_t st) {
-  k_mix_signal<<<(2 * n + 255) / 256, 256, 0, st>>>(samples, side_stride, n, out);
+  launch_kernel(k_mix_signal, dim3((2 * n + 255) / 256), dim3(256), 0, st, samples, side_stride, n, out);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -545,7 +550,7 @@ cudaError_t launch_fuse_s2(const FuseS2Args& a0, cudaStream_t st) {
   }
   if (a.count > kMaxWave) return cudaErrorInvalidValue;
   const int tot = a.bw * (2 * a.bw - 1);
-  k_fuse_s2<<<dim3((tot + 255) / 256, a.count), 256, 0, st>>>(a);
+  launch_kernel(k_fuse_s2, dim3((tot + 255) / 256, a.count), dim3(256), 0, st, a);
   count_launches(1);
   return cudaGetLastError();
 }

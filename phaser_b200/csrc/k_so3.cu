@@ -39,6 +39,7 @@ constexpr int kSynthBetas = 4;
 
 __global__ void k_so3_synth(int bw_in, int bw_out, So3Batch bt, const double* __restrict__ btab,
                             const double* __restrict__ wtab) {
+  chain_begin();
   extern __shared__ double sm[];
   double* fa = sm;
   double* fb = fa + bw_in;
@@ -148,6 +149,7 @@ constexpr int kSo3FftAThreads = 320;
 template <int NF, int LOG2W>
 __global__ void __launch_bounds__(kSo3FftAThreads, NF > 0 ? 4 : 2)
     k_so3_fft_a(int bw_in, int bw_out, const __grid_constant__ So3Batch bt, const __grid_constant__ FftPlan plan) {
+  chain_begin();
   extern __shared__ __align__(16) float2 tile[];  // [a][beta tile] | float4 cs[] (runtime plans)
   constexpr int Wt = 1 << LOG2W;
   const int n = NF > 0 ? NF : 2 * bw_out;
@@ -196,6 +198,7 @@ constexpr int kSo3C2rThreads = 320;
 template <int NF>
 __global__ void __launch_bounds__(kSo3C2rThreads, NF > 0 ? 3 : 2)
     k_so3_c2r(int bw_in, int bw_out, const __grid_constant__ So3Batch bt, const __grid_constant__ FftPlan plan) {
+  chain_begin();
   extern __shared__ __align__(16) float2 zrow[];  // [kSo3Pairs][st] | float4 cs[] | int pos[n] (runtime plans)
   const int n = NF > 0 ? NF : 2 * bw_out;
   const int Bo = n / 2, st = n | 1;
@@ -333,7 +336,7 @@ cudaError_t launch_so3_synth(const So3Args& a, cudaStream_t st) {
   int thr = (((n + kSynthBetas - 1) / kSynthBetas + 31) / 32) * 32;
   if (thr > 512) thr = 512;
   const size_t sm1 = (size_t)a.bw_in * 3 * sizeof(double) + 2 * sizeof(double) + (size_t)a.bw_in * 4 * sizeof(float2);
-  k_so3_synth<<<dim3(ncls, a.batch.count), thr, sm1, st>>>(a.bw_in, a.bw_out, a.batch, a.beta_tab, a.wig_tab);
+  launch_kernel(k_so3_synth, dim3(ncls, a.batch.count), dim3(thr), sm1, st, a.bw_in, a.bw_out, a.batch, a.beta_tab, a.wig_tab);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -343,7 +346,7 @@ static void launch_so3_c2r(const So3Args& a, int n, cudaStream_t st) {
   const dim3 g((n + 2 * kSo3Pairs - 1) / (2 * kSo3Pairs), n, a.batch.count);
   size_t sm = (size_t)kSo3Pairs * (n | 1) * sizeof(float2);
   if (NF == 0) sm += so3_prime_scratch(n) + (size_t)n * sizeof(int);
-  k_so3_c2r<NF><<<g, pass_threads(*a.plan, kSo3Pairs, 1, 160, kSo3C2rThreads), sm, st>>>(a.bw_in, a.bw_out, a.batch,
+  launch_kernel(k_so3_c2r<NF>, dim3(g), dim3(pass_threads(*a.plan, kSo3Pairs, 1, 160, kSo3C2rThreads)), sm, st, a.bw_in, a.bw_out, a.batch,
                                                                                         *a.plan);
 }
 
@@ -353,11 +356,11 @@ static void launch_so3_fft_a(const So3Args& a, int n, int wt, cudaStream_t st) {
   const size_t sm = (size_t)n * wt * sizeof(float2) + so3_prime_scratch(n);
   const int thr = pass_threads(*a.plan, wt, 1, 160, kSo3FftAThreads);
   if (wt == 8)
-    k_so3_fft_a<NF, 3><<<g, thr, sm, st>>>(a.bw_in, a.bw_out, a.batch, *a.plan);
+    launch_kernel(k_so3_fft_a<NF, 3>, dim3(g), dim3(thr), sm, st, a.bw_in, a.bw_out, a.batch, *a.plan);
   else if (wt == 32)
-    k_so3_fft_a<NF, 5><<<g, thr, sm, st>>>(a.bw_in, a.bw_out, a.batch, *a.plan);
+    launch_kernel(k_so3_fft_a<NF, 5>, dim3(g), dim3(thr), sm, st, a.bw_in, a.bw_out, a.batch, *a.plan);
   else
-    k_so3_fft_a<NF, 4><<<g, thr, sm, st>>>(a.bw_in, a.bw_out, a.batch, *a.plan);
+    launch_kernel(k_so3_fft_a<NF, 4>, dim3(g), dim3(thr), sm, st, a.bw_in, a.bw_out, a.batch, *a.plan);
 }
 
 bool so3_beta_tile_ok(int bw_out, int wt) {

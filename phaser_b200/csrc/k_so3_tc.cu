@@ -147,6 +147,7 @@ struct WignerGemm {
 
 template <int PREC>
 __global__ void __launch_bounds__(kTcThreads, kTcCtasPerSm) k_so3_synth_tc(TcGemmArgs g, WignerGemm prob) {
+  chain_begin();
   tc_class_gemm<PREC>(g, prob);
 }
 
@@ -178,9 +179,9 @@ cudaError_t launch_so3_synth_tc(const So3Args& a, const So3Table& t, unsigned lo
   const int ncls = a.bw_in * (a.bw_in + 1) / 2;
   const int grid = ncls < sms * g.ctas_per_sm ? ncls : sms * g.ctas_per_sm;
   if (t.precision == kSo3Tf32x3)
-    k_so3_synth_tc<kSo3Tf32x3><<<grid, kTcThreads, g.smem, st>>>(g, prob);
+    launch_kernel(k_so3_synth_tc<kSo3Tf32x3>, dim3(grid), dim3(kTcThreads), g.smem, st, g, prob);
   else
-    k_so3_synth_tc<kSo3Bf16x3><<<grid, kTcThreads, g.smem, st>>>(g, prob);
+    launch_kernel(k_so3_synth_tc<kSo3Bf16x3>, dim3(grid), dim3(kTcThreads), g.smem, st, g, prob);
   count_launches(1);
   return cudaGetLastError();
 }

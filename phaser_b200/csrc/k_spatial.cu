@@ -56,6 +56,7 @@ __device__ __forceinline__ int histc_bin(float x, const float* __restrict__ E, i
 // of a sparse scan's 8 us kernel) -- so a warp sums each run of equal voxels
 // with shuffles and the run's last lane issues the atomics.
 __global__ void k_voxelize(const __grid_constant__ VoxelArgs a) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int np = a.n_dev ? (int)*a.n_dev : a.n_points;
   const int lane = threadIdx.x & 31;
@@ -133,7 +134,7 @@ __global__ void k_voxelize(const __grid_constant__ VoxelArgs a) {
 
 cudaError_t launch_voxelize(const VoxelArgs& a, cudaStream_t st) {
   if (a.n_points > 0) {
-    k_voxelize<<<(a.n_points + 255) / 256, 256, 0, st>>>(a);
+    launch_kernel(k_voxelize, dim3((a.n_points + 255) / 256), dim3(256), 0, st, a);
     count_launches(1);
   }
   return cudaGetLastError();
@@ -142,6 +143,7 @@ cudaError_t launch_voxelize(const VoxelArgs& a, cudaStream_t st) {
 // Zeroes what the voxelisation that left these indices wrote.
 __global__ void k_clear_voxels(const uint32_t* __restrict__ lin, int n_points, float4* __restrict__ sums,
                                float* __restrict__ counts, uint8_t* __restrict__ rowlive, int N) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_points) return;
   const uint32_t l = lin[i];
@@ -154,7 +156,7 @@ __global__ void k_clear_voxels(const uint32_t* __restrict__ lin, int n_points, f
 cudaError_t launch_clear_voxels(const uint32_t* lin, int n_points, float4* sums, float* counts, uint8_t* rowlive, int N,
                                 cudaStream_t st) {
   if (n_points > 0) {
-    k_clear_voxels<<<(n_points + 255) / 256, 256, 0, st>>>(lin, n_points, sums, counts, rowlive, N);
+    launch_kernel(k_clear_voxels, dim3((n_points + 255) / 256), dim3(256), 0, st, lin, n_points, sums, counts, rowlive, N);
     count_launches(1);
   }
   return cudaGetLastError();
@@ -198,6 +200,7 @@ static size_t scan_rows_smem(int N) { return (size_t)N * (8 + kRowsWarps * 18) +
 
 template <int CC>
 __global__ void __launch_bounds__(kRowsWarps * 32) k_scan_rows(const ScanRowArgs a) {
+  chain_begin();
   extern __shared__ __align__(16) float4 s_mem[];
   constexpr int U = 8, Q = 4;
   const int n = a.N, H2 = n / 2 + 1, H2p = spatial_h2p(n);
@@ -296,6 +299,7 @@ __global__ void __launch_bounds__(320, NF > 0 ? 3 : 2) k_r2c_rows(int N, const f
                                                                   size_t grid_stride, float2* __restrict__ specs,
                                                                   size_t spec_stride,
                                                                   const __grid_constant__ FftPlan plan) {
+  chain_begin();
   extern __shared__ __align__(16) float2 rows[];  // [kRowPairs][st] | float4 cs[] (runtime plans)
   __shared__ short s_pos[kMaxVoxels];
   const int n = NF > 0 ? NF : N;
@@ -345,6 +349,7 @@ template <int NF>
 __global__ void __launch_bounds__(320, NF > 0 ? 3 : 2) k_c2r_rows(int N, const float2* __restrict__ cspec, const __grid_constant__ FftPlan plan,
                                                   unsigned long long* __restrict__ argmax, float* __restrict__ volume,
                                                   uint32_t limit) {
+  chain_begin();
   extern __shared__ __align__(16) float2 rows[];  // [kInvPairs][st] | float4 cs[] | int pos[n] (runtime plans)
   const int n = NF > 0 ? NF : N;
   const int H2p = spatial_h2p(n), st = row_stride(n);
@@ -491,6 +496,7 @@ struct ColArgs {
 constexpr int kXThreads = 320;
 template <int NF, bool INV, int CC, int LW>
 __global__ void __launch_bounds__(kXThreads, NF > 0 ? 4 : 2) k_fft_x(const __grid_constant__ ColArgs a) {
+  chain_begin();
   extern __shared__ __align__(16) float2 tile[];  // [CC][n][W] | float4 cs[] (runtime plans) | uint8 live[n]
   __shared__ uint16_t s_mask[(INV || NF == 0) ? 1 : NF / 2];
   constexpr int W = 1 << LW;
@@ -634,6 +640,7 @@ constexpr int fuse_z_blocks() {
 // LW >= 0: the tile is 2^LW columns wide; LW < 0: 2^lw_arg.
 template <int NF, int CC, int LW>
 __global__ void __launch_bounds__(fuse_z_max_threads<NF>(), fuse_z_blocks<NF>()) k_fuse_z(const __grid_constant__ SpatialArgs a, const __grid_constant__ FftPlan plan, int lw_arg) {
+  chain_begin();
   // [CC + 1][z_off(n)][W] | float4 cs[] (runtime plans) | int16 kz[n], uint16 mask[n], uint8 live[2 n], op[n], gop[n]
   extern __shared__ __align__(16) float2 tile[];
   __shared__ FusionBands s_bands;
@@ -967,20 +974,20 @@ cudaError_t launch_spatial_forward(const SpatialArgs& a, int side, cudaStream_t 
     const dim3 gr((N * N + 2 * kRowPairs - 1) / (2 * kRowPairs), nch);
     const size_t smr = (size_t)kRowPairs * row_stride(N) * sizeof(float2) + prime_scratch(N);
     const int tr = pass_threads(*a.plan, kRowPairs, 1, 128, 320);
-    PHGPU_DISPATCH_N(N, k_r2c_rows<NF><<<gr, tr, smr, st>>>(N, grids, nv, spec, plane, *a.plan));
+    PHGPU_DISPATCH_N(N, launch_kernel(k_r2c_rows<NF>, dim3(gr), dim3(tr), smr, st, N, grids, nv, spec, plane, *a.plan));
   } else {
     const ScanRowArgs r{N, reinterpret_cast<float4*>(grids), grids + 4 * nv, a.plan->tw, a.rowlive[side],
                         a.rowmask + (size_t)side * N * N, spec, plane, a.clear};
     const dim3 gr(N, (N + kRowsBlock - 1) / kRowsBlock);
     const size_t smr = scan_rows_smem(N);
     if (nch == 1)
-      k_scan_rows<1><<<gr, kRowsWarps * 32, smr, st>>>(r);
+      launch_kernel(k_scan_rows<1>, dim3(gr), dim3(kRowsWarps * 32), smr, st, r);
     else if (nch == 2)
-      k_scan_rows<2><<<gr, kRowsWarps * 32, smr, st>>>(r);
+      launch_kernel(k_scan_rows<2>, dim3(gr), dim3(kRowsWarps * 32), smr, st, r);
     else if (nch == 3)
-      k_scan_rows<3><<<gr, kRowsWarps * 32, smr, st>>>(r);
+      launch_kernel(k_scan_rows<3>, dim3(gr), dim3(kRowsWarps * 32), smr, st, r);
     else
-      k_scan_rows<4><<<gr, kRowsWarps * 32, smr, st>>>(r);
+      launch_kernel(k_scan_rows<4>, dim3(gr), dim3(kRowsWarps * 32), smr, st, r);
   }
   // channels of one launch: as many as leave two blocks an SM's shared memory
   const size_t per = (size_t)N * (1 << kXFwdLog2) * sizeof(float2), extra = prime_scratch(N) + (size_t)N;
@@ -995,7 +1002,7 @@ cudaError_t launch_spatial_forward(const SpatialArgs& a, int side, cudaStream_t 
     const int tx = pass_threads(*a.plan, (1 << kXFwdLog2) * (fixed ? 1 : k), fixed ? k : 1, 160, kXThreads);
     FftXFn fn = nullptr;
     PHGPU_DISPATCH_N(N, fn = fft_x_forward<NF>(k));
-    fn<<<gx, tx, k * per + extra, st>>>(cx);
+    launch_kernel(fn, dim3(gx), dim3(tx), k * per + extra, st, cx);
     count_launches(1);
   }
   count_launches(1);
@@ -1013,7 +1020,7 @@ cudaError_t launch_spatial_fuse_z(const SpatialArgs& a, cudaStream_t st) {
   const int lw = wt == 16 ? 4 : (wt == 8 ? 3 : (wt == 4 ? 2 : 1));
   FuseZFn fn = nullptr;
   PHGPU_DISPATCH_N(N, fn = fuse_z_kernel<NF>(C, wt));
-  fn<<<g, fuse_z_threads(*a.plan, C, wt), sm, st>>>(a, *a.plan, lw);
+  launch_kernel(fn, dim3(g), dim3(fuse_z_threads(*a.plan, C, wt)), sm, st, a, *a.plan, lw);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -1028,8 +1035,8 @@ cudaError_t launch_spatial_inverse(const SpatialArgs& a, cudaStream_t st) {
   const size_t smr = (size_t)kInvPairs * row_stride(N) * sizeof(float2) +
                      (fixed_length(N) ? 0 : prime_scratch(N) + (size_t)N * sizeof(int) + 16);
   const int tr = pass_threads(*a.plan, kInvPairs, 1, 128, 320), tx = pass_threads(*a.plan, 1 << kXInvLog2, 1, 160, kXThreads);
-  PHGPU_DISPATCH_N(N, k_fft_x<NF, true, 1, kXInvLog2><<<gx, tx, smx, st>>>(c);
-                   k_c2r_rows<NF><<<nblk, tr, smr, st>>>(N, a.cspec, *a.plan, a.argmax, a.volume, limit));
+  PHGPU_DISPATCH_N(N, launch_kernel(k_fft_x<NF, true, 1, kXInvLog2>, dim3(gx), dim3(tx), smx, st, c);
+                   launch_kernel(k_c2r_rows<NF>, dim3(nblk), dim3(tr), smr, st, N, a.cspec, *a.plan, a.argmax, a.volume, limit));
   count_launches(2);
   return cudaGetLastError();
 }

@@ -22,6 +22,34 @@ inline void count_launches(int n) {
   if (!g_capture_depth) g_launch_count.fetch_add((unsigned long long)n, std::memory_order_relaxed);
 }
 
+// Kernel launches of the registration chain.  On one pair's own stream each
+// kernel waits for the one before it, so the gaps between dependent launches
+// (1-2 us each, twenty of them) are a third of a small registration.  With
+// programmatic launch the next kernel's blocks are set up while the last ones
+// of this kernel run, and wait inside chain_begin().  Off by default: captured
+// waves and other concurrent streams would only lose the slots that waiting
+// blocks hold.
+extern thread_local bool g_chain_launch;
+struct ChainScope {
+  bool before;
+  explicit ChainScope(bool on) : before(g_chain_launch) { g_chain_launch = on; }
+  ~ChainScope() { g_chain_launch = before; }
+};
+template <class... P, class... A>
+inline cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = g_chain_launch ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // ------------------------------------------------------------ S^2 sampling
 struct SampleArgs {
   const float4* xyzi;   // [n_points] x, y, z, intensity

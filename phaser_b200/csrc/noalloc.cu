@@ -105,6 +105,9 @@ int phgpu_sample_s2_noalloc(const phgpu_params* params, const phgpu_cloud* cloud
     }
     scratch = slot.scratch;
   }
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) return PHGPU_ERR_CUDA;
+  ChainScope chain(capturing == cudaStreamCaptureStatusNone);
   SampleArgs a;
   a.xyzi = reinterpret_cast<const float4*>(cloud->xyzi);
   a.refl = cloud->reflectivity;
