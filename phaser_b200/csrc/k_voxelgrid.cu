@@ -59,6 +59,7 @@ struct VgState {
   int32_t status;
   int32_t min_b[3];
   uint32_t mul[3];
+  uint32_t short_keys;  // every leaf index below 2^16: the last two radix passes have nothing to do
   uint32_t n_valid;   // finite points
   uint32_t n_leaves;  // occupied leaves
   uint32_t n_out;     // leaves kept (>= min points)
@@ -76,6 +77,7 @@ constexpr int kBoundsBlocks = 148 * 4;
 
 __global__ void __launch_bounds__(kVgThreads) k_vg_bounds(const float4* __restrict__ pts, uint32_t n,
                                                           uint32_t* __restrict__ part) {
+  chain_begin();
   uint32_t m[6] = {0, 0, 0, 0, 0, 0};
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float4 p = pts[i];
@@ -106,6 +108,7 @@ __global__ void __launch_bounds__(kVgThreads) k_vg_bounds(const float4* __restri
 // Reduces the bounds partials (one warp), then lane 0 plans the grid.
 __global__ void k_vg_plan(const uint32_t* __restrict__ part, int n_part, VgState* st, float inv_x, float inv_y,
                           float inv_z) {
+  chain_begin();
   const int lane = threadIdx.x & 31;
   uint32_t m[6] = {0, 0, 0, 0, 0, 0};
   for (int b = lane; b < n_part; b += 32)
@@ -159,6 +162,7 @@ __global__ void k_vg_plan(const uint32_t* __restrict__ part, int n_part, VgState
     st->status = kVgRange;
     return;
   }
+  st->short_keys = cells <= 0x10000ull ? 1u : 0u;
   st->mul[0] = 1u;
   st->mul[1] = (uint32_t)div[0];
   st->mul[2] = (uint32_t)div[0] * (uint32_t)div[1];
@@ -169,6 +173,7 @@ __global__ void k_vg_plan(const uint32_t* __restrict__ part, int n_part, VgState
 // Exclusive scan of `len` words by one block; *total gets the sum.
 __global__ void __launch_bounds__(kScanThreads) k_scan_words(const uint32_t* __restrict__ in, uint32_t len,
                                                              uint32_t* __restrict__ out, uint32_t* total) {
+  chain_begin();
   __shared__ uint32_t s_warp[kScanThreads / 32];
   const uint32_t chunk = (len + kScanThreads - 1) / kScanThreads;
   const uint32_t b = threadIdx.x * chunk;
@@ -207,6 +212,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_words(const uint32_t* __r
 //     is (round, thread), i.e. ascending index, so ranks are stable.
 template <class Op>
 __global__ void __launch_bounds__(kVgThreads) k_flag_count(Op op, uint32_t* __restrict__ counts) {
+  chain_begin();
   const uint32_t n = op.n();
   const uint32_t base = blockIdx.x * kVgTile;
   bool f[kVgRounds];  // all of the tile's flags first: one load latency, not one per round
@@ -230,6 +236,7 @@ __global__ void __launch_bounds__(kVgThreads) k_flag_count(Op op, uint32_t* __re
 
 template <class Op>
 __global__ void __launch_bounds__(kVgThreads) k_flag_scatter(Op op, const uint32_t* __restrict__ offsets) {
+  chain_begin();
   const uint32_t n = op.n();
   const uint32_t base = blockIdx.x * kVgTile;
   if (base >= n) return;
@@ -320,10 +327,15 @@ struct KeepOp {
 };
 
 // ---------------------------------------------------------------- radix passes
+// Passes over bits 16.. return at once when every leaf index is below 2^16 (a
+// 20 x 12 x 4 m room at 0.25 m has 61 k cells); an even number of passes is
+// skipped, so the sorted pairs end in the same buffers.
 __global__ void __launch_bounds__(kVgThreads) k_radix_count(const uint32_t* __restrict__ keys, const VgState* st,
                                                             int shift, uint32_t n_tiles,
                                                             uint32_t* __restrict__ counts) {
+  chain_begin();
   __shared__ uint32_t s_hist[kBins];
+  if (shift >= 16 && st->short_keys) return;
   const uint32_t n = st->n_valid;
   s_hist[threadIdx.x] = 0;
   __syncthreads();
@@ -349,8 +361,10 @@ __global__ void __launch_bounds__(kVgThreads) k_radix_count(const uint32_t* __re
 // coalesced 128-byte row, and a warp scan per row carries the running sum).
 constexpr int kScanRows = 16;
 
-__global__ void __launch_bounds__(kVgThreads) k_radix_scan(uint32_t* __restrict__ counts, uint32_t n_tiles,
-                                                           uint32_t* __restrict__ digit_total) {
+__global__ void __launch_bounds__(kVgThreads) k_radix_scan(const VgState* st, int shift, uint32_t* __restrict__ counts,
+                                                           uint32_t n_tiles, uint32_t* __restrict__ digit_total) {
+  chain_begin();
+  if (shift >= 16 && st->short_keys) return;
   const int lane = threadIdx.x & 31;
   const uint32_t d = blockIdx.x * kVgWarps + (threadIdx.x >> 5);
   uint32_t* row = counts + (size_t)d * n_tiles;
@@ -387,6 +401,7 @@ __global__ void __launch_bounds__(kVgThreads) k_radix_scatter(const uint32_t* __
                                                               int shift, uint32_t n_tiles,
                                                               const uint32_t* __restrict__ offsets,
                                                               const uint32_t* __restrict__ digit_total) {
+  chain_begin();
   __shared__ uint32_t s_key[kVgTile];
   __shared__ uint32_t s_val[kVgTile];
   __shared__ uint32_t s_local[kBins];  // start of each digit in the sorted tile
@@ -395,7 +410,7 @@ __global__ void __launch_bounds__(kVgThreads) k_radix_scatter(const uint32_t* __
   __shared__ uint32_t s_wc[kVgWarps][kBins];
   const uint32_t n = st->n_valid;
   const uint32_t base = blockIdx.x * kVgTile;
-  if (base >= n) return;
+  if (base >= n || (shift >= 16 && st->short_keys)) return;
   const uint32_t tile_n = min((uint32_t)kVgTile, n - base);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint32_t k[kVgRounds], v[kVgRounds], dg[kVgRounds];
@@ -494,6 +509,7 @@ __global__ void __launch_bounds__(kVgThreads) k_vg_centroid(const float4* __rest
                                                             const uint32_t* __restrict__ leaf_start,
                                                             VgState* st, float4* out, float* out_refl,
                                                             float* out_amb, int direct) {
+  chain_begin();
   __shared__ float4 s_p[kVgWarps][kBatch];
   __shared__ float2 s_ra[kVgWarps][kBatch];
   const uint32_t n_leaves = st->n_leaves;
@@ -719,6 +735,7 @@ int phgpu_voxel_grid_filter(phgpu_voxel_grid* vg, const phgpu_cloud* in, const f
     return PHGPU_ERR_INVALID;
   }
   DeviceGuard g(vg->device);
+  ChainScope chain(true);
   cudaStream_t st = vg->st;
   const uint32_t n = in->n_points;
   *n_out = 0;
@@ -750,22 +767,22 @@ int phgpu_voxel_grid_filter(phgpu_voxel_grid* vg, const phgpu_cloud* in, const f
   int launches = 0;
   VG_CK(cudaMemsetAsync(s, 0, sizeof(VgState), st));
   const int bounds_blocks = (int)std::min<uint32_t>((n + kVgThreads - 1) / kVgThreads, (uint32_t)kBoundsBlocks);
-  k_vg_bounds<<<bounds_blocks, kVgThreads, 0, st>>>(pts, n, vg->offsets);
-  k_vg_plan<<<1, 32, 0, st>>>(vg->offsets, bounds_blocks, s, inv[0], inv[1], inv[2]);
+  launch_kernel(k_vg_bounds, dim3(bounds_blocks), dim3(kVgThreads), 0, st, pts, n, vg->offsets);
+  launch_kernel(k_vg_plan, dim3(1), dim3(32), 0, st, vg->offsets, bounds_blocks, s, inv[0], inv[1], inv[2]);
   launches += 2;
 
   ValidOp vop{pts, n, {inv[0], inv[1], inv[2]}, s, vg->keys[0], vg->vals[0]};
-  k_flag_count<ValidOp><<<tiles, kVgThreads, 0, st>>>(vop, vg->counts);
-  k_scan_words<<<1, kScanThreads, 0, st>>>(vg->counts, tiles, vg->offsets, &s->n_valid);
-  k_flag_scatter<ValidOp><<<tiles, kVgThreads, 0, st>>>(vop, vg->offsets);
+  launch_kernel(k_flag_count<ValidOp>, dim3(tiles), dim3(kVgThreads), 0, st, vop, vg->counts);
+  launch_kernel(k_scan_words, dim3(1), dim3(kScanThreads), 0, st, vg->counts, tiles, vg->offsets, &s->n_valid);
+  launch_kernel(k_flag_scatter<ValidOp>, dim3(tiles), dim3(kVgThreads), 0, st, vop, vg->offsets);
   launches += 3;
 
   int cur = 0;
   for (int pass = 0; pass < 4; ++pass) {
     const int shift = 8 * pass;
-    k_radix_count<<<tiles, kVgThreads, 0, st>>>(vg->keys[cur], s, shift, tiles, vg->counts);
-    k_radix_scan<<<kBins / kVgWarps, kVgThreads, 0, st>>>(vg->counts, tiles, vg->digit_total);
-    k_radix_scatter<<<tiles, kVgThreads, 0, st>>>(vg->keys[cur], vg->vals[cur], vg->keys[cur ^ 1],
+    launch_kernel(k_radix_count, dim3(tiles), dim3(kVgThreads), 0, st, vg->keys[cur], s, shift, tiles, vg->counts);
+    launch_kernel(k_radix_scan, dim3(kBins / kVgWarps), dim3(kVgThreads), 0, st, s, shift, vg->counts, tiles, vg->digit_total);
+    launch_kernel(k_radix_scatter, dim3(tiles), dim3(kVgThreads), 0, st, vg->keys[cur], vg->vals[cur], vg->keys[cur ^ 1],
                                                   vg->vals[cur ^ 1], s, shift, tiles, vg->counts,
                                                   vg->digit_total);
     cur ^= 1;
@@ -773,23 +790,23 @@ int phgpu_voxel_grid_filter(phgpu_voxel_grid* vg, const phgpu_cloud* in, const f
   }
 
   HeadOp hop{vg->keys[cur], s, vg->leaf_start};
-  k_flag_count<HeadOp><<<tiles, kVgThreads, 0, st>>>(hop, vg->counts);
-  k_scan_words<<<1, kScanThreads, 0, st>>>(vg->counts, tiles, vg->offsets, &s->n_leaves);
-  k_flag_scatter<HeadOp><<<tiles, kVgThreads, 0, st>>>(hop, vg->offsets);
+  launch_kernel(k_flag_count<HeadOp>, dim3(tiles), dim3(kVgThreads), 0, st, hop, vg->counts);
+  launch_kernel(k_scan_words, dim3(1), dim3(kScanThreads), 0, st, vg->counts, tiles, vg->offsets, &s->n_leaves);
+  launch_kernel(k_flag_scatter<HeadOp>, dim3(tiles), dim3(kVgThreads), 0, st, hop, vg->offsets);
   launches += 3;
 
   const bool direct = min_points_per_voxel <= 1;
   const uint32_t leaf_blocks = std::min<uint32_t>((n + kVgWarps - 1) / kVgWarps, 148u * 16u);
-  k_vg_centroid<<<leaf_blocks, kVgThreads, 0, st>>>(pts, o_refl ? refl : nullptr, o_amb ? amb : nullptr,
+  launch_kernel(k_vg_centroid, dim3(leaf_blocks), dim3(kVgThreads), 0, st, pts, o_refl ? refl : nullptr, o_amb ? amb : nullptr,
                                                     vg->vals[cur], vg->leaf_start, s, direct ? out : vg->d_tmp,
                                                     direct ? o_refl : (o_refl ? vg->d_tmp_refl : nullptr),
                                                     direct ? o_amb : (o_amb ? vg->d_tmp_amb : nullptr), direct ? 1 : 0);
   launches += 1;
   if (!direct) {
     KeepOp kop{vg->leaf_start, s, min_points_per_voxel, vg->d_tmp, vg->d_tmp_refl, vg->d_tmp_amb, out, o_refl, o_amb};
-    k_flag_count<KeepOp><<<tiles, kVgThreads, 0, st>>>(kop, vg->counts);
-    k_scan_words<<<1, kScanThreads, 0, st>>>(vg->counts, tiles, vg->offsets, &s->n_out);
-    k_flag_scatter<KeepOp><<<tiles, kVgThreads, 0, st>>>(kop, vg->offsets);
+    launch_kernel(k_flag_count<KeepOp>, dim3(tiles), dim3(kVgThreads), 0, st, kop, vg->counts);
+    launch_kernel(k_scan_words, dim3(1), dim3(kScanThreads), 0, st, vg->counts, tiles, vg->offsets, &s->n_out);
+    launch_kernel(k_flag_scatter<KeepOp>, dim3(tiles), dim3(kVgThreads), 0, st, kop, vg->offsets);
     launches += 3;
   }
   count_launches(launches);
