@@ -33,19 +33,45 @@
 
 namespace phgpu {
 
-// KB betas per thread (k = t, t + ceil(n / KB), ...): the coefficient loads
-// from shared memory serve KB recurrences.
-constexpr int kSynthBetas = 4;
+// KB betas per thread (k = t, t + ceil(n / KB), ...): KB recurrences in flight
+// per thread cover the double-precision latency, and the coefficients loaded
+// from shared memory serve KB of them.  The host picks the KB that leaves the
+// fewest lanes idle (n = 200: 7 betas in 29 of a warp's 32 lanes, where 4 betas
+// fill 50 of 64).  A step is three double-precision operations, one conversion
+// and four packed multiply-adds, and the issue of these 64-bit operations
+// bounds the kernel; two steps are written out, the second in the registers of
+// the value it replaces, which takes the moves between them out (16 -> 11.5
+// instructions a step).  Four separate FMA pairs, one step and 4 betas for every
+// length: B = 150 with padding 10 185 us, now 124; B = 256 1077 -> 860; B = 100
+// 46 -> 41.  Packing two betas of a component (no duplicated operand, doubled
+// coefficients) takes more registers: 160, 958 and 50 us.
+template <int KB>
+__device__ __forceinline__ void so3_step(const float4* __restrict__ c, double a, double b, double g, const double (&cb)[KB],
+                                         double (&dprev)[KB], const double (&dcur)[KB], float2 (&acc)[KB][4]) {
+  const float4 c01 = c[0], c23 = c[1];
+#pragma unroll
+  for (int u = 0; u < KB; ++u) {
+    const float d = (float)dcur[u];
+    const float2 dd = make_float2(d, d);
+    acc[u][0] = __ffma2_rn(make_float2(c01.x, c01.y), dd, acc[u][0]);
+    acc[u][1] = __ffma2_rn(make_float2(c01.z, c01.w), dd, acc[u][1]);
+    acc[u][2] = __ffma2_rn(make_float2(c23.x, c23.y), dd, acc[u][2]);
+    acc[u][3] = __ffma2_rn(make_float2(c23.z, c23.w), dd, acc[u][3]);
+    dprev[u] = wig_step(a, b, g, cb[u], dprev[u], dcur[u]);
+  }
+}
 
-__global__ void k_so3_synth(int bw_in, int bw_out, So3Batch bt, const double* __restrict__ btab,
-                            const double* __restrict__ wtab) {
+constexpr int kSynthThreads = 128;
+
+template <int KB>
+__global__ void __launch_bounds__(kSynthThreads, KB > 5 ? 4 : 5)
+    k_so3_synth(int bw_in, int bw_out, const __grid_constant__ So3Batch bt, const double* __restrict__ btab,
+                const double* __restrict__ wtab) {
   chain_begin();
-  extern __shared__ double sm[];
-  double* fa = sm;
-  double* fb = fa + bw_in;
-  double* gs = fb + bw_in;            // fb * shift
-  double* s_lnorm = gs + bw_in;       // one value (slot padded to 16 bytes)
-  float2* cv = (float2*)(s_lnorm + 2);  // [4][bw_in]
+  extern __shared__ __align__(16) double sm[];
+  double* fa = sm;                      // [bw_in] pairs {a, b}, then shifts
+  double* gs = fa + 2 * bw_in;          // fb * shift
+  float2* cv = (float2*)(gs + bw_in + (bw_in & 1));  // [bw_in][4]
   const float2* __restrict__ fz = bt.fused[blockIdx.y];
   float2* __restrict__ S = bt.out[blockIdx.y].S;
   int p, q;
@@ -53,52 +79,41 @@ __global__ void k_so3_synth(int bw_in, int bw_out, So3Batch bt, const double* __
   const int nl = bw_in - q;
   const WigTab W = wig_tab(wtab, bw_in);
   const int b1 = bw_in + 1;
+  const int n = 2 * bw_out;
+  const int stride = (n + KB - 1) / KB;
   for (int i = threadIdx.x; i < nl; i += blockDim.x) {
     const int l = q + i;
-    wig_factors(W, b1, p, q, l, &fa[i], &fb[i], &gs[i]);
+    wig_factors(W, b1, p, q, l, &fa[2 * i], &fa[2 * i + 1], &gs[i]);
     float2 v[4];
     so3_coefs(fz, bw_in, p, q, l, (float)__ldg(&W.wl[l]), v);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) cv[u * bw_in + i] = v[u];
+    for (int u = 0; u < 4; ++u) cv[4 * i + u] = v[u];
   }
-  if (threadIdx.x == 0) *s_lnorm = wig_lnorm(W, p, q);
+  const double lnorm = wig_lnorm(W, p, q);
   __syncthreads();
-  const int n = 2 * bw_out;
-  const int stride = (n + kSynthBetas - 1) / kSynthBetas;
-  const double lnorm = *s_lnorm;
   for (int k0 = threadIdx.x; k0 < stride; k0 += blockDim.x) {
-    double cb[kSynthBetas], dcur[kSynthBetas], dprev[kSynthBetas];
-    float2 acc[kSynthBetas][4];
+    double cb[KB], d0[KB], d1[KB];
+    float2 acc[KB][4];
 #pragma unroll
-    for (int u = 0; u < kSynthBetas; ++u) {
+    for (int u = 0; u < KB; ++u) {
       const int k = min(k0 + u * stride, n - 1);
       cb[u] = __ldg(&btab[k]);
-      dcur[u] = wig_seed(btab, n, k, lnorm, p, q);
-      dprev[u] = 0.0;
+      d0[u] = wig_seed(btab, n, k, lnorm, p, q);
+      d1[u] = 0.0;
 #pragma unroll
       for (int v = 0; v < 4; ++v) acc[u][v] = make_float2(0.f, 0.f);
     }
-    for (int i = 0; i < nl; ++i) {
-      const float2 c0 = cv[i], c1 = cv[bw_in + i], c2 = cv[2 * bw_in + i], c3 = cv[3 * bw_in + i];
-      const double a = fa[i], b = fb[i], g = gs[i];
-#pragma unroll
-      for (int u = 0; u < kSynthBetas; ++u) {
-        const float d = (float)dcur[u];
-        acc[u][0].x = fmaf(c0.x, d, acc[u][0].x);
-        acc[u][0].y = fmaf(c0.y, d, acc[u][0].y);
-        acc[u][1].x = fmaf(c1.x, d, acc[u][1].x);
-        acc[u][1].y = fmaf(c1.y, d, acc[u][1].y);
-        acc[u][2].x = fmaf(c2.x, d, acc[u][2].x);
-        acc[u][2].y = fmaf(c2.y, d, acc[u][2].y);
-        acc[u][3].x = fmaf(c3.x, d, acc[u][3].x);
-        acc[u][3].y = fmaf(c3.y, d, acc[u][3].y);
-        const double dn = wig_step(a, b, g, cb[u], dprev[u], dcur[u]);
-        dprev[u] = dcur[u];
-        dcur[u] = dn;
-      }
+    int i = 0;
+#pragma unroll 1
+    for (; i + 1 < nl; i += 2) {
+      const double2 ab0 = *reinterpret_cast<const double2*>(&fa[2 * i]);
+      so3_step<KB>((const float4*)&cv[4 * i], ab0.x, ab0.y, gs[i], cb, d1, d0, acc);
+      const double2 ab1 = *reinterpret_cast<const double2*>(&fa[2 * i + 2]);
+      so3_step<KB>((const float4*)&cv[4 * i + 4], ab1.x, ab1.y, gs[i + 1], cb, d0, d1, acc);
     }
+    if (i < nl) so3_step<KB>((const float4*)&cv[4 * i], 0.0, 0.0, 0.0, cb, d1, d0, acc);
 #pragma unroll
-    for (int u = 0; u < kSynthBetas; ++u) {
+    for (int u = 0; u < KB; ++u) {
       const int k = k0 + u * stride;
       if (k < n) so3_store(S, n, p, q, k, acc[u]);
     }
@@ -333,10 +348,23 @@ cudaError_t launch_so3_synth(const So3Args& a, cudaStream_t st) {
   if (a.batch.count < 1 || a.batch.count > kMaxWave) return cudaErrorInvalidValue;
   const int ncls = a.bw_in * (a.bw_in + 1) / 2;
   const int n = 2 * a.bw_out;
-  int thr = (((n + kSynthBetas - 1) / kSynthBetas + 31) / 32) * 32;
-  if (thr > 512) thr = 512;
-  const size_t sm1 = (size_t)a.bw_in * 3 * sizeof(double) + 2 * sizeof(double) + (size_t)a.bw_in * 4 * sizeof(float2);
-  launch_kernel(k_so3_synth, dim3(ncls, a.batch.count), dim3(thr), sm1, st, a.bw_in, a.bw_out, a.batch, a.beta_tab, a.wig_tab);
+  // betas per thread: the largest share of busy lanes, the smaller count where it is as good (fewer registers)
+  int kb = 0, thr = 0;
+  double best = 0.0;
+  for (int c : {2, 4, 5, 7}) {
+    const int stride = (n + c - 1) / c;
+    const int rounds = (stride + kSynthThreads - 1) / kSynthThreads;
+    const int t = ((stride + rounds - 1) / rounds + 31) / 32 * 32;
+    const double busy = (double)n / ((double)t * rounds * c);
+    if (busy > best + 0.02 && (c > 2 || n <= 64)) {
+      best = busy;
+      kb = c;
+      thr = t;
+    }
+  }
+  const size_t sm = (size_t)(a.bw_in * 3 + 1) * sizeof(double) + (size_t)a.bw_in * 4 * sizeof(float2);
+  auto fn = kb == 2 ? k_so3_synth<2> : (kb == 4 ? k_so3_synth<4> : (kb == 5 ? k_so3_synth<5> : k_so3_synth<7>));
+  launch_kernel(fn, dim3(ncls, a.batch.count), dim3(thr), sm, st, a.bw_in, a.bw_out, a.batch, a.beta_tab, a.wig_tab);
   count_launches(1);
   return cudaGetLastError();
 }

@@ -91,10 +91,10 @@ __device__ __forceinline__ double wig_seed(const double* __restrict__ btab, int 
   return exp(lg);
 }
 
-// d^{l+1} = a d^{l-1} + (b cos beta + g) d^l, evaluated without contraction so
-// every kernel that runs it produces the same values.
+// d^{l+1} = a d^{l-1} + (b cos beta + g) d^l: two fused multiply-adds and a
+// product, written out so that every kernel that runs it produces the same values.
 __device__ __forceinline__ double wig_step(double a, double b, double g, double cb, double dprev, double dcur) {
-  return __dadd_rn(__dmul_rn(a, dprev), __dmul_rn(__dadd_rn(__dmul_rn(b, cb), g), dcur));
+  return __fma_rn(__fma_rn(b, cb, g), dcur, __dmul_rn(a, dprev));
 }
 
 __device__ __forceinline__ float2 so3_fused_at(const float2* __restrict__ fz, int bw, int side, int l, int m) {
