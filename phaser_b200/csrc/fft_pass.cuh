@@ -334,10 +334,16 @@ __device__ __forceinline__ void pass_rt(const FftPlan& p, PassMap first, PassMap
   }
 }
 
-// Threads per block (a multiple of 32 in [lo, hi]) that leave the fewest idle
-// in the plan's stages over `cols` items per butterfly, each of ng transforms
-// (host).
-inline int pass_threads(const FftPlan& p, int cols, int ng_item, int lo, int hi) {
+// Threads per block (a multiple of 32 in [lo, hi]) of a pass over `cols` items
+// per butterfly, each of ng transforms (host).  With regs == 0 (compile-time
+// plans) the ones that leave the fewest threads idle in the plan's stages.
+// Runtime plans hold 80 to 96 registers a thread and wait for most of their
+// time, so theirs is that time over the threads resident on an SM (`regs` a
+// thread, `smem` bytes a block): blocks of 5 or 7 warps leave one of the four
+// register files short.  The z pass of n = 100 takes 33 us with 128 threads, 46
+// with 160, 41 with 256; the fewest idle threads alone took 84 us at n = 110
+// and 214 at n = 180, now 58 and 162.
+inline int pass_threads(const FftPlan& p, int cols, int ng_item, int lo, int hi, int regs = 0, size_t smem = 0) {
   int best = lo;
   double best_cost = 1e300;
   for (int t = lo; t <= hi; t += 32) {
@@ -354,8 +360,13 @@ inline int pass_threads(const FftPlan& p, int cols, int ng_item, int lo, int hi)
         cost += (double)((items + t - 1) / t) * t * R;
       }
     }
-    // ties and near-ties: the larger block (fewer rounds between barriers)
-    if (cost <= best_cost * 1.0001) {
+    if (regs > 0) {
+      const int by_regs = 4 * (65536 / 4 / (regs * 32)) / (t / 32), by_smem = (int)((size_t)(228 * 1024) / (smem + 1024));
+      const int blocks = by_regs < by_smem ? by_regs : by_smem;
+      cost /= (blocks > 0 ? blocks : 1) * t;
+    }
+    // ties and near-ties of the idle threads: the larger block (fewer rounds between barriers)
+    if (cost <= best_cost * (regs > 0 ? 0.9999 : 1.0001)) {
       best_cost = cost;
       best = t;
     }

@@ -374,15 +374,17 @@ static void launch_so3_c2r(const So3Args& a, int n, cudaStream_t st) {
   const dim3 g((n + 2 * kSo3Pairs - 1) / (2 * kSo3Pairs), n, a.batch.count);
   size_t sm = (size_t)kSo3Pairs * (n | 1) * sizeof(float2);
   if (NF == 0) sm += so3_prime_scratch(n) + (size_t)n * sizeof(int);
-  launch_kernel(k_so3_c2r<NF>, dim3(g), dim3(pass_threads(*a.plan, kSo3Pairs, 1, 160, kSo3C2rThreads)), sm, st, a.bw_in, a.bw_out, a.batch,
-                                                                                        *a.plan);
+  const int thr = NF > 0 ? pass_threads(*a.plan, kSo3Pairs, 1, 160, kSo3C2rThreads)
+                         : pass_threads(*a.plan, kSo3Pairs, 1, 128, kSo3C2rThreads, 96, sm);
+  launch_kernel(k_so3_c2r<NF>, dim3(g), dim3(thr), sm, st, a.bw_in, a.bw_out, a.batch, *a.plan);
 }
 
 template <int NF>
 static void launch_so3_fft_a(const So3Args& a, int n, int wt, cudaStream_t st) {
   const dim3 g((n + wt - 1) / wt, a.bw_in, a.batch.count);
   const size_t sm = (size_t)n * wt * sizeof(float2) + so3_prime_scratch(n);
-  const int thr = pass_threads(*a.plan, wt, 1, 160, kSo3FftAThreads);
+  const int thr = NF > 0 ? pass_threads(*a.plan, wt, 1, 160, kSo3FftAThreads)
+                         : pass_threads(*a.plan, wt, 1, 128, kSo3FftAThreads, 96, sm);
   if (wt == 8)
     launch_kernel(k_so3_fft_a<NF, 3>, dim3(g), dim3(thr), sm, st, a.bw_in, a.bw_out, a.batch, *a.plan);
   else if (wt == 32)

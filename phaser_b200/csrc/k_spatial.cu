@@ -916,6 +916,11 @@ static bool fixed_length(int N) {
   return fixed;
 }
 
+static bool prime_stage(const FftPlan& p) { return p.radix[p.nstage - 1] > 13; }
+
+// Registers a thread of the passes with runtime plans (their launch bounds' share); 0 for compile-time ones.
+static int pass_regs(int N) { return fixed_length(N) ? 0 : 96; }
+
 // Shared memory of the prime-radix scratch of runtime plans.
 static size_t prime_scratch(int N) { return fixed_length(N) ? 0 : kMaxGenericRadix * sizeof(float4); }
 
@@ -943,7 +948,12 @@ static int fuse_z_tile(int N, int C) {
 // compile-time plan an item carries the C channels of a side; runtime plans
 // take the channels as transforms of their own.
 static int fuse_z_threads(const FftPlan& p, int C, int wt) {
-  if (!fixed_length(p.n)) return pass_threads(p, C * wt, 1, 192, fuse_z_max_threads<0>());
+  if (!fixed_length(p.n))
+    return pass_threads(p, C * wt, 1, 128, fuse_z_max_threads<0>(), 80, fuse_z_smem(p.n, C, wt));
+  // a grid of at most three blocks an SM (N = 64): one thread per item of the first stage, whose items are one
+  // channel's (15 -> 13 us)
+  if ((p.n / 2 + wt) / wt * p.n <= 3 * 148)
+    return std::max(64, std::min((C * wt * p.n / p.radix[0] + 31) / 32 * 32, fuse_z_max_threads<64>()));
   int best = 256;
   double best_cost = 1e300;
   const int lo = std::min(192, (wt * p.n / p.radix[0] + 31) / 32 * 32);
@@ -973,7 +983,7 @@ cudaError_t launch_spatial_forward(const SpatialArgs& a, int side, cudaStream_t 
   if (a.grids_are_means) {
     const dim3 gr((N * N + 2 * kRowPairs - 1) / (2 * kRowPairs), nch);
     const size_t smr = (size_t)kRowPairs * row_stride(N) * sizeof(float2) + prime_scratch(N);
-    const int tr = pass_threads(*a.plan, kRowPairs, 1, 128, 320);
+    const int tr = pass_threads(*a.plan, kRowPairs, 1, 128, 320, pass_regs(N), smr);
     PHGPU_DISPATCH_N(N, launch_kernel(k_r2c_rows<NF>, dim3(gr), dim3(tr), smr, st, N, grids, nv, spec, plane, *a.plan));
   } else {
     const ScanRowArgs r{N, reinterpret_cast<float4*>(grids), grids + 4 * nv, a.plan->tw, a.rowlive[side],
@@ -999,7 +1009,8 @@ cudaError_t launch_spatial_forward(const SpatialArgs& a, int side, cudaStream_t 
     cx.spec += (size_t)ch * plane;
     const int k = std::min(cc, nch - ch);
     const bool fixed = fixed_length(N);  // an item carries all channels, or one of them
-    const int tx = pass_threads(*a.plan, (1 << kXFwdLog2) * (fixed ? 1 : k), fixed ? k : 1, 160, kXThreads);
+    const int tx = pass_threads(*a.plan, (1 << kXFwdLog2) * (fixed ? 1 : k), fixed ? k : 1, fixed || prime_stage(*a.plan) ? 160 : 128, kXThreads,
+                                pass_regs(N), k * per + extra);
     FftXFn fn = nullptr;
     PHGPU_DISPATCH_N(N, fn = fft_x_forward<NF>(k));
     launch_kernel(fn, dim3(gx), dim3(tx), k * per + extra, st, cx);
@@ -1034,7 +1045,8 @@ cudaError_t launch_spatial_inverse(const SpatialArgs& a, cudaStream_t st) {
   const int nblk = (N * N + 2 * kInvPairs - 1) / (2 * kInvPairs);
   const size_t smr = (size_t)kInvPairs * row_stride(N) * sizeof(float2) +
                      (fixed_length(N) ? 0 : prime_scratch(N) + (size_t)N * sizeof(int) + 16);
-  const int tr = pass_threads(*a.plan, kInvPairs, 1, 128, 320), tx = pass_threads(*a.plan, 1 << kXInvLog2, 1, 160, kXThreads);
+  const int tr = pass_threads(*a.plan, kInvPairs, 1, 128, 320, pass_regs(N), smr);
+  const int tx = pass_threads(*a.plan, 1 << kXInvLog2, 1, fixed_length(N) ? 160 : 128, kXThreads, pass_regs(N), smx);
   PHGPU_DISPATCH_N(N, launch_kernel(k_fft_x<NF, true, 1, kXInvLog2>, dim3(gx), dim3(tx), smx, st, c);
                    launch_kernel(k_c2r_rows<NF>, dim3(nblk), dim3(tr), smr, st, N, a.cspec, *a.plan, a.argmax, a.volume, limit));
   count_launches(2);
