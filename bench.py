@@ -205,17 +205,18 @@ def pair_bytes(bw, N, C, P):
     return rot + trans
 
 
-# Kernels of each profiled stage (one launch of each per stage call).
+# Kernels of each profiled stage (one launch of each per stage call; the x
+# transform's two directions have a row each in the table).
 STAGE_KERNELS = {
     "s2_sample": ("k_project", "k_bin_scan", "k_bin_scatter", "k_nn_rows"),
     "sht": ("k_sht_phi", "k_sht_leg", "k_sht_leg_tc"),
     "fuse_s2": ("k_fuse_s2",),
     "so3_synth": ("k_so3_synth", "k_so3_synth_tc"),
-    "so3_fft": ("k_so3_fft_a", "k_so3_c2r_tail"),
+    "so3_fft": ("k_so3_fft_a", "k_so3_c2r", "k_so3_c2r_tail"),
     "voxelize": ("k_voxelize",),
-    "spatial_fwd": ("k_slab_fwd",),
+    "spatial_fwd": ("k_scan_rows", "k_fft_x_fwd"),
     "fuse_z": ("k_fuse_z",),
-    "spatial_inv": ("k_slab_inv",),
+    "spatial_inv": ("k_fft_x_inv", "k_c2r_rows"),
 }
 
 TRAFFIC_PROFILE = os.path.join(ROOT, "profiles", "traffic_register_pair_B100_N200.md")
@@ -294,6 +295,8 @@ def roofline(nat, pool, params, tuning, served_value):
     stages = {}
     for k, (ms, calls) in tot.items():
         nb = stage_bytes(k, bw, N, C, P)
+        if k == "s2_sample":  # both clouds in one call
+            nb *= max(1, 2 * nrep // calls)
         per = ms / calls
         e = {"ms_per_call": round(per, 4), "calls_per_pair": round(calls / nrep, 2),
              "ms_per_pair": round(ms / nrep, 4)}

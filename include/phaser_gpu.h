@@ -292,7 +292,8 @@ double phgpu_translation_from_index(double index, uint32_t n_voxels, int32_t low
  * of runtime FFT plans (lengths other than 64, 128, 200, 256, 320 and 512) and
  * so their FP32 rounding. */
 typedef struct {
-  uint32_t fuse_z_tile;    /* ky columns per block of the translation z pass: 2, 4, 8, 16 */
+  uint32_t fuse_z_tile;    /* ky columns per block of the translation z pass: 2, 4, 8, 16
+                              (compile-time lengths: 4, or 8 from 8 on) */
   uint32_t so3_beta_tile;  /* betas per block of the SO(3) alpha transform: 8, 16, 32 */
   uint32_t tc_chunk;       /* degrees per chunk of the tensor-core synthesis: 16, 32 */
   uint32_t radix_order;    /* runtime FFT plans: 0 radix 8 first, 1 radix 4 first, 2 odd radices first */

@@ -471,11 +471,6 @@ struct FixedFft<320> {  // 2 bw_out for bw_out = 160 (B = 150 with zero padding 
   static constexpr int r[3] = {8, 8, 5};
 };
 
-template <int N>
-constexpr bool fixed_fft_supported() {
-  return FixedFft<N>::count > 0;
-}
-
 template <int N, int S>
 __host__ __device__ constexpr int fixed_L() {
   if constexpr (S == 0) {

@@ -138,7 +138,8 @@ __device__ __forceinline__ void pass_stage_rt(const FftPlan& p, int s, PassMap m
 // a quarter of the products of the plain sum, each a packed pair times a real
 // constant (one FFMA2).  A work item is kPrimeOuts values of k for kPrimeBfs
 // butterflies; items of whole butterflies are summed in rounds of one item
-// per thread, since the outputs overwrite the inputs.  cs: shared scratch of R
+// per thread, since the outputs overwrite the inputs (z pass of N = 201: 1065 us
+// with plain complex sums, 388 so).  cs: shared scratch of R
 // float4 (cos, cos, sin, sin), filled here.  Every thread must call it; it
 // begins after a barrier of the caller's and ends with one.
 constexpr int kPrimeOuts = 4;

