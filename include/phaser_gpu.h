@@ -89,7 +89,8 @@ typedef struct {
 
 /* A point cloud: x, y, z, intensity as float4 plus optional per-point
  * reflectivity and ambient values (phaser_common/include/phaser/model/
- * point-cloud.h:18-88).  on_device = 1 when the pointers are device memory. */
+ * point-cloud.h:18-88).  on_device = 1 when the pointers are device memory;
+ * whole clouds that are 16-byte aligned are then read in place during the call. */
 typedef struct {
   const float* xyzi;          /* 4 * n_points floats */
   const float* reflectivity;  /* n_points floats or NULL */
