@@ -1,6 +1,6 @@
-"""The voxel grid's radix passes on both sides of the 2^16-cell line (the last
-two passes are skipped below it): leaf order, counts and centroids equal the
-oracle's bit for bit."""
+"""The voxel grid's radix passes around the cell counts where their number
+changes, leaf lengths around the centroid's batches and clouds around the scan
+kernels' limits: leaf order, counts and centroids equal the oracle's bit for bit."""
 import numpy as np
 import pytest
 
