@@ -760,6 +760,8 @@ __global__ void __launch_bounds__(kVgThreads) k_vg_centroid(const float4* __rest
       }
       __syncthreads();
     }
+    // no warp writes the next batch's s_b, s_n before every warp has read this one's to the last leaf
+    __syncthreads();
   }
 }
 

@@ -71,3 +71,26 @@ def test_tiles_around_the_scan_kernels(n):
     rng = np.random.default_rng(1)
     x = (rng.integers(0, 400, (n, 4)) / np.float32(4)).astype(np.float32)
     _both(x, 4.0, 2, None)
+
+
+@pytest.mark.parametrize("seed", [0, 1, 2])
+def test_long_leaves_in_consecutive_batches(seed):
+    """More leaves than the centroid's grid takes at a time (8 warps of 2368 blocks): blocks that have long leaves in
+    one batch and, in other warps' places, in the next, with short ones between them."""
+    rng = np.random.default_rng(seed)
+    blocks, batch = 2368, 8 * 2368
+    counts = rng.integers(1, 5, 2 * batch + 5000)
+    lengths = np.array([129, 130, 895, 896, 897, 1793, 3000])
+    for b in rng.choice(blocks, 60, replace=False):
+        for turn in range(3):
+            w = rng.choice(8, rng.integers(1, 4), replace=False)
+            leaf = turn * batch + b + w * blocks
+            leaf = leaf[leaf < len(counts)]
+            counts[leaf] = rng.choice(lengths, len(leaf))
+    ijk = rng.permutation(np.repeat(np.arange(len(counts)), counts))
+    x = rng.uniform(0.1, 0.9, (len(ijk), 4)).astype(np.float32)
+    x[:, 0] += ijk
+    from phaser_b200 import native
+    vg = native.VoxelGrid(len(x))
+    for _ in range(3):
+        _both(x, 1.0, 0, vg)
