@@ -36,6 +36,12 @@ __device__ __forceinline__ int fast_div(int x, uint32_t mul) {
   return mul ? (int)__umulhi((uint32_t)x, mul) : x;
 }
 
+// Whether a plan ends in a prime stage above the small radices.  A transform of
+// length 1 has no stage.
+__host__ __device__ constexpr bool ends_in_prime_stage(const FftPlan& p) {
+  return p.nstage > 0 && p.radix[p.nstage - 1] > 13;
+}
+
 // Largest radix of the passes' register butterflies (fft_pass.cuh); larger
 // primes take the shared-memory stage there.
 constexpr int kMaxRegRadix = 8;

@@ -921,8 +921,6 @@ static bool fixed_length(int N) {
   return fixed;
 }
 
-static bool prime_stage(const FftPlan& p) { return p.radix[p.nstage - 1] > 13; }
-
 // Registers a thread of the passes with runtime plans (their launch bounds' share); 0 for compile-time ones.
 static int pass_regs(int N) { return fixed_length(N) ? 0 : 96; }
 
@@ -1014,7 +1012,7 @@ cudaError_t launch_spatial_forward(const SpatialArgs& a, int side, cudaStream_t 
     cx.spec += (size_t)ch * plane;
     const int k = std::min(cc, nch - ch);
     const bool fixed = fixed_length(N);  // an item carries all channels, or one of them
-    const int tx = pass_threads(*a.plan, (1 << kXFwdLog2) * (fixed ? 1 : k), fixed ? k : 1, fixed || prime_stage(*a.plan) ? 160 : 128, kXThreads,
+    const int tx = pass_threads(*a.plan, (1 << kXFwdLog2) * (fixed ? 1 : k), fixed ? k : 1, fixed || ends_in_prime_stage(*a.plan) ? 160 : 128, kXThreads,
                                 pass_regs(N), k * per + extra);
     FftXFn fn = nullptr;
     PHGPU_DISPATCH_N(N, fn = fft_x_forward<NF>(k));
