@@ -211,7 +211,7 @@ struct VoxelArgs {
 };
 cudaError_t launch_voxelize(const VoxelArgs& a, cudaStream_t st);
 // Zeroes what one voxelisation wrote: every point's voxel (lin[i] !=
-// 0xffffffff) and row flag.
+// 0xffffffff) or whole flagged rows, and the row flags.
 cudaError_t launch_clear_voxels(const uint32_t* lin, int n_points, float4* sums, float* counts, uint8_t* rowlive, int N,
                                 cudaStream_t st);
 struct SpatialArgs {

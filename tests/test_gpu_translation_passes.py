@@ -112,3 +112,32 @@ def test_voxels_of_a_smaller_cloud_are_cleared(nat):
     c.register_pair(large[:2], small[:2])
     vol = volume(c, small, large)
     np.testing.assert_allclose(vol, fresh, rtol=0, atol=1e-6 * np.abs(fresh).max())
+
+
+@pytest.mark.parametrize("first", [1, 511, 512, 513, 5000])
+def test_voxels_are_cleared_by_points_and_by_rows(nat, first):
+    """The next voxelisation clears the last one's voxels point by point below an eighth of the 16^3 voxels, its
+    rows whole from there on; points outside the grid and a second cloud of another size in between."""
+    rng = np.random.default_rng(first)
+    N, half = 16, 10
+
+    def points(n):
+        xyzi = rng.uniform(-1.1 * half, 1.1 * half, (n, 4)).astype(np.float32)
+        return xyzi, rng.uniform(0.1, 1.0, n).astype(np.float32)
+
+    kw = dict(spherical_bandwidth=2, spatial_n_voxels=N, spatial_discretize_lower=-half, spatial_discretize_upper=half,
+              flags=nat.PHGPU_FLAG_KEEP_VOLUMES)
+    small, other = points(40), points(60)
+
+    def volume(c):
+        c.voxelize(*small, side=0)
+        c.voxelize(*other, side=1)
+        c.spatial_correlate_voxelized()
+        return c.spatial_result(volume=True)[2]
+
+    fresh = volume(nat.Context(**kw))
+    c = nat.Context(max_points=6000, **kw)
+    for n in (first, 600, first):
+        for side in range(2):
+            c.voxelize(*points(n), side=side)
+    np.testing.assert_allclose(volume(c), fresh, rtol=0, atol=1e-6 * np.abs(fresh).max())
