@@ -236,9 +236,12 @@ __global__ void __launch_bounds__(kSo3C2rThreads, NF > 0 ? 3 : 2)
   };
   const float K = (float)((1.0 / (double)n) * ((double)Bo / M_PI));
   float* volume = o.volume;
-  // per thread: the largest value, the lowest index among equal ones
+  // per thread: the largest value, the lowest index among equal ones (NaN
+  // compares false); a volume whose first value is NaN has its peak there, as
+  // for the reference's max_element
   float bv = -1.0f;
   uint32_t bi = 0xffffffffu;
+  bool nan_first = false;
   if constexpr (NF > 0) {
     constexpr int cnt = FixedFft<NF>::count;
     constexpr int R = FixedFft<NF>::r[cnt - 1], nb = NF / R;
@@ -273,6 +276,7 @@ __global__ void __launch_bounds__(kSo3C2rThreads, NF > 0 ? 3 : 2)
       for (int k = 1; k < R0; ++k) x[k] = cmul(x[k], cconj(__ldg(plan.tw + j2 * k)));
       dft_small<R0, true>(x);
       const uint32_t idx = ((uint32_t)(k0 + 2 * pk) * n + (uint32_t)alpha) * n + j2;
+      nan_first |= idx == 0 && isnan(x[0].x);
 #pragma unroll
       for (int h = 0; h < 2; ++h)
 #pragma unroll
@@ -300,9 +304,10 @@ __global__ void __launch_bounds__(kSo3C2rThreads, NF > 0 ? 3 : 2)
     __syncthreads();
     const int lwp = 32 - __clz(np - 1);
     auto at = [=](int g, int t, int i, int m) { return SmemCursor{zrow + (g + t) * st + i, m, 0}; };
-    auto sv = [=, &bv, &bi](int g, int t, int i, int m) {
+    auto sv = [=, &bv, &bi, &nan_first](int g, int t, int i, int m) {
       const uint32_t idx = ((uint32_t)(k0 + 2 * (g + t)) * n + (uint32_t)alpha) * n + i;
-      return [=, &bv, &bi](int, int j, float2 z) {
+      return [=, &bv, &bi, &nan_first](int, int j, float2 z) {
+        nan_first |= idx == 0 && j == 0 && isnan(z.x);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const float v = (h ? z.y : z.x) * K, v2 = v * v;
@@ -316,6 +321,10 @@ __global__ void __launch_bounds__(kSo3C2rThreads, NF > 0 ? 3 : 2)
       };
     };
     pass_rt<true, 1, true>(plan, PassMap{1, lwp}, PassMap{1, lwp}, PassMap{np, 0}, cs, tid, nthr, at, at, sv);
+  }
+  if (nan_first) {
+    bv = __int_as_float(0x7fffffff);  // orders above every number
+    bi = 0;
   }
   warp_argmax_commit(bi == 0xffffffffu ? 0ull : pack_argmax(bv, bi), o.argmax);
 }

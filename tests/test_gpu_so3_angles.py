@@ -42,3 +42,17 @@ def test_equal_values_take_the_first_bin(nat):
     c.sph_correlate(list(z), list(z))
     b, peak, vol = c.sph_result(volume=True)
     assert b == 0 and peak == 0.0 and not vol.any()
+
+
+@pytest.mark.parametrize("bw", [8, 32, 37])
+def test_undefined_volume_has_its_peak_at_the_first_bin(nat, bw):
+    """One NaN sample makes every bin NaN: the reference's max_element then stays at the first one."""
+    rng = np.random.default_rng(bw)
+    f, g = rng.standard_normal((2, 1, 4 * bw * bw))
+    f[0, 5] = np.nan
+    c = nat.Context(spherical_bandwidth=bw, spatial_n_voxels=4, spherical_fusion=nat.PHGPU_FUSION_NONE,
+                    flags=nat.PHGPU_FLAG_KEEP_VOLUMES)
+    c.sph_correlate(list(f), list(g))
+    b, peak, vol = c.sph_result(volume=True)
+    assert np.isnan(vol).all()
+    assert b == O.argmax(vol) == 0 and np.isnan(peak)
