@@ -215,7 +215,7 @@ template <int NF>
 __global__ void __launch_bounds__(kSo3C2rThreads, NF > 0 ? 3 : 2)
     k_so3_c2r(int bw_in, int bw_out, const __grid_constant__ So3Batch bt, const __grid_constant__ FftPlan plan) {
   chain_begin();
-  extern __shared__ __align__(16) float2 zrow[];  // [kSo3Pairs][st] | float4 cs[] | int pos[n] (runtime plans)
+  extern __shared__ __align__(16) float2 zrow[];  // [kSo3Pairs][st] | float4 cs[] | int16 pos[n] (runtime plans)
   const int n = NF > 0 ? NF : 2 * bw_out;
   const int Bo = n / 2, st = n | 1;
   const So3Out& o = bt.out[blockIdx.z];
@@ -292,8 +292,8 @@ __global__ void __launch_bounds__(kSo3C2rThreads, NF > 0 ? 3 : 2)
     }
   } else {
     float4* cs = reinterpret_cast<float4*>(zrow + (size_t)kSo3Pairs * st);
-    int* pos = reinterpret_cast<int*>(cs + kMaxGenericRadix);
-    for (int k = tid; k < n; k += nthr) pos[k] = freq2pos<NF>(k, plan);
+    short* pos = reinterpret_cast<short*>(cs + kMaxGenericRadix);
+    for (int k = tid; k < n; k += nthr) pos[k] = (short)freq2pos<NF>(k, plan);
     __syncthreads();
     for (int it = tid; it < kSo3Pairs * (Bo + 1); it += nthr) {
       const int pk = it % kSo3Pairs, b = it / kSo3Pairs;
@@ -383,7 +383,7 @@ template <int NF>
 static void launch_so3_c2r(const So3Args& a, int n, cudaStream_t st) {
   const dim3 g((n + 2 * kSo3Pairs - 1) / (2 * kSo3Pairs), n, a.batch.count);
   size_t sm = (size_t)kSo3Pairs * (n | 1) * sizeof(float2);
-  if (NF == 0) sm += so3_prime_scratch(n) + (size_t)n * sizeof(int);
+  if (NF == 0) sm += so3_prime_scratch(n) + (size_t)n * sizeof(short);  // fits up to n = 1770
   const int thr = NF > 0 ? pass_threads(*a.plan, kSo3Pairs, 1, 160, kSo3C2rThreads)
                          : pass_threads(*a.plan, kSo3Pairs, 1, 128, kSo3C2rThreads, 96, sm);
   launch_kernel(k_so3_c2r<NF>, dim3(g), dim3(thr), sm, st, a.bw_in, a.bw_out, a.batch, *a.plan);

@@ -56,3 +56,21 @@ def test_undefined_volume_has_its_peak_at_the_first_bin(nat, bw):
     b, peak, vol = c.sph_result(volume=True)
     assert np.isnan(vol).all()
     assert b == O.argmax(vol) == 0 and np.isnan(peak)
+
+
+@pytest.mark.parametrize("pad", [871, 873, 878])
+def test_longest_transforms(nat, pad):
+    """Lengths 1746 = 2 9 97, 1750 and 1760, the longest whose tiles fit (22 GB of spectra).  The correlation of two
+    signals of bandwidth 2 is a trigonometric polynomial of degree 1 per angle, its square z^2 of degree 2 with
+    |d^2 z^2| <= 4 max z^2: grids of spacing h <= 2 pi / 804 miss its maximum by at most 3 * 4 / 2 (h / 2)^2 = 9.2e-5
+    of it, and the transforms add 1e-5."""
+    rng = np.random.default_rng(9)
+    f, g = rng.standard_normal((2, 1, 16))
+    peaks = []
+    for p in (400, pad):
+        c = nat.Context(spherical_bandwidth=2, spherical_zero_padding=p, spatial_n_voxels=4,
+                        spherical_fusion=nat.PHGPU_FUSION_NONE)
+        c.sph_correlate(list(f), list(g))
+        peaks.append(c.sph_result()[1])
+        c.close()
+    assert abs(peaks[1] - peaks[0]) <= 1.2e-4 * peaks[0]
