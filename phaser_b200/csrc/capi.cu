@@ -559,6 +559,17 @@ int phgpu_ctx_init(phgpu_ctx* ctx) {
     ctx->err = perr;
     return PHGPU_ERR_INVALID;
   }
+  if (N % 2 == 0 && *std::max_element(ctx->plan_sp.radix, ctx->plan_sp.radix + ctx->plan_sp.nstage) <= kMaxRegRadix) {
+    if (!make_fft_plan(N / 2, &ctx->plan_sp_half, &ctx->d_tw[3], &perr)) {
+      ctx->err = perr;
+      return PHGPU_ERR_INVALID;
+    }
+    std::vector<uint16_t> pos(N / 2);
+    for (int k = 0; k < N / 2; ++k) pos[k] = (uint16_t)fft_freq2pos(k, ctx->plan_sp_half);
+    CKV(dalloc(ctx, &ctx->d_half_pos, sizeof(uint16_t) * pos.size()));
+    CK(cudaMemcpy(ctx->d_half_pos, pos.data(), sizeof(uint16_t) * pos.size(), cudaMemcpyHostToDevice));
+    ctx->has_sp_half = true;
+  }
   if (ctx->pad) {
     if (!make_fft_plan(ctx->M, &ctx->plan_pad, &ctx->d_tw_pad, &perr)) {
       ctx->err = perr;
@@ -698,7 +709,7 @@ int phgpu_ctx_destroy(phgpu_ctx* ctx) {
   if (ctx->s1) cudaStreamSynchronize(ctx->s1);
   for (void* p : ctx->allocs) cudaFree(p);
   ctx->allocs.clear();
-  for (int i = 0; i < 3; ++i)
+  for (int i = 0; i < 4; ++i)
     if (ctx->d_tw[i]) cudaFree(ctx->d_tw[i]);
   if (ctx->d_tw_pad) cudaFree(ctx->d_tw_pad);
   if (ctx->h_argmax) cudaFreeHost(ctx->h_argmax);
@@ -1147,6 +1158,8 @@ static SpatialArgs spatial_args(phgpu_ctx* ctx, int n_data, int n_total, int lap
   a.spec = ctx->d_spec;
   a.cspec = ctx->d_cspec;
   a.plan = &ctx->plan_sp;
+  a.plan_half = ctx->has_sp_half ? &ctx->plan_sp_half : nullptr;
+  a.half_pos = ctx->d_half_pos;
   a.argmax = ctx->d_argmax + 1;
   a.volume = ctx->d_transvol;
   a.fuse_tile = (int)ctx->tune.fuse_z_tile;

@@ -38,8 +38,10 @@ struct phgpu_ctx {
   cudaStream_t s0 = nullptr, s1 = nullptr;
   cudaEvent_t ev_a = nullptr, ev_b = nullptr;
   // plans and tables
-  phgpu::FftPlan plan_s2, plan_so3, plan_sp;
-  float2* d_tw[3] = {nullptr, nullptr, nullptr};
+  phgpu::FftPlan plan_s2, plan_so3, plan_sp, plan_sp_half;
+  bool has_sp_half = false;  // N is even and N / 2 has register radices only
+  uint16_t* d_half_pos = nullptr;
+  float2* d_tw[4] = {nullptr, nullptr, nullptr, nullptr};
   phgpu::FusionBands bands_s2, bands_sp;
   float4* d_grid = nullptr;
   double* d_weights = nullptr;

@@ -200,7 +200,7 @@ constexpr int kMaxVoxels = 1024;  // longest transform
 // packed multiply-add per channel.  Rows without a point are neither read nor
 // written: the x transform takes them as zero.
 //
-// Block: kRowsBlock rows of one z-slab; a warp takes a live row, gathers its
+// Block: 16 rows (fewer on small grids, scan_rows_block) of one z-slab; a warp takes a live row, gathers its
 // occupied voxels in order (counts, then every channel's sums, all loads of 256
 // voxels in flight) into shared memory and gives each lane up to four
 // frequencies at a time.  Small blocks spread a slab full of long rows (a floor
@@ -209,19 +209,30 @@ constexpr int kMaxVoxels = 1024;  // longest transform
 // separate pass before its next voxelisation.  With the x pass behind it a side
 // of an N = 200 room takes 39 us (whole slabs at one block an SM: 43 to 65) and
 // of an N = 512 one 285 (dense rows and columns: some 1450).
-constexpr int kRowsBlock = 16;
 constexpr int kRowsWarps = 4;
 // One running sum over a row rounds in proportion to the root of its voxels:
-// past some twenty it is further off than an FFT (a full row of 512: 3.9e-7
-// against 0.9e-7, relative L2).  Sums of 8 voxels, of 8 such sums and then over
-// the row stay below the FFT's error at every length and occupancy (0.9e-7
-// there; rows of up to 8 voxels, a scan's, are summed as before).  Sums beyond
-// the first 64 voxels are added to the stored ones: no third set of registers.
+// from some twenty on it is further off than an FFT (a full row of 512: 3.9e-7
+// against 0.9e-7, relative L2; of 16 voxels 0.7e-7 against 0.8e-7).  Lengths with a
+// half plan (below) sum shorter rows only; at the others, sums of 8 voxels, of
+// 8 such sums and then over the row stay below the FFT's error at every length
+// and occupancy (0.9e-7 there).  Sums beyond the first 64 voxels are added to the
+// stored ones: no third set of registers.
 constexpr int kPartSum = 8;
 constexpr int kRunSum = 64;
 
+// A row of many voxels takes an FFT after all: a real transform of n points as
+// a complex one of n / 2 (even and odd columns as real and imaginary parts) per
+// channel, by the warp that gathered the row, where n / 2 has a plan of
+// register radices (n is even, no prime above 7).  A voxel's sum costs every
+// frequency an addition, the FFT costs the same whatever the row holds: they
+// meet at 16 to 24 voxels, and from 16 on the sum rounds more.  A row of a room's
+// scan has four to six; the correlation of two full grids took 107 us summed at
+// N = 64 and now 73, 376 and 205 at N = 128, 1370 and 510 at N = 200, 4518 and
+// 1385 at N = 256.
+constexpr int kDenseRow = 16;
+
 struct ScanRowArgs {
-  int N;
+  int N, rows_block;
   float4* sums;         // [N^3] channel sums
   float* counts;        // [N^3] points
   const float2* tw;     // N twiddles
@@ -230,19 +241,90 @@ struct ScanRowArgs {
   float2* spec;         // [channel][z][x][H2p]
   size_t spec_stride;
   int clear;
+  FftPlan half;         // length N / 2 for dense rows; n = 0: every row is summed
+  const uint16_t* half_pos;  // [N / 2] position of each of its frequencies
 };
+
+// Channel c of a row as N / 2 complex values in place of its [N] float4 means:
+// element i is columns 2 i and 2 i + 1.
+struct EvenOddCursor {
+  float* p;
+  int es;
+  __device__ __forceinline__ float2 operator()(int, int j) const { return make_float2(p[j * es], p[j * es + 4]); }
+  __device__ __forceinline__ void operator()(int, int j, float2 v) const {
+    p[j * es] = v.x;
+    p[j * es + 4] = v.y;
+  }
+};
+
+// Transforms one dense row by the calling warp.  s_val, s_y: the row's cnt
+// occupied columns in order; occ: lane w's bits are columns 32 w .. 32 w + 31.
+template <int CC>
+__device__ __noinline__ void dense_row(const ScanRowArgs& a, float4* s_val, const uint16_t* s_y,
+                                          const float2* __restrict__ s_tw, unsigned occ, int cnt, int lane, float2* out) {
+  const int n = a.N, nh = n / 2;
+  // the list spread to its columns, last entries first: a column is never before its place in the list
+  for (int e0 = (cnt - 1) & ~31; e0 >= 0; e0 -= 32) {
+    const bool ok = e0 + lane < cnt;
+    const float4 v = ok ? s_val[e0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int y = ok ? s_y[e0 + lane] : 0;
+    __syncwarp();
+    if (ok) s_val[y] = v;
+    __syncwarp();
+  }
+  for (int w = 0; 32 * w < n; ++w) {
+    const unsigned m = __shfl_sync(0xffffffffu, occ, w);
+    if (32 * w + lane < n && !((m >> lane) & 1u)) s_val[32 * w + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  __syncwarp();
+  float* f = reinterpret_cast<float*>(s_val);
+  auto at = [=](int, int t, int i, int m) { return EvenOddCursor{f + 8 * i + t, 8 * m}; };
+  const PassMap map{1, CC == 1 ? 0 : (CC == 2 ? 1 : 2)};
+  for (int s = 0; s < a.half.nstage; ++s) {
+    pass_stage_rt<false, 1>(a.half, s, map, lane, 32, at, at);
+    __syncwarp();
+  }
+  // X[k] = (Z[k] + conj Z[-k]) / 2 + w^k (Z[k] - conj Z[-k]) / 2i
+  for (int k = lane; k < nh; k += 32) {
+    const int p0 = 2 * __ldg(a.half_pos + k), p1 = 2 * __ldg(a.half_pos + (k == 0 ? 0 : nh - k));
+    const float4 ur = s_val[p0], ui = s_val[p0 + 1], vr = s_val[p1], vi = s_val[p1 + 1];
+    const float2 w = s_tw[k];
+    auto bin = [&](int c, float xr, float xi, float yr, float yi) {
+      if (c >= CC) return;
+      float2* o = out + c * a.spec_stride + k;
+      *o = cadd(make_float2(0.5f * (xr + yr), 0.5f * (xi - yi)), cmul(w, make_float2(0.5f * (xi + yi), -0.5f * (xr - yr))));
+      if (k == 0) o[nh] = make_float2(xr - xi, 0.f);
+    };
+    bin(0, ur.x, ui.x, vr.x, vi.x);
+    bin(1, ur.y, ui.y, vr.y, vi.y);
+    bin(2, ur.z, ui.z, vr.z, vi.z);
+    bin(3, ur.w, ui.w, vr.w, vi.w);
+  }
+}
 
 // Shared memory: N twiddles, then per warp N float4 (means) and N uint16 (y).
 static size_t scan_rows_smem(int N) { return (size_t)N * (8 + kRowsWarps * 18) + 16 * (kRowsWarps + 1); }
 
-template <int CC>
-__global__ void __launch_bounds__(kRowsWarps * 32) k_scan_rows(const ScanRowArgs a) {
+// Rows of a block: 16, halved down to one a warp while the blocks are fewer
+// than twice those resident (six an SM), so a slab of dense rows does not wait
+// for one warp's four in turn (the correlation of two full grids with 16 rows: N =
+// 64 87 us, with 4 75; N = 128 215, with 8 202; with 4 rows at N = 200 a scan's
+// empty blocks cost 11 us).
+static int scan_rows_block(int N) {
+  int rows = 16;
+  while (rows > kRowsWarps && N * ((N + rows - 1) / rows) < 2 * 6 * 148) rows /= 2;
+  return rows;
+}
+
+// FFT: the length has a half plan (dense rows are transformed, the others' sums are short).
+template <int CC, bool FFT>
+__global__ void __launch_bounds__(kRowsWarps * 32) k_scan_rows(const __grid_constant__ ScanRowArgs a) {
   chain_begin();
   extern __shared__ __align__(16) float4 s_mem[];
   constexpr int U = 8, Q = 4;
   const int n = a.N, H2 = n / 2 + 1, H2p = spatial_h2p(n);
-  const int z = blockIdx.x, x0 = blockIdx.y * kRowsBlock, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const bool mine = lane < kRowsBlock && x0 + lane < n;
+  const int z = blockIdx.x, x0 = blockIdx.y * a.rows_block, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool mine = lane < a.rows_block && x0 + lane < n;
   const bool live_l = mine && a.rowlive[(size_t)z * n + x0 + lane];
   const unsigned live = __ballot_sync(0xffffffffu, live_l);  // every warp: the block's rows
   if (warp == 0 && mine) a.rowmask[(size_t)z * n + x0 + lane] = live_l ? 1 : 0;
@@ -261,6 +343,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32) k_scan_rows(const ScanRowArgs
     float* c = a.counts + row * n;
     float4* g = a.sums + row * n;
     int cnt = 0;
+    unsigned bits = 0;  // occupied columns 32 lane .. 32 lane + 31
     for (int y0 = 0; y0 < n; y0 += 32 * U) {
       float q[U];
 #pragma unroll
@@ -272,6 +355,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32) k_scan_rows(const ScanRowArgs
       for (int u = 0; u < U; ++u) {
         const bool occ = q[u] > 0.f;
         const unsigned m = __ballot_sync(0xffffffffu, occ);
+        if (lane == y0 / 32 + u) bits = m;
         if (occ) {
           const int y = y0 + 32 * u + lane, at = cnt + __popc(m & ((1u << lane) - 1u));
           const float inv = __frcp_rn(q[u]);  // mean = sum * (1 / count)
@@ -287,52 +371,72 @@ __global__ void __launch_bounds__(kRowsWarps * 32) k_scan_rows(const ScanRowArgs
     }
     __syncwarp();
     float2* out = a.spec + row * H2p;
-    for (int k0 = 0; k0 < H2; k0 += 32 * Q) {
-      int e = 0;
-      do {
-        float2 sum[CC][Q];
-#pragma unroll
-        for (int ch = 0; ch < CC; ++ch)
-#pragma unroll
-          for (int i = 0; i < Q; ++i) sum[ch][i] = make_float2(0.f, 0.f);
-        const int stored = e, run = min(cnt, e + kRunSum);
-        while (e < run) {
-          float2 acc[CC][Q];
-#pragma unroll
-          for (int ch = 0; ch < CC; ++ch)
-#pragma unroll
-            for (int i = 0; i < Q; ++i) acc[ch][i] = make_float2(0.f, 0.f);
-          const int end = min(run, e + kPartSum);
+    if constexpr (FFT) {
+      if (cnt > kDenseRow) {
+        dense_row<CC>(a, s_val, s_y, s_tw, bits, cnt, lane, out);
+        __syncwarp();
+        continue;
+      }
+    }
+    // X[k0 + 32 i + lane] plus the sum over entries [e, end) of the list
+    auto add = [&](float2 (&acc)[CC][Q], int k0, int& e, int end) {
 #pragma unroll 2
-          for (; e < end; ++e) {
-            const uint32_t y = s_y[e];
-            const float4 w = s_val[e];
-            const float ws[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-            for (int i = 0; i < Q; ++i) {
-              const uint32_t k = (uint32_t)(k0 + 32 * i + lane) * y;
-              const float2 t = s_tw[k - __umulhi(k, mul) * (uint32_t)n];
-#pragma unroll
-              for (int ch = 0; ch < CC; ++ch) acc[ch][i] = __ffma2_rn(make_float2(ws[ch], ws[ch]), t, acc[ch][i]);
-            }
-          }
-#pragma unroll
-          for (int ch = 0; ch < CC; ++ch)
-#pragma unroll
-            for (int i = 0; i < Q; ++i) sum[ch][i] = cadd(sum[ch][i], acc[ch][i]);
-        }
+      for (; e < end; ++e) {
+        const uint32_t y = s_y[e];
+        const float4 w = s_val[e];
+        const float ws[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
         for (int i = 0; i < Q; ++i) {
-          const int ky = k0 + 32 * i + lane;
-          if (ky < H2) {
+          const uint32_t k = (uint32_t)(k0 + 32 * i + lane) * y;
+          const float2 t = s_tw[k - __umulhi(k, mul) * (uint32_t)n];
 #pragma unroll
-            for (int ch = 0; ch < CC; ++ch) {
-              float2* o = out + ch * a.spec_stride + ky;
-              *o = stored ? cadd(*o, sum[ch][i]) : sum[ch][i];
-            }
+          for (int ch = 0; ch < CC; ++ch) acc[ch][i] = __ffma2_rn(make_float2(ws[ch], ws[ch]), t, acc[ch][i]);
+        }
+      }
+    };
+    auto zero = [](float2 (&acc)[CC][Q]) {
+#pragma unroll
+      for (int ch = 0; ch < CC; ++ch)
+#pragma unroll
+        for (int i = 0; i < Q; ++i) acc[ch][i] = make_float2(0.f, 0.f);
+    };
+    auto put = [&](const float2 (&acc)[CC][Q], int k0, bool more) {
+#pragma unroll
+      for (int i = 0; i < Q; ++i) {
+        const int ky = k0 + 32 * i + lane;
+        if (ky < H2) {
+#pragma unroll
+          for (int ch = 0; ch < CC; ++ch) {
+            float2* o = out + ch * a.spec_stride + ky;
+            *o = more ? cadd(*o, acc[ch][i]) : acc[ch][i];
           }
         }
-      } while (e < cnt);
+      }
+    };
+    for (int k0 = 0; k0 < H2; k0 += 32 * Q) {
+      int e = 0;
+      if constexpr (FFT) {
+        float2 sum[CC][Q];
+        zero(sum);
+        add(sum, k0, e, cnt);
+        put(sum, k0, false);
+      } else {
+        do {
+          float2 sum[CC][Q];
+          zero(sum);
+          const int stored = e, run = min(cnt, e + kRunSum);
+          while (e < run) {
+            float2 part[CC][Q];
+            zero(part);
+            add(part, k0, e, min(run, e + kPartSum));
+#pragma unroll
+            for (int ch = 0; ch < CC; ++ch)
+#pragma unroll
+              for (int i = 0; i < Q; ++i) sum[ch][i] = cadd(sum[ch][i], part[ch][i]);
+          }
+          put(sum, k0, stored > 0);
+        } while (e < cnt);
+      }
     }
     __syncwarp();
   }
@@ -945,6 +1049,13 @@ static FftXFn fft_x_forward(int C) {
                           : (C == 3 ? k_fft_x<NF, false, 3, kXFwdLog2> : k_fft_x<NF, false, 4, kXFwdLog2>));
 }
 
+using ScanRowsFn = void (*)(const ScanRowArgs);
+template <bool FFT>
+static ScanRowsFn scan_rows_channels(int C) {
+  return C == 1 ? k_scan_rows<1, FFT> : (C == 2 ? k_scan_rows<2, FFT> : (C == 3 ? k_scan_rows<3, FFT> : k_scan_rows<4, FFT>));
+}
+static ScanRowsFn scan_rows_kernel(int C, bool fft) { return fft ? scan_rows_channels<true>(C) : scan_rows_channels<false>(C); }
+
 template <int NF>
 static cudaError_t set_attrs() {
   cudaError_t e = cudaSuccess;
@@ -962,9 +1073,9 @@ cudaError_t spatial_init_attributes(int N, int M) {
   cudaError_t e = cudaSuccess;
   PHGPU_DISPATCH_N(N, e = set_attrs<NF>());
   if (e == cudaSuccess && M != N) PHGPU_DISPATCH_N(M, e = set_attrs<NF>());
-  for (auto fn : {(const void*)k_scan_rows<1>, (const void*)k_scan_rows<2>, (const void*)k_scan_rows<3>,
-                  (const void*)k_scan_rows<4>})
-    if (e == cudaSuccess) e = allow_max_smem(fn);
+  for (int C = 1; C <= 4; ++C)
+    for (bool fft : {false, true})
+      if (e == cudaSuccess) e = allow_max_smem((const void*)scan_rows_kernel(C, fft));
   return e;
 }
 
@@ -1043,18 +1154,12 @@ cudaError_t launch_spatial_forward(const SpatialArgs& a, int side, cudaStream_t 
     const int tr = pass_threads(*a.plan, kRowPairs, 1, 128, 320, pass_regs(N), smr);
     PHGPU_DISPATCH_N(N, launch_kernel(k_r2c_rows<NF>, dim3(gr), dim3(tr), smr, st, N, grids, nv, spec, plane, *a.plan));
   } else {
-    const ScanRowArgs r{N, reinterpret_cast<float4*>(grids), grids + 4 * nv, a.plan->tw, a.rowlive[side],
-                        a.rowmask + (size_t)side * N * N, spec, plane, a.clear};
-    const dim3 gr(N, (N + kRowsBlock - 1) / kRowsBlock);
+    const ScanRowArgs r{N, scan_rows_block(N), reinterpret_cast<float4*>(grids), grids + 4 * nv, a.plan->tw, a.rowlive[side],
+                        a.rowmask + (size_t)side * N * N, spec, plane, a.clear,
+                        a.plan_half ? *a.plan_half : FftPlan{}, a.half_pos};
+    const dim3 gr(N, (N + r.rows_block - 1) / r.rows_block);
     const size_t smr = scan_rows_smem(N);
-    if (nch == 1)
-      launch_kernel(k_scan_rows<1>, dim3(gr), dim3(kRowsWarps * 32), smr, st, r);
-    else if (nch == 2)
-      launch_kernel(k_scan_rows<2>, dim3(gr), dim3(kRowsWarps * 32), smr, st, r);
-    else if (nch == 3)
-      launch_kernel(k_scan_rows<3>, dim3(gr), dim3(kRowsWarps * 32), smr, st, r);
-    else
-      launch_kernel(k_scan_rows<4>, dim3(gr), dim3(kRowsWarps * 32), smr, st, r);
+    launch_kernel(scan_rows_kernel(nch, a.plan_half != nullptr), dim3(gr), dim3(kRowsWarps * 32), smr, st, r);
   }
   // channels of one launch: as many as leave two blocks an SM's shared memory
   const size_t per = (size_t)N * (1 << kXFwdLog2) * sizeof(float2), extra = prime_scratch(N) + (size_t)N;

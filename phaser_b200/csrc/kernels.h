@@ -235,6 +235,8 @@ struct SpatialArgs {
   float2* spec;           // [2 n_data_ch][N (z)][N (x)][H2p (ky)]
   float2* cspec;          // [N][N][H2p]
   const FftPlan* plan;    // length N
+  const FftPlan* plan_half;  // length N / 2 (dense rows of voxelised clouds), null where it has none
+  const uint16_t* half_pos;  // [N / 2] positions of its frequencies
   unsigned long long* argmax;  // reset by the z pass, taken by the inverse
   float* volume;          // optional N^3 correlation, [z][x][y]
   uint32_t argmax_limit = 0;   // argmax over indices < limit (0: all)

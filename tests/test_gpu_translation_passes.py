@@ -181,3 +181,50 @@ def test_full_rows_round_no_more_than_an_fft(nat, N):
     fft = error(c.spatial_result(volume=True)[2])
     print(f"N {N}: sums {rows:.3g}, FFT {fft:.3g}")
     assert rows <= 1.2 * fft <= REL_L2
+
+
+@pytest.mark.parametrize("N,channels", [(28, 1), (30, 2), (48, 3), (50, 4), (64, 3), (98, 2), (100, 3), (108, 4), (200, 1), (256, 1),
+                                        (320, 1)])
+def test_rows_around_the_density_limit(nat, N, channels):
+    """Rows of 16 (summed), 17 and N - 1 voxels (transformed), full ones and ones with a gap at either end, in one
+    slab: the correlation against FP64 at the bar for volumes, twice from kept grids, and again after a registration
+    that clears them on the way."""
+    rng = np.random.default_rng(N)
+    half = 10
+    edges = np.linspace(-half, half, N, dtype=np.float32)
+    at = np.clip(edges + 0.4 * (edges[1] - edges[0]), -half, half)
+    plain = channels == 1
+    kw = dict(spherical_bandwidth=8, spatial_n_voxels=N, spatial_discretize_lower=-half, spatial_discretize_upper=half,
+              spatial_fusion=nat.PHGPU_FUSION_NONE if plain else nat.PHGPU_FUSION_LAPLACE, flags=nat.PHGPU_FLAG_KEEP_VOLUMES)
+    c = nat.Context(**kw)
+    clouds, grids = [], []
+    for side in range(2):
+        cols = [np.arange(16), rng.choice(N, 16, replace=False), rng.choice(N, 17, replace=False), np.arange(N - 17, N),
+                np.arange(N), np.arange(1, N), np.arange(N - 1), np.array([N // 2])]
+        xyz = np.concatenate([np.stack([np.full(len(y), at[(3 * i + side) % N]), at[y], np.full(len(y), at[N // 3 + side])], 1)
+                              for i, y in enumerate(cols)])
+        xyzi = np.concatenate([xyz, rng.uniform(0.1, 1.0, (len(xyz), 1))], 1).astype(np.float32)
+        refl, amb = rng.uniform(0.1, 1.0, (2, len(xyzi))).astype(np.float32)
+        clouds.append((xyzi, refl if channels > 2 else None, amb if channels > 3 else None))
+        grids.append(O.discretize(*clouds[-1], N, -half, half).reshape(4, -1)[:1 if plain else 4])
+        c.voxelize(*clouds[-1], side=side)
+    if plain:
+        ax = (0, 1, 2)
+        F, G = (np.fft.rfftn(g.reshape(N, N, N), axes=ax) for g in grids)
+        ref = np.fft.irfftn(F * np.conj(G), (N, N, N), axes=ax).reshape(-1) * N ** 3
+    else:
+        ref = O.spatial_correlation(grids[0], grids[1], N, laplace=True)
+
+    def check():
+        c.spatial_correlate_voxelized()
+        vol = c.spatial_result(volume=True)[2]
+        err = np.linalg.norm(vol - ref) / np.linalg.norm(ref) if plain else tie_masked_rel_l2(vol, ref, grids[0], grids[1], N)[0]
+        assert err <= REL_L2
+        return vol
+
+    vol = check()
+    assert np.array_equal(check(), vol)
+    c.register_pair(clouds[0][:2], clouds[1][:2])
+    for side in range(2):
+        c.voxelize(*clouds[side], side=side)
+    check()
