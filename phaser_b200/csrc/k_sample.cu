@@ -15,7 +15,7 @@
 // every run of neighbouring columns of a row, is one contiguous point range.
 // A direction (i, j), one group of 8 lanes, sweeps the non-empty rows outward from its
 // own row while the row's colatitude distance |theta_q - row| can still beat
-// the bound; a row whose window is wide is probed at columns j-1..j+1 for a
+// the bound; a row whose window is wide and full is probed at columns j-1..j+1 for a
 // tighter bound, and in each row only the columns whose longitudes lie within
 // the bound's spherical cap are scanned (the cap's longitude half-width at
 // the row's colatitudes).  A LiDAR scan needs about two rows and fifty
@@ -328,16 +328,29 @@ __device__ __forceinline__ void scan_range(uint32_t k, uint32_t e, int g, float 
 
 // Columns c0 .. c0 + len - 1 (mod n2b) of row r (len <= 0: none): one run of
 // the sorted points, two where the columns wrap.
-__device__ __forceinline__ void scan_cols(int r, int c0, int len, int n2b, int g, float qx, float qy, float qz,
-                                          const uint32_t* __restrict__ bin_start, const float4* __restrict__ sorted,
-                                          NnKey& best) {
+struct Window {
+  uint32_t k0, e0, k1, e1;
+  __device__ __forceinline__ uint32_t points() const { return e0 - k0 + e1 - k1; }
+};
+__device__ __forceinline__ Window window(int r, int c0, int len, int n2b, const uint32_t* __restrict__ bin_start) {
+  Window w{0, 0, 0, 0};
   if (len > 0) {
     c0 = c0 < 0 ? c0 + n2b : (c0 >= n2b ? c0 - n2b : c0);
     const uint32_t* rs = bin_start + (size_t)r * n2b;
     const int over = c0 + len - n2b;
-    scan_range(__ldg(&rs[c0]), __ldg(&rs[over > 0 ? n2b : c0 + len]), g, qx, qy, qz, sorted, best);
-    if (over > 0) scan_range(__ldg(&rs[0]), __ldg(&rs[over]), g, qx, qy, qz, sorted, best);
+    w.k0 = __ldg(&rs[c0]);
+    w.e0 = __ldg(&rs[over > 0 ? n2b : c0 + len]);
+    if (over > 0) {
+      w.k1 = __ldg(&rs[0]);
+      w.e1 = __ldg(&rs[over]);
+    }
   }
+  return w;
+}
+__device__ __forceinline__ void scan_window(const Window& w, int g, float qx, float qy, float qz,
+                                            const float4* __restrict__ sorted, NnKey& best) {
+  scan_range(w.k0, w.e0, g, qx, qy, qz, sorted, best);
+  if (w.e1 > w.k1) scan_range(w.k1, w.e1, g, qx, qy, qz, sorted, best);
 }
 
 // Minimum over the group; every lane gets it.  The whole warp takes part:
@@ -356,9 +369,13 @@ __device__ __forceinline__ void group_nn_min(NnKey& best) {
 // away from phi_q, and a point of the row within the bound has
 //   hav(dphi) <= x^2 = (hb - hav(row distance)) / (min(sin a, sin b) sin t_q)
 // (sin is concave, so its minimum over the row's colatitudes [a, b] is at an
-// edge).  dphi = 2 asin x is bounded by 2 x (1 + (pi/2 - 1) x^2): asin(x) / x is
-// convex in x^2, so its chord over [0, 1] lies above it.  The approximate
-// quotient and root are covered by the factor 1 + 1e-5.  n2b: the whole row.
+// edge).  dphi = 2 asin x takes Abramowitz and Stegun 4.4.45, which is within
+// 7e-5 of asin on [0, 1]; the approximate quotient and root are covered by the
+// factor 1 + 1e-5 on x^2 (a larger x has a larger asin).  Its error does not
+// grow with the window: a looser bound (10 % at x = 1) takes in the middle of a
+// cloud far from most directions, which the window of its near edge keeps out
+// (100 k points within a degree, B = 256: 13.1 ms so, 3.5 with asinf).  n2b: the
+// whole row.
 __device__ __forceinline__ int row_window(int r, int d, int n2b, float inv_2w, float stq, float hb,
                                           const float* __restrict__ sin_tab, const float* __restrict__ hav_tab) {
   if (hb >= 1.0f) return n2b;
@@ -366,19 +383,27 @@ __device__ __forceinline__ int row_window(int r, int d, int n2b, float inv_2w, f
   const float den = fminf(__ldg(&sin_tab[r]), __ldg(&sin_tab[r + 1])) * stq;
   if (!(num < den)) return n2b;  // the bound reaches every longitude (or a pole row)
   if (num <= 0.0f) return 0;
-  const float x2 = __fdividef(num, den) * (1.0f + 1e-5f);
-  const float e = 2.0f * sqrt_approx(x2) * fmaf(0.5708f, x2, 1.0f) * (1.0f + 1e-5f) + kAngleMargin;
+  const float x = sqrt_approx(__fdividef(num, den) * (1.0f + 1e-5f));
+  const float p = fmaf(fmaf(fmaf(-0.0187293f, x, 0.0742610f), x, -0.2121144f), x, 1.5707288f);
+  const float e = 3.14159265f - 2.0f * sqrt_approx(fmaxf(1.0f - x, 0.0f)) * p + 2e-4f + kAngleMargin;
   const float kf = fmaf(e, inv_2w, 0.5f);
   return kf >= (float)n2b ? n2b : (int)kf;
 }
 
 constexpr int kQueryThreads = 256;
+// Points of a wide window from which on it is probed.  A probe is a chain of
+// dependent loads of its own: with every wide window probed, sparse clouds and
+// ones seen through a narrow opening took longer than with one probe per
+// direction (37 points, B = 256: 285 us against 183; now 165).  256 rather than 64
+// or 128: 120 k points in a cone of 60 degrees, B = 100: 241, 288 and 276 us, scans of
+// full circles within 1 us of one another.
+constexpr uint32_t kProbePoints = 256;
 
 // One group of kGroup lanes per direction of the 2B x 2B grid: the
 // non-empty rows are visited outward from the direction's own row, nearest
 // colatitude first, while their colatitude distance can beat the bound.  A row
-// whose window is wide is probed at columns j - 1 .. j + 1 first, which makes
-// the bound finite at the first row and keeps it tight when that row holds
+// whose window is wide and holds many points is probed at columns j - 1 .. j + 1
+// first, which makes the bound finite at the first row and keeps it tight when that row holds
 // only stray points (the outermost beam's, split over two rows by rounding: a
 // bound from far along such a row had 37 % of the directions of a 128-beam scan
 // take the whole next row, 690 points a direction instead of about 60); then
@@ -431,25 +456,26 @@ k_nn_rows(int n2b, uint32_t mul_n2b, const __grid_constant__ CloudPair pr) {
     act = act && next_row();
     if (!__any_sync(0xffffffffu, act)) break;
     int k = act ? row_window(r, d, n2b, inv_2w, stq, hb, sin_tab, hav_tab) : 0;
-    // a wide window is probed at columns j - 1 .. j + 1 first
-    const bool probe = act && k >= 3;
-    const bool any_probe = __any_sync(0xffffffffu, probe);
-    if (any_probe) {
-      scan_cols(r, j - 1, probe ? pw : 0, n2b, g, q.x, q.y, q.z, bin_start, sorted, best);
+    bool all = 2 * k + 1 >= n2b;
+    int c0 = all ? 0 : j - k, len = act ? (all ? n2b : 2 * k + 1) : 0;
+    Window w = window(r, c0, len, n2b, bin_start);
+    // a wide window of many points is probed at columns j - 1 .. j + 1 first
+    const bool probe = act && k >= 3 && w.points() > kProbePoints;
+    if (__any_sync(0xffffffffu, probe)) {
+      scan_window(window(r, j - 1, probe ? pw : 0, n2b, bin_start), g, q.x, q.y, q.z, sorted, best);
       __syncwarp();
       group_nn_min(best);
       hb = hav_of_l2(nn_dist(best));
-      if (probe) k = row_window(r, d, n2b, inv_2w, stq, hb, sin_tab, hav_tab);
+      if (probe) {  // what the probe left: one piece of a whole row, else both sides
+        k = row_window(r, d, n2b, inv_2w, stq, hb, sin_tab, hav_tab);
+        all = 2 * k + 1 >= n2b;
+        c0 = all ? j + 2 : j - k;
+        len = all ? n2b - pw : k - 1;
+      }
+      scan_window(window(r, j + 2, probe && !all ? k - 1 : 0, n2b, bin_start), g, q.x, q.y, q.z, sorted, best);
+      w = window(r, c0, len, n2b, bin_start);
     }
-    const bool all = 2 * k + 1 >= n2b;
-    int c0 = all ? 0 : j - k, len = all ? n2b : 2 * k + 1;
-    if (probe) {  // what the probe left: one piece of a whole row, else both sides
-      c0 = all ? j + 2 : j - k;
-      len = all ? n2b - pw : k - 1;
-    }
-    scan_cols(r, c0, act ? len : 0, n2b, g, q.x, q.y, q.z, bin_start, sorted, best);
-    if (any_probe)
-      scan_cols(r, j + 2, probe && !all ? k - 1 : 0, n2b, g, q.x, q.y, q.z, bin_start, sorted, best);
+    scan_window(w, g, q.x, q.y, q.z, sorted, best);
     __syncwarp();
     group_nn_min(best);
     hb = hav_of_l2(nn_dist(best));

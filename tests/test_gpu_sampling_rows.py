@@ -77,3 +77,41 @@ def test_longitude_bound_is_an_upper_bound():
     x = np.sqrt(x2.astype(np.float32)).astype(np.float32)
     bound = 2 * x * (np.float32(0.5708) * x2.astype(np.float32) + 1) * np.float32(1 + 1e-5)
     assert np.all(bound.astype(np.float64) >= 2 * np.arcsin(np.sqrt(x2)))
+
+
+def test_arc_sine_bound_is_an_upper_bound():
+    """pi - 2 sqrt(1 - x) P(x) + 2e-4 >= 2 asin of the exact root on [0, 1], with x evaluated as the kernel does (float32,
+    a root short of 2^-22)."""
+    x2 = np.concatenate([np.linspace(0, 1, 200001), 1 - np.logspace(-12, -1, 20001)])
+    f = np.float32
+    x = np.sqrt(x2.astype(f) * f(1 + 1e-5)) * f(1 - 2.0 ** -22)
+    p = ((f(-0.0187293) * x + f(0.0742610)) * x + f(-0.2121144)) * x + f(1.5707288)
+    bound = f(3.14159265) - f(2) * (np.sqrt(np.maximum(f(1) - x, f(0))) * p) + f(2e-4)
+    slack = bound.astype(np.float64) - 2 * np.arcsin(np.sqrt(x2))
+    assert slack.min() >= 0 and slack.max() < 0.01
+
+
+@pytest.mark.parametrize("bw", [5, 16, 40, 64])
+@pytest.mark.parametrize("opening,n", [(60.0, 20000), (5.0, 20000), (0.3, 20000), (60.0, 300), (360.0, 40)])
+def test_narrow_openings(nat, bw, opening, n):
+    """Clouds seen through a narrow opening (windows of many and of few points, wide and far from the points)."""
+    rng = np.random.default_rng(bw + n)
+    a = 0.5 * np.deg2rad(opening)
+    if opening < 360:
+        v = np.stack([np.ones(n), np.tan(rng.uniform(-a, a, n)), np.tan(rng.uniform(-a, a, n))], 1) * rng.uniform(2, 9, (n, 1))
+        v = v @ np.linalg.qr(rng.standard_normal((3, 3)))[0]
+    else:
+        v = rng.standard_normal((n, 3))
+    xyzi = np.concatenate([v, rng.uniform(0, 1, (n, 1))], 1).astype(np.float32)
+    c = nat.Context(spherical_bandwidth=bw, spatial_n_voxels=4)
+    grid = O.dh_grid(bw)
+    pts, _ = O.project(xyzi)
+    idx, _ = O.nn(grid, pts)
+    c.sample_s2(xyzi, side=0)
+    _, got = c.samples(0)
+    bad = got != idx
+    if bad.any():  # as above: equal distances up to the projections' last bit
+        a = ((grid[bad] - pts[got[bad]]).astype(np.float64) ** 2).sum(1)
+        b = ((grid[bad] - pts[idx[bad]]).astype(np.float64) ** 2).sum(1)
+        assert np.all(np.sqrt(a) <= np.sqrt(b) + 3e-7)
+        assert bad.mean() < 0.01
