@@ -44,6 +44,7 @@
 
 #include "../../include/phaser_gpu.h"
 #include "ctx.h"
+#include "so3_common.cuh"
 
 using namespace phgpu;
 
@@ -79,20 +80,31 @@ ShapeKey key_of(const phgpu_params& p, const phgpu_cloud& t, const phgpu_cloud& 
                   p.spherical_low_pass_lower, p.spherical_low_pass_upper, p.precision, sig);
 }
 
-// Device bytes of one slot before any exists (an upper estimate; executors
-// are then accounted with their allocators' counts).
-uint64_t estimate_slot_bytes(const phgpu_params& p, uint32_t max_points) {
-  const uint64_t bw = p.spherical_bandwidth, bo = bw + p.spherical_zero_padding, N = p.spatial_n_voxels;
-  const uint64_t nv = N * N * N, H = N * N * ((N / 2 + 1 + 7) / 8 * 8);
-  uint64_t b = 0;
-  b += 4 * 4 * bw * bw * 2 + 8 * bw * bw * 8 + 8 * bw * 2 * bw * 8;  // samples, coefficients, SHT scratch
-  b += 8 * bo * bo * bo;                                           // S
-  b += 2 * 5 * nv * 4 + 9 * H * 8 + 4 * N * N;                     // grids, spectra, row flags
-  b += bw * bw * (bw + 1) * 4;                                     // Legendre table
-  if (p.flags & PHGPU_FLAG_KEEP_VOLUMES || p.rot_peak_neighbors) b += 8 * bo * bo * bo * 4;
-  if (p.flags & PHGPU_FLAG_KEEP_VOLUMES || p.trans_peak_neighbors) b += nv * 4;
-  b += 2ull * max_points * (16 + 4 + 4 + 4 + 16 + 8 + 4 + 16) + 2ull * 32768 * 48;
-  return b + (8ull << 20);
+// Device bytes of an executor of kmax slots before one exists: what
+// phgpu_ctx_init allocates per slot, and the shape's Wigner-d table (executors are
+// then accounted with their allocators' counts).  Never less than those: a
+// budget would be passed unseen.  (A padded translation is not served.)
+uint64_t estimate_executor_bytes(const phgpu_params& p, uint32_t max_points, int kmax) {
+  if (p.spherical_bandwidth > 512 || p.spatial_n_voxels > 1024) return 0;  // refused when the slots are made
+  const uint64_t bw = p.spherical_bandwidth, bo = bw + p.spherical_zero_padding, no = 2 * bo, nq = 4 * bw * bw;
+  const uint64_t N = p.spatial_n_voxels, nv = N * N * N;
+  const uint64_t H = N * N * spatial_h2p((int)N);
+  const bool tc = p.precision != PHGPU_PRECISION_FP32;
+  uint64_t b = nq * (16 + 2 * 4 * 4 + 2 * 4) + 8 * 2 * bw + 4 * N;               // directions, samples, weights, edges
+  if (p.spherical_fusion == PHGPU_FUSION_MIX) b += 2 * 4 * nq;
+  b += 4 * legendre_table_entries((int)bw) + (tc ? 4 * legendre_tc_floats((int)bw) : 0);
+  b += 8 * (8 * bw * bw + sht_scratch_entries((int)bw) + 2 * bw * (2 * bw - 1));  // coefficients, SHT scratch, fused
+  b += 8 * no * no * bo + 8 * (3 * no + wigner_table_entries((int)bw));           // S, angle and recurrence tables
+  b += 2 * (20 * nv + N * N) + 2 * N * N + 3 * N + 8 * 9 * H;                     // grids, row flags, spectra
+  if (p.flags & PHGPU_FLAG_KEEP_VOLUMES || p.rot_peak_neighbors) b += 4 * no * no * no;
+  if (p.flags & PHGPU_FLAG_KEEP_VOLUMES || p.trans_peak_neighbors) b += 4 * nv;
+  const uint64_t cap = max_points ? max_points : 1u << 18;
+  b += 2 * (cap * (16 + 4 + 4 + 4) + sampler_scratch_bytes((int)cap, (int)nq) + 256);
+  b += 64 << 10;  // pose, counts, maxima, one word for each empty buffer
+  b *= (uint64_t)kmax;
+  if (tc)  // classes (p, q), p <= q: degrees q .. bw - 1 rounded up to 8, and the class's offset
+    for (uint64_t q = 0; q < bw; ++q) b += (q + 1) * (4 * no * ((bw - q + 7) / 8 * 8) + sizeof(size_t));
+  return b;
 }
 
 // A Wigner-d table shared by the executors of one (bandwidth, output bandwidth).
@@ -163,7 +175,7 @@ struct phgpu_server {
       const int kmax = std::max(1, std::min<int>((int)prm.max_wave, kMaxWave));
       auto mb = measured_bytes.find(key);
       const uint64_t need =
-          mb != measured_bytes.end() ? mb->second : estimate_slot_bytes(rp, prm.max_points) * (uint64_t)kmax;
+          mb != measured_bytes.end() ? mb->second : estimate_executor_bytes(rp, prm.max_points, kmax);
       // evict idle executors (any shape, least recently used first) until the new one fits
       while (used_bytes + need > prm.hbm_budget_bytes) {
         Executor* lru = nullptr;

@@ -127,6 +127,49 @@ def test_budget_below_two_shapes_drains():
     srv.close()
 
 
+@pytest.mark.parametrize("bw,N,max_points,kw", [(16, 16, 4 << 20, {}), (128, 16, 1000, {}), (16, 128, 1000, {}),
+                                                (64, 16, 1000, {"precision": 1}), (32, 40, 1000, {"flags": 1})])
+def test_first_executor_of_a_shape_stays_within_the_budget(bw, N, max_points, kw):
+    """A budget a little short of two shapes' executors: the second shape is admitted by an estimate (its executors were
+    not counted yet), which must not be less than what it then allocates."""
+    from phaser_b200 import native as nat
+    rng = np.random.default_rng(1)
+    pts = np.concatenate([rng.uniform(-9, 9, (500, 3)), rng.uniform(0, 1, (500, 1))], 1).astype(np.float32)
+    shapes = [nat.default_params(spherical_bandwidth=b, spatial_n_voxels=n, spatial_discretize_lower=-10,
+                                 spatial_discretize_upper=10, **k) for b, n, k in ((8, 8, {}), (bw, N, kw))]
+
+    def used(params, **server):
+        srv = nat.Server(max_wave=2, lanes=1, device=0, max_points=max_points, **server)
+        for p in params:
+            t = srv.submit(p, (pts, None), (pts, None))
+            srv.drain()
+            assert srv.poll(t) is not None
+        st = srv.stats()
+        srv.close()
+        return st
+
+    alone = [used([p])["bytes_in_use"] for p in shapes]
+    budget = sum(alone) - min(alone) // 64
+    st = used(shapes, hbm_budget_bytes=budget)
+    assert st["bytes_in_use"] <= budget
+    assert st["evictions"] == 1
+    # and no more than an eighth above: a budget of both with that much room holds both
+    assert used(shapes, hbm_budget_bytes=sum(alone) + alone[1] // 8 + (1 << 20))["evictions"] == 0
+
+
+@pytest.mark.parametrize("kw", [{"spherical_bandwidth": 0xffffffff}, {"spherical_bandwidth": 70000, "precision": 1},
+                                {"spatial_n_voxels": 0xfffffff0}, {"spherical_bandwidth": 0}])
+def test_sizes_out_of_range_are_refused(kw):
+    from phaser_b200 import native as nat
+    pts = np.ones((8, 4), np.float32)
+    srv = nat.Server(max_wave=2, lanes=1, device=0)
+    t = srv.submit(nat.default_params(**dict(dict(spherical_bandwidth=4, spatial_n_voxels=4), **kw)), (pts, None), (pts, None))
+    srv.drain()
+    with pytest.raises(nat.PhgpuError):
+        srv.poll(t)
+    srv.close()
+
+
 def test_server_reports_bad_request():
     from phaser_b200 import native as nat
     srv = nat.Server(max_wave=2, lanes=1, device=0)
