@@ -1100,16 +1100,18 @@ static size_t fuse_z_smem(int N, int C, int wt) {
 
 constexpr size_t kFuseZStatic = 2 * 1024;  // the kernel's static and the system's shared memory, rounded up
 
-bool fuse_z_tile_ok(int N, int A, int wt) {
-  return (wt == 2 || wt == 4 || wt == 8 || wt == 16) && fuse_z_smem(N, A / 2, wt) + kFuseZStatic <= (size_t)kMaxSmem;
-}
-
 // Tile width of the z pass: the widest (<= 8: 64-byte rows) of which two
 // blocks fit on an SM, since the blocks hide one another's barriers and loads.
 static int fuse_z_tile(int N, int C) {
   int wt = 8;
   while (wt > 2 && fuse_z_smem(N, C, wt) + kFuseZStatic > (size_t)kMaxSmem / 2) wt >>= 1;
   return wt;
+}
+
+int fuse_z_width(int N, int C, int tile) {
+  const bool fits = (tile == 2 || tile == 4 || tile == 8 || tile == 16) && fuse_z_smem(N, C, tile) + kFuseZStatic <= (size_t)kMaxSmem;
+  const int wt = fits ? tile : fuse_z_tile(N, C);
+  return fixed_length(N) ? (wt >= 8 ? 8 : 4) : wt;
 }
 
 // Threads of a z-pass block: the least idle time over its stages.  With a
@@ -1185,8 +1187,7 @@ cudaError_t launch_spatial_forward(const SpatialArgs& a, int side, cudaStream_t 
 cudaError_t launch_spatial_fuse_z(const SpatialArgs& a, cudaStream_t st) {
   const int N = a.N, H2 = N / 2 + 1;
   const int C = a.laplace ? a.n_data_ch : 1;
-  int wt = fuse_z_tile_ok(N, 2 * C, a.fuse_tile) ? a.fuse_tile : fuse_z_tile(N, C);
-  if (fixed_length(N)) wt = wt >= 8 ? 8 : 4;  // the widths built for compile-time lengths
+  const int wt = fuse_z_width(N, C, a.fuse_tile);
   const size_t sm = fuse_z_smem(N, C, wt);
   if (sm + kFuseZStatic > (size_t)kMaxSmem) return cudaErrorInvalidConfiguration;
   const dim3 g((H2 + wt - 1) / wt, N);

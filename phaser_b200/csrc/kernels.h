@@ -242,8 +242,9 @@ struct SpatialArgs {
   uint32_t argmax_limit = 0;   // argmax over indices < limit (0: all)
   int fuse_tile = 0;           // ky columns per k_fuse_z block (2, 4, 8, 16; 0 = the widest up to 8 with two blocks per SM): tuned
 };
-// Whether a k_fuse_z tile of wt ky columns fits shared memory for N and A arrays.
-bool fuse_z_tile_ok(int N, int A, int wt);
+// Width of the z pass's tiles for N, C channels a side and a wanted width (0: none): that width if it fits shared
+// memory, one of the two built (4, 8) at compile-time lengths.
+int fuse_z_width(int N, int C, int tile);
 cudaError_t launch_spatial_forward(const SpatialArgs& a, int side, cudaStream_t st);
 cudaError_t launch_spatial_fuse_z(const SpatialArgs& a, cudaStream_t st);   // z FFTs + fusion + cross power
 cudaError_t launch_spatial_inverse(const SpatialArgs& a, cudaStream_t st);  // inverse x + C2R y + argmax

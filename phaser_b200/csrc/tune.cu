@@ -102,8 +102,17 @@ int phgpu_autotune(phgpu_ctx* ctx, const phgpu_cloud* target, const phgpu_cloud*
     std::vector<uint32_t> cand;
     int stage;
   };
-  std::vector<Param> params = {{&phgpu_tuning::fuse_z_tile, {0, 2, 4, 8, 16}, PS_FUSE_Z},
-                               {&phgpu_tuning::so3_beta_tile, {8, 16, 32}, PS_SO3_FFT}};
+  std::vector<Param> params;
+  if (!ctx->pad) {  // the padded translation has no tiles
+    // the widths that differ in what they launch: two at compile-time lengths
+    const PairPlan pp = pair_plan(ctx, target->reflectivity, target->ambient, source->reflectivity, source->ambient);
+    const int C = pp.laplace_sp ? pp.nd_sp : 1;
+    Param widths{&phgpu_tuning::fuse_z_tile, {}, PS_FUSE_Z};
+    for (uint32_t v : {2u, 4u, 8u, 16u})
+      if (fuse_z_width(ctx->N, C, (int)v) == (int)v) widths.cand.push_back(v);
+    params.push_back(widths);
+  }
+  params.push_back({&phgpu_tuning::so3_beta_tile, {8, 16, 32}, PS_SO3_FFT});
   if (ctx->prm.precision != PHGPU_PRECISION_FP32) params.push_back({&phgpu_tuning::tc_chunk, {16, 32}, PS_SO3_SYNTH});
   if (has_runtime_plan(ctx)) params.push_back({&phgpu_tuning::radix_order, {0, 1, 2}, -1});
   phgpu_tuning cur = ctx->tune;

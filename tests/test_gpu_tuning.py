@@ -65,3 +65,20 @@ def test_radix_orders_keep_parity(nat, order):
     assert (pose.rot_bin, pose.voxel) == (res[0].rot_bin, res[0].voxel)
     assert np.linalg.norm(rv - res[1]) <= 1e-5 * np.linalg.norm(res[1])
     assert np.linalg.norm(tv - res[2]) <= 1e-5 * np.linalg.norm(res[2])
+
+
+@pytest.mark.parametrize("bw,N,pad,searched", [(32, 64, 0, 2 + 3), (32, 48, 0, 4 + 3 + 3), (32, 64, 32, 3)])
+def test_every_candidate_launches_something_else(nat, bw, N, pad, searched):
+    """The search times each z-pass width that exists (two at compile-time lengths, none for the padded translation)
+    once, and what it reports is the width that runs."""
+    from phaser_b200 import scene
+    pair = scene.workload_pair(1, 1)
+    clouds = ((pair.target.xyzi, None), (pair.source.xyzi, None))
+    c = nat.Context(spherical_bandwidth=bw, spatial_n_voxels=N, spatial_zero_padding=pad)
+    c.register_pair(*clouds)
+    before = nat.launch_count()
+    c.register_pair(*clouds)
+    one = nat.launch_count() - before
+    best, _ = c.autotune(*clouds, reps=1)
+    assert nat.launch_count() - before == one * (1 + 2 * (searched + 1))
+    assert best["fuse_z_tile"] in ((0,) if pad else (4, 8) if N == 64 else (2, 4, 8, 16))
