@@ -432,21 +432,6 @@ struct FixedFft {
   static constexpr int count = 0;
 };
 template <>
-struct FixedFft<16> {
-  static constexpr int count = 2;
-  static constexpr int r[2] = {8, 2};
-};
-template <>
-struct FixedFft<32> {
-  static constexpr int count = 2;
-  static constexpr int r[2] = {8, 4};
-};
-template <>
-struct FixedFft<100> {
-  static constexpr int count = 3;
-  static constexpr int r[3] = {4, 5, 5};
-};
-template <>
 struct FixedFft<64> {
   static constexpr int count = 2;
   static constexpr int r[2] = {8, 8};
@@ -508,9 +493,8 @@ __host__ __device__ __forceinline__ int fixed_pos2freq(int pos) {
   }
 }
 
-// One stage with compile-time length, radix and block length.  LOG2T >= 0:
-// column mode with 2^LOG2T transforms and the transform index fastest;
-// LOG2T < 0: row mode (estride 1), butterfly index fastest.
+// One stage with compile-time length, radix and block length.  LOG2T == -2:
+// columns, transform index fastest; -1: rows (estride 1), butterfly index fastest.
 template <int N, int R, int L, bool INV, int LOG2T>
 __device__ __forceinline__ void fixed_stage(float2* buf, int ntrans, int tstride, int estride,
                                             const float2* __restrict__ tw, int tid, int nthr) {
@@ -521,10 +505,7 @@ __device__ __forceinline__ void fixed_stage(float2* buf, int ntrans, int tstride
   const int es = m * estride;
   for (int it = tid; it < total; it += nthr) {
     int t, bf;
-    if constexpr (LOG2T >= 0) {
-      bf = it >> LOG2T;
-      t = it & ((1 << LOG2T) - 1);
-    } else if constexpr (LOG2T == -2) {
+    if constexpr (LOG2T == -2) {
       bf = it / ntrans;
       t = it - bf * ntrans;
     } else {
@@ -563,8 +544,7 @@ __device__ __forceinline__ void fixed_stages(float2* buf, int ntrans, int tstrid
 }
 
 // Batched in-place transform with a compile-time plan (same contract as
-// fft_smem).  LOG2T >= 0: columns, ntrans == 2^LOG2T; LOG2T == -2: columns,
-// any ntrans; LOG2T == -1: rows (estride 1).
+// fft_smem).  LOG2T == -2: columns; LOG2T == -1: rows (estride 1).
 template <int N, bool INV, int LOG2T = -1>
 __device__ __forceinline__ void fft_fixed(float2* buf, int ntrans, int tstride, int estride,
                                           const float2* __restrict__ tw) {

@@ -1,4 +1,5 @@
-// Register-tail FFT engine for the fixed lengths of the workloads (FP32).
+// Register-tail FFT engine for the fixed lengths of the workloads (FP32), kept
+// with its self-test: the library's kernels use fft_pass.cuh.
 //
 // A length N is split as N = R0 (* R1) * M: one or two in-place radix stages
 // through shared memory, then every block of M contiguous positions is
@@ -18,6 +19,18 @@
 #include "fft.cuh"
 
 namespace phgpu {
+
+// compile-time plans of two lengths that the library runs on runtime plans
+template <>
+struct FixedFft<32> {
+  static constexpr int count = 2;
+  static constexpr int r[2] = {8, 4};
+};
+template <>
+struct FixedFft<100> {
+  static constexpr int count = 3;
+  static constexpr int r[3] = {4, 5, 5};
+};
 
 // ---------------------------------------------------------------- register blocks
 
