@@ -200,10 +200,10 @@ constexpr int kMaxVoxels = 1024;  // longest transform
 // packed multiply-add per channel.  Rows without a point are neither read nor
 // written: the x transform takes them as zero.
 //
-// Block: 16 rows (fewer on small grids, scan_rows_block) of one z-slab; a warp takes a live row, gathers its
-// occupied voxels in order (counts, then every channel's sums, all loads of 256
-// voxels in flight) into shared memory and gives each lane up to four
-// frequencies at a time.  Small blocks spread a slab full of long rows (a floor
+// Block: 16 rows (fewer on small grids, scan_rows_block) of one z-slab; a warp
+// takes a live row, gathers its occupied voxels in order (counts, then every
+// channel's sums, all loads of 256 voxels in flight) into shared memory and gives
+// each lane up to four frequencies at a time.  Small blocks spread a slab full of long rows (a floor
 // seen level) over many SMs.  With `clear` the voxels and row flags are zeroed
 // on the way, so a grid that is only transformed needs no memset and no
 // separate pass before its next voxelisation.  With the x pass behind it a side
@@ -1120,8 +1120,8 @@ int fuse_z_width(int N, int C, int tile) {
 static int fuse_z_threads(const FftPlan& p, int C, int wt) {
   if (!fixed_length(p.n))
     return pass_threads(p, C * wt, 1, 128, fuse_z_max_threads<0>(), 80, fuse_z_smem(p.n, C, wt));
-  // a grid of at most three blocks an SM (N = 64): one thread per item of the first stage, whose items are one
-  // channel's (15 -> 13 us)
+  // a grid of at most three blocks an SM (of the compile-time lengths N = 64): one thread per item of the first
+  // stage, whose items are one channel's (15 -> 13 us); runtime plans weigh the threads resident on an SM above
   if ((p.n / 2 + wt) / wt * p.n <= 3 * 148)
     return std::max(64, std::min((C * wt * p.n / p.radix[0] + 31) / 32 * 32, fuse_z_max_threads<64>()));
   int best = 256;

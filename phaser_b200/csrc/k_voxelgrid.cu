@@ -29,8 +29,10 @@
 // reduction that ends in the plan, stable 8-bit LSD radix passes over the
 // leaf index's bits (a ranked scatter per tile, which also counts the tile's
 // items for the next pass; the first makes the (leaf, point) pairs of the
-// finite points), a compaction of the leaf heads, and one warp per leaf for the centroid (gathers pipelined two
-// batches ahead, in-order float sums).
+// finite points), a compaction of the leaf heads, and the centroids: a leaf of up
+// to 128 points by a warp that stages them in one batch, a longer one by its
+// block, whose other warps gather the next 896 points while the first adds, one
+// lane per component, in input order.
 // Nothing synchronises the host until the output count is read.  Bound by the
 // latency of the nine dependent launches: a 131072-point scan at 0.25 m takes
 // 84 us (154 with twenty-one launches and one lane adding a leaf).

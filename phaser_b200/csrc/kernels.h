@@ -27,8 +27,10 @@ inline void count_launches(int n) {
 // (1-2 us each, twenty of them) are a third of a small registration.  With
 // programmatic launch the next kernel's blocks are set up while the last ones
 // of this kernel run, and wait inside chain_begin().  Off by default: captured
-// waves and other concurrent streams would only lose the slots that waiting
-// blocks hold.  B = 32, N = 64: 165 -> 136 us with the clouds read in place.
+// waves would only lose the slots that waiting blocks hold.  B = 32, N = 64: 165 ->
+// 136 us with the clouds read in place.  Contexts on threads of their own launch
+// so too: eight of them at N = 64 31 us a pair (35 without), at B = 100 / N = 200 310
+// (300), where the device is full anyway; four 298 (297), one 394 (414).
 extern thread_local bool g_chain_launch;
 struct ChainScope {
   bool before;
