@@ -212,11 +212,12 @@ constexpr int kMaxVoxels = 1024;  // longest transform
 constexpr int kRowsWarps = 4;
 // One running sum over a row rounds in proportion to the root of its voxels:
 // from some twenty on it is further off than an FFT (a full row of 512: 3.9e-7
-// against 0.9e-7, relative L2; of 16 voxels 0.7e-7 against 0.8e-7).  Lengths with a
-// half plan (below) sum shorter rows only; at the others, sums of 8 voxels, of
-// 8 such sums and then over the row stay below the FFT's error at every length
-// and occupancy (0.9e-7 there).  Sums beyond the first 64 voxels are added to the
-// stored ones: no third set of registers.
+// against 0.9e-7, relative L2; of 16 voxels 0.7e-7 against 0.8e-7).  Rows of more
+// than kShortRow voxels are summed in parts: sums of 8 voxels, of 8 such sums and
+// then over the row stay below the FFT's error at every length and occupancy
+// (0.9e-7 there).  Sums beyond the first 64 voxels are added to the stored ones: no
+// third set of registers.
+constexpr int kShortRow = 16;
 constexpr int kPartSum = 8;
 constexpr int kRunSum = 64;
 
@@ -224,12 +225,14 @@ constexpr int kRunSum = 64;
 // a complex one of n / 2 (even and odd columns as real and imaginary parts) per
 // channel, by the warp that gathered the row, where n / 2 has a plan of
 // register radices (n is even, no prime above 7).  A voxel's sum costs every
-// frequency an addition, the FFT costs the same whatever the row holds: they
-// meet at 16 to 24 voxels, and from 16 on the sum rounds more.  A row of a room's
-// scan has four to six; the correlation of two full grids took 107 us summed at
-// N = 64 and now 73, 376 and 205 at N = 128, 1370 and 510 at N = 200, 4518 and
-// 1385 at N = 256.
-constexpr int kDenseRow = 16;
+// frequency an addition, the FFT costs the same whatever the row holds.  Over
+// grids full of such rows they meet at 12 (N = 64) to 30 voxels, but among a
+// scan's rows (four to six voxels) a single one that takes the FFT's stages in turn
+// is the last to finish: with 16 voxels for the limit a side of some N = 200 rooms
+// takes 2 to 3 us more, with 40 none.  The correlation of two full grids took 107 us
+// summed at N = 64 and now 73, 376 and 211 at N = 128, 1370 and 515 at N = 200, 4518
+// and 1395 at N = 256.
+static int dense_row_limit(int N) { return std::min(std::max(N / 5, 16), 40); }
 
 struct ScanRowArgs {
   int N, rows_block;
@@ -241,7 +244,8 @@ struct ScanRowArgs {
   float2* spec;         // [channel][z][x][H2p]
   size_t spec_stride;
   int clear;
-  FftPlan half;         // length N / 2 for dense rows; n = 0: every row is summed
+  int dense;            // rows of more voxels are transformed
+  FftPlan half;         // length N / 2 for them
   const uint16_t* half_pos;  // [N / 2] position of each of its frequencies
 };
 
@@ -302,6 +306,72 @@ __device__ __noinline__ void dense_row(const ScanRowArgs& a, float4* s_val, cons
   }
 }
 
+// Adds a voxel to the sums for frequencies k + 32 i.
+template <int CC, int Q>
+__device__ __forceinline__ void add_voxel(float2 (&acc)[CC][Q], float4 w, uint32_t y, const float2* s_tw, int n,
+                                          uint32_t mul, int k) {
+  const float ws[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+  for (int i = 0; i < Q; ++i) {
+    const uint32_t p = (uint32_t)(k + 32 * i) * y;
+    const float2 t = s_tw[p - __umulhi(p, mul) * (uint32_t)n];
+#pragma unroll
+    for (int ch = 0; ch < CC; ++ch) acc[ch][i] = __ffma2_rn(make_float2(ws[ch], ws[ch]), t, acc[ch][i]);
+  }
+}
+template <int CC, int Q>
+__device__ __forceinline__ void zero_sums(float2 (&acc)[CC][Q]) {
+#pragma unroll
+  for (int ch = 0; ch < CC; ++ch)
+#pragma unroll
+    for (int i = 0; i < Q; ++i) acc[ch][i] = make_float2(0.f, 0.f);
+}
+template <int CC, int Q>
+__device__ __forceinline__ void store_sums(const float2 (&acc)[CC][Q], float2* out, size_t stride, int k, int H2,
+                                           bool more) {
+#pragma unroll
+  for (int i = 0; i < Q; ++i) {
+    const int ky = k + 32 * i;
+    if (ky < H2) {
+#pragma unroll
+      for (int ch = 0; ch < CC; ++ch) {
+        float2* o = out + ch * stride + ky;
+        *o = more ? cadd(*o, acc[ch][i]) : acc[ch][i];
+      }
+    }
+  }
+}
+
+// The sums of a row in parts.
+template <int CC>
+__device__ __noinline__ void part_row(const ScanRowArgs& a, const float4* s_val, const uint16_t* s_y, const float2* s_tw,
+                                      int cnt, int lane, float2* out) {
+  const int n = a.N, H2 = n / 2 + 1;
+  const uint32_t mul = fast_div_mul(n);
+  constexpr int Q = 2;  // two sets of sums: fewer frequencies at a time, for the caller's registers
+  for (int k = lane; k < H2 + lane; k += 32 * Q) {
+    for (int e = 0; e < cnt;) {
+      float2 sum[CC][Q];
+      zero_sums(sum);
+      const int stored = e, run = min(cnt, e + kRunSum);
+      for (; e < run; e = min(run, e + kPartSum)) {
+        float2 part[CC][Q];
+        zero_sums(part);
+#pragma unroll
+        for (int u = 0; u < kPartSum; ++u) {  // all the part's loads in flight; past the end a zero at column 0
+          const bool in = e + u < run;
+          add_voxel(part, in ? s_val[e + u] : make_float4(0.f, 0.f, 0.f, 0.f), in ? s_y[e + u] : 0, s_tw, n, mul, k);
+        }
+#pragma unroll
+        for (int ch = 0; ch < CC; ++ch)
+#pragma unroll
+          for (int i = 0; i < Q; ++i) sum[ch][i] = cadd(sum[ch][i], part[ch][i]);
+      }
+      store_sums(sum, out, a.spec_stride, k, H2, stored > 0);
+    }
+  }
+}
+
 // Shared memory: N twiddles, then per warp N float4 (means) and N uint16 (y).
 static size_t scan_rows_smem(int N) { return (size_t)N * (8 + kRowsWarps * 18) + 16 * (kRowsWarps + 1); }
 
@@ -316,12 +386,11 @@ static int scan_rows_block(int N) {
   return rows;
 }
 
-// FFT: the length has a half plan (dense rows are transformed, the others' sums are short).
-template <int CC, bool FFT>
+template <int CC>
 __global__ void __launch_bounds__(kRowsWarps * 32) k_scan_rows(const __grid_constant__ ScanRowArgs a) {
   chain_begin();
   extern __shared__ __align__(16) float4 s_mem[];
-  constexpr int U = 8, Q = 4;
+  constexpr int U = 8;
   const int n = a.N, H2 = n / 2 + 1, H2p = spatial_h2p(n);
   const int z = blockIdx.x, x0 = blockIdx.y * a.rows_block, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool mine = lane < a.rows_block && x0 + lane < n;
@@ -371,71 +440,19 @@ __global__ void __launch_bounds__(kRowsWarps * 32) k_scan_rows(const __grid_cons
     }
     __syncwarp();
     float2* out = a.spec + row * H2p;
-    if constexpr (FFT) {
-      if (cnt > kDenseRow) {
+    if (cnt > kShortRow) {
+      if (cnt > a.dense)
         dense_row<CC>(a, s_val, s_y, s_tw, bits, cnt, lane, out);
-        __syncwarp();
-        continue;
-      }
-    }
-    // X[k0 + 32 i + lane] plus the sum over entries [e, end) of the list
-    auto add = [&](float2 (&acc)[CC][Q], int k0, int& e, int end) {
-#pragma unroll 2
-      for (; e < end; ++e) {
-        const uint32_t y = s_y[e];
-        const float4 w = s_val[e];
-        const float ws[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-        for (int i = 0; i < Q; ++i) {
-          const uint32_t k = (uint32_t)(k0 + 32 * i + lane) * y;
-          const float2 t = s_tw[k - __umulhi(k, mul) * (uint32_t)n];
-#pragma unroll
-          for (int ch = 0; ch < CC; ++ch) acc[ch][i] = __ffma2_rn(make_float2(ws[ch], ws[ch]), t, acc[ch][i]);
-        }
-      }
-    };
-    auto zero = [](float2 (&acc)[CC][Q]) {
-#pragma unroll
-      for (int ch = 0; ch < CC; ++ch)
-#pragma unroll
-        for (int i = 0; i < Q; ++i) acc[ch][i] = make_float2(0.f, 0.f);
-    };
-    auto put = [&](const float2 (&acc)[CC][Q], int k0, bool more) {
-#pragma unroll
-      for (int i = 0; i < Q; ++i) {
-        const int ky = k0 + 32 * i + lane;
-        if (ky < H2) {
-#pragma unroll
-          for (int ch = 0; ch < CC; ++ch) {
-            float2* o = out + ch * a.spec_stride + ky;
-            *o = more ? cadd(*o, acc[ch][i]) : acc[ch][i];
-          }
-        }
-      }
-    };
-    for (int k0 = 0; k0 < H2; k0 += 32 * Q) {
-      int e = 0;
-      if constexpr (FFT) {
+      else
+        part_row<CC>(a, s_val, s_y, s_tw, cnt, lane, out);
+    } else {
+      constexpr int Q = 4;
+      for (int k0 = 0; k0 < H2; k0 += 32 * Q) {
         float2 sum[CC][Q];
-        zero(sum);
-        add(sum, k0, e, cnt);
-        put(sum, k0, false);
-      } else {
-        do {
-          float2 sum[CC][Q];
-          zero(sum);
-          const int stored = e, run = min(cnt, e + kRunSum);
-          while (e < run) {
-            float2 part[CC][Q];
-            zero(part);
-            add(part, k0, e, min(run, e + kPartSum));
-#pragma unroll
-            for (int ch = 0; ch < CC; ++ch)
-#pragma unroll
-              for (int i = 0; i < Q; ++i) sum[ch][i] = cadd(sum[ch][i], part[ch][i]);
-          }
-          put(sum, k0, stored > 0);
-        } while (e < cnt);
+        zero_sums(sum);
+#pragma unroll 2
+        for (int e = 0; e < cnt; ++e) add_voxel(sum, s_val[e], s_y[e], s_tw, n, mul, k0 + lane);
+        store_sums(sum, out, a.spec_stride, k0 + lane, H2, false);
       }
     }
     __syncwarp();
@@ -1049,12 +1066,9 @@ static FftXFn fft_x_forward(int C) {
                           : (C == 3 ? k_fft_x<NF, false, 3, kXFwdLog2> : k_fft_x<NF, false, 4, kXFwdLog2>));
 }
 
-using ScanRowsFn = void (*)(const ScanRowArgs);
-template <bool FFT>
-static ScanRowsFn scan_rows_channels(int C) {
-  return C == 1 ? k_scan_rows<1, FFT> : (C == 2 ? k_scan_rows<2, FFT> : (C == 3 ? k_scan_rows<3, FFT> : k_scan_rows<4, FFT>));
+static auto scan_rows_kernel(int C) {
+  return C == 1 ? k_scan_rows<1> : (C == 2 ? k_scan_rows<2> : (C == 3 ? k_scan_rows<3> : k_scan_rows<4>));
 }
-static ScanRowsFn scan_rows_kernel(int C, bool fft) { return fft ? scan_rows_channels<true>(C) : scan_rows_channels<false>(C); }
 
 template <int NF>
 static cudaError_t set_attrs() {
@@ -1074,8 +1088,7 @@ cudaError_t spatial_init_attributes(int N, int M) {
   PHGPU_DISPATCH_N(N, e = set_attrs<NF>());
   if (e == cudaSuccess && M != N) PHGPU_DISPATCH_N(M, e = set_attrs<NF>());
   for (int C = 1; C <= 4; ++C)
-    for (bool fft : {false, true})
-      if (e == cudaSuccess) e = allow_max_smem((const void*)scan_rows_kernel(C, fft));
+    if (e == cudaSuccess) e = allow_max_smem((const void*)scan_rows_kernel(C));
   return e;
 }
 
@@ -1158,10 +1171,10 @@ cudaError_t launch_spatial_forward(const SpatialArgs& a, int side, cudaStream_t 
   } else {
     const ScanRowArgs r{N, scan_rows_block(N), reinterpret_cast<float4*>(grids), grids + 4 * nv, a.plan->tw, a.rowlive[side],
                         a.rowmask + (size_t)side * N * N, spec, plane, a.clear,
-                        a.plan_half ? *a.plan_half : FftPlan{}, a.half_pos};
+                        a.plan_half ? dense_row_limit(N) : N, a.plan_half ? *a.plan_half : FftPlan{}, a.half_pos};
     const dim3 gr(N, (N + r.rows_block - 1) / r.rows_block);
     const size_t smr = scan_rows_smem(N);
-    launch_kernel(scan_rows_kernel(nch, a.plan_half != nullptr), dim3(gr), dim3(kRowsWarps * 32), smr, st, r);
+    launch_kernel(scan_rows_kernel(nch), dim3(gr), dim3(kRowsWarps * 32), smr, st, r);
   }
   // channels of one launch: as many as leave two blocks an SM's shared memory
   const size_t per = (size_t)N * (1 << kXFwdLog2) * sizeof(float2), extra = prime_scratch(N) + (size_t)N;

@@ -186,8 +186,8 @@ def test_full_rows_round_no_more_than_an_fft(nat, N):
 @pytest.mark.parametrize("N,channels", [(28, 1), (30, 2), (48, 3), (50, 4), (64, 3), (98, 2), (100, 3), (108, 4), (200, 1), (256, 1),
                                         (320, 1)])
 def test_rows_around_the_density_limit(nat, N, channels):
-    """Rows of 16 (summed), 17 and N - 1 voxels (transformed), full ones and ones with a gap at either end, in one
-    slab: the correlation against FP64 at the bar for volumes, twice from kept grids, and again after a registration
+    """Rows of 16 voxels (one sum), of 17 and of as many as are still summed in parts, of one more (transformed), full
+    ones and ones with a gap at either end, in one slab: the correlation against FP64 at the bar for volumes, twice from kept grids, and again after a registration
     that clears them on the way."""
     rng = np.random.default_rng(N)
     half = 10
@@ -201,7 +201,9 @@ def test_rows_around_the_density_limit(nat, N, channels):
     for side in range(2):
         cols = [np.arange(16), rng.choice(N, 16, replace=False), rng.choice(N, 17, replace=False), np.arange(N - 17, N),
                 np.arange(N), np.arange(1, N), np.arange(N - 1), np.array([N // 2])]
-        xyz = np.concatenate([np.stack([np.full(len(y), at[(3 * i + side) % N]), at[y], np.full(len(y), at[N // 3 + side])], 1)
+        limit = min(max(N // 5, 16), 40)
+        cols[4:4] = [rng.choice(N, min(limit + k, N), replace=False) for k in (0, 1)]
+        xyz = np.concatenate([np.stack([np.full(len(y), at[(2 * i + side) % N]), at[y], np.full(len(y), at[N // 3 + side])], 1)
                               for i, y in enumerate(cols)])
         xyzi = np.concatenate([xyz, rng.uniform(0.1, 1.0, (len(xyz), 1))], 1).astype(np.float32)
         refl, amb = rng.uniform(0.1, 1.0, (2, len(xyzi))).astype(np.float32)
